@@ -93,6 +93,27 @@ __device__ __forceinline__ float det_expf(float x) {
     return scale_pow2(p, (int)k);
 }
 
+// det_expf for x <= 0 (or NaN), without branches: the same operations, the
+// cases that a negative argument cannot reach left out.
+__device__ __forceinline__ float det_expf_neg(float x) {
+    float k = rintf(fmul(x, 1.44269502f));
+    float r = __fmaf_rn(-k, UDS_LN2_HI, x);
+    r = __fmaf_rn(-k, UDS_LN2_LO, r);
+    float p = 1.0f / 5040.0f;
+    p = __fmaf_rn(p, r, 1.0f / 720.0f);
+    p = __fmaf_rn(p, r, 1.0f / 120.0f);
+    p = __fmaf_rn(p, r, 1.0f / 24.0f);
+    p = __fmaf_rn(p, r, 1.0f / 6.0f);
+    p = __fmaf_rn(p, r, 0.5f);
+    p = __fmaf_rn(p, r, 1.0f);
+    p = __fmaf_rn(p, r, 1.0f);
+    int n = (int)k;
+    bool sub = n < -126;  // two exact scalings, as scale_pow2
+    p = fmul(p, sub ? 0x1p-126f : 1.0f);
+    p = fmul(p, __uint_as_float((unsigned)(n + (sub ? 253 : 127)) << 23));
+    return x < -103.972084f ? 0.0f : p;
+}
+
 __device__ __forceinline__ float det_logf(float x) {
     if (x != x) return x;
     if (x < 0.0f) return __int_as_float(0x7fc00000);
@@ -134,7 +155,7 @@ __device__ __forceinline__ float facf(unsigned n) {
 // Salmon, Moraes, Dror & Shaw, "Parallel random numbers: as easy as 1, 2, 3"
 // (SC'11).  counter = (pixel, view, round*ceil(K/4)+group, 0), key = seed.
 __device__ __forceinline__ void philox4x32_10(uint32_t c[4], uint32_t k0, uint32_t k1) {
-#pragma unroll
+#pragma unroll 2
     for (int r = 0; r < 10; ++r) {
         uint32_t hi0 = __umulhi(0xD2511F53u, c[0]), lo0 = 0xD2511F53u * c[0];
         uint32_t hi1 = __umulhi(0xCD9E8D57u, c[2]), lo1 = 0xCD9E8D57u * c[2];

@@ -645,72 +645,72 @@ __global__ void __launch_bounds__(32 * kP2MWarps) k_p2m(const ViewState* vs, con
     float* tx = s_tx[warp];
     float* ty = s_ty[warp];
     while (todo) {
-        int k = __ffs(todo) - 1;
-        todo &= todo - 1;
-        float4 c;
-        c.x = __shfl_sync(full, cl.x, k);
-        c.y = __shfl_sync(full, cl.y, k);
-        c.w = __shfl_sync(full, cl.w, k);
-        int first = __shfl_sync(full, Ll.z, k), count = __shfl_sync(full, Ll.w, k);
-        int p = meta_degree(c.w);
-        int off = meta_offset(c.w);
-        int P1 = p + 1;
-        int BR = kP2MBlock[P1][0], BC = kP2MBlock[P1][1];
-        int nC = (P1 + BC - 1) / BC, nR = (P1 + BR - 1) / BR;
-        int gr = lane / nC, gc = lane % nC;
-        bool owner = gr < nR;
-        // this lane's rows and columns; reads past the table repeat its last
-        // row / column (their sums are not written)
-        int ra[3], cb[4];
+            int k = __ffs(todo) - 1;
+            todo &= todo - 1;
+            float4 c;
+            c.x = __shfl_sync(full, cl.x, k);
+            c.y = __shfl_sync(full, cl.y, k);
+            c.w = __shfl_sync(full, cl.w, k);
+            int first = __shfl_sync(full, Ll.z, k), count = __shfl_sync(full, Ll.w, k);
+            int p = meta_degree(c.w);
+            int off = meta_offset(c.w);
+            int P1 = p + 1;
+            int BR = kP2MBlock[P1][0], BC = kP2MBlock[P1][1];
+            int nC = (P1 + BC - 1) / BC, nR = (P1 + BR - 1) / BR;
+            int gr = lane / nC, gc = lane % nC;
+            bool owner = gr < nR;
+            // this lane's rows and columns; reads past the table repeat its last
+            // row / column (their sums are not written)
+            int ra[3], cb[4];
 #pragma unroll
-        for (int i = 0; i < 3; ++i) ra[i] = min(gr * BR + i, p);
+            for (int i = 0; i < 3; ++i) ra[i] = min(gr * BR + i, p);
 #pragma unroll
-        for (int q = 0; q < 4; ++q) cb[q] = min(gc * BC + q, p);
-        float acc[3][4];
-#pragma unroll
-        for (int i = 0; i < 3; ++i)
-#pragma unroll
-            for (int q = 0; q < 4; ++q) acc[i][q] = 0.0f;
-        int end = first + count;
-        for (int i0 = first; i0 < end; i0 += 32) {
-            int cnt = min(32, end - i0);
-            if (lane < cnt) {
-                float2 q = leaf_xy[i0 + lane];
-                float s0 = fmul(fsub(q.x, c.x), isq);
-                float s1 = fmul(fsub(q.y, c.y), isq);
-                float ax = 1.0f, ay = 1.0f;
-                tx[lane * kTStride] = 1.0f;
-                ty[lane * kTStride] = 1.0f;
-                for (int a = 1; a <= p; ++a) {
-                    ax = fmul(fmul(ax, s0), kInvInt[a]);
-                    ay = fmul(fmul(ay, s1), kInvInt[a]);
-                    tx[lane * kTStride + a] = ax;
-                    ty[lane * kTStride + a] = ay;
-                }
-            }
-            __syncwarp();
-            if (owner) {
-                switch (BR * 8 + BC) {  // uniform over the warp
-                    case 9: p2m_block<1, 1>(tx, ty, cnt, ra, cb, acc); break;
-                    case 10: p2m_block<1, 2>(tx, ty, cnt, ra, cb, acc); break;
-                    case 11: p2m_block<1, 3>(tx, ty, cnt, ra, cb, acc); break;
-                    case 18: p2m_block<2, 2>(tx, ty, cnt, ra, cb, acc); break;
-                    case 19: p2m_block<2, 3>(tx, ty, cnt, ra, cb, acc); break;
-                    case 20: p2m_block<2, 4>(tx, ty, cnt, ra, cb, acc); break;
-                    default: p2m_block<3, 4>(tx, ty, cnt, ra, cb, acc); break;
-                }
-            }
-            __syncwarp();
-        }
-        if (owner) {
+            for (int q = 0; q < 4; ++q) cb[q] = min(gc * BC + q, p);
+            float acc[3][4];
 #pragma unroll
             for (int i = 0; i < 3; ++i)
 #pragma unroll
-                for (int q = 0; q < 4; ++q) {
-                    int a = gr * BR + i, b = gc * BC + q;
-                    if (i < BR && q < BC && a <= p && b <= p) coef[off + a * P1 + b] = acc[i][q];
+                for (int q = 0; q < 4; ++q) acc[i][q] = 0.0f;
+            int end = first + count;
+            for (int i0 = first; i0 < end; i0 += 32) {
+                int cnt = min(32, end - i0);
+                if (lane < cnt) {
+                    float2 q = leaf_xy[i0 + lane];
+                    float s0 = fmul(fsub(q.x, c.x), isq);
+                    float s1 = fmul(fsub(q.y, c.y), isq);
+                    float ax = 1.0f, ay = 1.0f;
+                    tx[lane * kTStride] = 1.0f;
+                    ty[lane * kTStride] = 1.0f;
+                    for (int a = 1; a <= p; ++a) {
+                        ax = fmul(fmul(ax, s0), kInvInt[a]);
+                        ay = fmul(fmul(ay, s1), kInvInt[a]);
+                        tx[lane * kTStride + a] = ax;
+                        ty[lane * kTStride + a] = ay;
+                    }
                 }
-        }
+                __syncwarp();
+                if (owner) {
+                    switch (BR * 8 + BC) {  // uniform over the warp
+                        case 9: p2m_block<1, 1>(tx, ty, cnt, ra, cb, acc); break;
+                        case 10: p2m_block<1, 2>(tx, ty, cnt, ra, cb, acc); break;
+                        case 11: p2m_block<1, 3>(tx, ty, cnt, ra, cb, acc); break;
+                        case 18: p2m_block<2, 2>(tx, ty, cnt, ra, cb, acc); break;
+                        case 19: p2m_block<2, 3>(tx, ty, cnt, ra, cb, acc); break;
+                        case 20: p2m_block<2, 4>(tx, ty, cnt, ra, cb, acc); break;
+                        default: p2m_block<3, 4>(tx, ty, cnt, ra, cb, acc); break;
+                    }
+                }
+                __syncwarp();
+            }
+            if (owner) {
+#pragma unroll
+                for (int i = 0; i < 3; ++i)
+#pragma unroll
+                    for (int q = 0; q < 4; ++q) {
+                        int a = gr * BR + i, b = gc * BC + q;
+                        if (i < BR && q < BC && a <= p && b <= p) coef[off + a * P1 + b] = acc[i][q];
+                    }
+            }
     }
 }
 
@@ -743,8 +743,8 @@ struct Tree {
 __device__ __forceinline__ float leaf_mass(const Tree& T, float4 c, float qx, float qy) {
     float tx = fmul(fsub(qx, c.x), T.isq);
     float ty = fmul(fsub(qy, c.y), T.isq);
-    float ex = det_expf(-fmul(tx, tx));
-    float ey = det_expf(-fmul(ty, ty));
+    float ex = det_expf_neg(-fmul(tx, tx));
+    float ey = det_expf_neg(-fmul(ty, ty));
     return fadd(0.0f, fmul(fmul(1.0f, ex), ey));
 }
 
@@ -752,8 +752,8 @@ __device__ __forceinline__ float hermite_eval(const Tree& T, int v, float4 c, fl
     if (v >= T.n - 1) return leaf_mass(T, c, qx, qy);
     float tx = fmul(fsub(qx, c.x), T.isq);
     float ty = fmul(fsub(qy, c.y), T.isq);
-    float ex = det_expf(-fmul(tx, tx));
-    float ey = det_expf(-fmul(ty, ty));
+    float ex = det_expf_neg(-fmul(tx, tx));
+    float ey = det_expf_neg(-fmul(ty, ty));
     int p = meta_degree(c.w);
     const float* C = T.coef + meta_offset(c.w);
     float hy[kMaxDegree + 1];
@@ -761,54 +761,45 @@ __device__ __forceinline__ float hermite_eval(const Tree& T, int v, float4 c, fl
     hy[0] = ey;
     hy[1] = fmul(ty2, ey);
 #pragma unroll
-    for (int k = 2; k <= kMaxDegree; ++k)
-        if (k <= p) hy[k] = fsub(fmul(ty2, hy[k - 1]), fmul(fmul(2.0f, (float)(k - 1)), hy[k - 2]));
+    for (int k = 2; k <= kMaxDegree; ++k) {
+        if ((k & 3) == 0 && k > p) break;
+        hy[k] = fsub(fmul(ty2, hy[k - 1]), fmul(2.0f * (float)(k - 1), hy[k - 2]));
+    }
     float tx2 = fmul(2.0f, tx);
     float hxm2 = 0.0f, hxm1 = 0.0f;
     float w = 0.0f;
     const int P1 = p + 1;
-    int a = 0;
     // Rows four at a time: the four row sums are independent chains, so they
-    // are interleaved; each chain and the outer sum keep their order.
-    for (; a + 4 <= P1; a += 4) {
-        float h[4];
-#pragma unroll
-        for (int q = 0; q < 4; ++q) {
-            int aa = a + q;
-            float hx = aa == 0 ? ex
-                               : (aa == 1 ? fmul(tx2, ex)
-                                          : fsub(fmul(tx2, hxm1), fmul(fmul(2.0f, (float)(aa - 1)), hxm2)));
-            h[q] = hx;
-            hxm2 = hxm1;
-            hxm1 = hx;
-        }
+    // are interleaved; each chain and the outer sum keep their order.  The
+    // columns go in blocks of four as well: a block past p costs nothing.
+#pragma unroll 1
+    for (int a = 0; a < P1; a += 4) {
         const float* C0 = C + a * P1;
+        const int n1 = a + 1 < P1 ? P1 : 0, n2 = a + 2 < P1 ? 2 * P1 : 0, n3 = a + 3 < P1 ? 3 * P1 : 0;
         float r0 = 0.0f, r1 = 0.0f, r2 = 0.0f, r3 = 0.0f;
 #pragma unroll
         for (int b = 0; b <= kMaxDegree; ++b) {
+            if ((b & 3) == 0 && b > p) break;
             if (b <= p) {
                 r0 = __fmaf_rn(C0[b], hy[b], r0);
-                r1 = __fmaf_rn(C0[P1 + b], hy[b], r1);
-                r2 = __fmaf_rn(C0[2 * P1 + b], hy[b], r2);
-                r3 = __fmaf_rn(C0[3 * P1 + b], hy[b], r3);
+                r1 = __fmaf_rn(C0[n1 + b], hy[b], r1);
+                r2 = __fmaf_rn(C0[n2 + b], hy[b], r2);
+                r3 = __fmaf_rn(C0[n3 + b], hy[b], r3);
             }
         }
-        w = __fmaf_rn(h[0], r0, w);
-        w = __fmaf_rn(h[1], r1, w);
-        w = __fmaf_rn(h[2], r2, w);
-        w = __fmaf_rn(h[3], r3, w);
-    }
-    for (; a <= p; ++a) {
-        float hx = a == 0 ? ex
-                          : (a == 1 ? fmul(tx2, ex) : fsub(fmul(tx2, hxm1), fmul(fmul(2.0f, (float)(a - 1)), hxm2)));
-        const float* Ca = C + a * P1;
-        float r = 0.0f;
+        const float r[4] = {r0, r1, r2, r3};
 #pragma unroll
-        for (int b = 0; b <= kMaxDegree; ++b)
-            if (b <= p) r = __fmaf_rn(Ca[b], hy[b], r);
-        w = __fmaf_rn(hx, r, w);
-        hxm2 = hxm1;
-        hxm1 = hx;
+        for (int q = 0; q < 4; ++q) {
+            if (a + q <= p) {
+                float hx = q == 0 && a == 0 ? ex
+                                            : (q == 1 && a == 0 ? fmul(tx2, ex)
+                                                                : fsub(fmul(tx2, hxm1),
+                                                                       fmul(2.0f * (float)(a + q - 1), hxm2)));
+                w = __fmaf_rn(hx, r[q], w);
+                hxm2 = hxm1;
+                hxm1 = hx;
+            }
+        }
     }
     return w;
 }
@@ -855,179 +846,456 @@ __device__ float node_weight(const Tree& T, int v, float qx, float qy) {
     return w;
 }
 
+// The same out of line, for the rare callers outside the descent's loop.
 __device__ __noinline__ float node_weight_out_of_line(Tree T, int v, float qx, float qy) {
     return node_weight(T, v, qx, qy);
 }
 
 // --------------------------------------------------------------- 8 sampler
-// Per-pixel mass cache.  getWeight(v) of a node without expansion that the
-// truncation circle reaches is the running sum, in depth-first order, of the
-// expansions below it; one walk from the root therefore yields getWeight of
-// every node it opens if each opened node keeps its own running sum, fed the
-// same values in the same order (so the sums are bit-identical to separate
-// walks).  The opened nodes and the frontier nodes whose expansion the walk
-// evaluated are stored in pre-order, one 8-byte record each: the mass and
-// the entries of the two children.  A child entry is -1 when the child's box
-// misses the truncation circle (it has no expansion, so its getWeight is
-// exactly 0) and -2 below an expansion (not walked: its children's masses
-// are evaluated when needed).  The descent reads one record per child and
-// level.
-constexpr int kTable = 160;
-constexpr int kNotWalked = -2;
+// Masses of every node the pixels of a warp meet.
+//
+// getWeight(v) of a node without expansion that the truncation circle
+// reaches is the sum, in depth-first order, of the expansions below it.  The
+// 32 pixels of a warp (a tile of the image) share one table of the union of
+// their trees:
+//   topology: level by level, the nodes opened by at least one lane; each
+//     lane fetches one opened node's children, so a level costs one memory
+//     round trip however many nodes it has.  Counts up the levels and
+//     offsets down them then number the expansions they lead to in
+//     depth-first order;
+//   masses: the expansions one after another, each evaluated by the whole
+//     warp for its 32 pixels (hermite_tile), the next one's coefficients on
+//     their way meanwhile.  Lanes that are not inside an expansion hold 0.
+// The expansions below a node are a range of that list, and its mass is the
+// range's sum in order: the additions of a walk from that node (adding the
+// zeros of other lanes changes nothing), so bit-identical to it.  The descent
+// sums a range when it meets the node.
+//
+// Lists and masses live in the warp's shared memory, one row of 32 floats
+// per expansion (a lane reads its own column: no bank conflicts whatever row
+// it is at); rows past kRows go to local memory.  Where the tables are full
+// (pixels far apart in units of the bandwidth share little of the tree), the
+// caller takes half the lanes at a time.
+constexpr int kOpen = 224, kEvals = 192;  // table entries
+constexpr int kRows = 64;                 // masses in shared memory
+constexpr int kLevels = 64;               // a radix tree over 62-bit keys is at most 63 deep
+// Per-lane records of the descent in shared memory: local memory that is
+// written and read back costs an L2 round trip here (about 700 cycles).
+constexpr int kPathRows = 32;
+// 65536 / S rounded up: e * kReciprocal[S] >> 16 = e / S for e < S * S
+__constant__ unsigned kReciprocal[21] = {0,    65536, 32768, 21846, 16384, 13108, 10923, 9363, 8192, 7282, 6554,
+                                         5958, 5462,  5042,  4682,  4370,  4096,  3856,  3641, 3450, 3277};
+constexpr int kSide = 20;                 // Hermite functions and coefficients per side (17, in blocks of four)
 
-__device__ __forceinline__ int2 mass_rec(float mass, int left, int right) {
-    return make_int2(__float_as_int(mass), (int)(((unsigned)left & 0xffffu) | ((unsigned)right << 16)));
+// A child's link: kind, stop bit (the child holds at most M splats), entry
+// of an opened child.
+constexpr unsigned kLinkOpen = 0u, kLinkEval = 0x4000u, kLinkNone = 0x8000u;
+constexpr unsigned kLinkKind = 0xC000u, kLinkStop = 0x2000u, kLinkEntry = 0x1FFFu;
+
+struct WarpTables {
+    uint4 open[kOpen];               // links (left | right << 16), left child, right child, lanes that opened it
+    unsigned short split[kOpen];     // first expansion of the right subtree
+    union {
+        float val[kRows][32];
+        struct {                     // while the topology is built
+            unsigned short count[kOpen], first[kOpen], level[kLevels + 8];
+            float4 box[2][32];       // children of up to 32 nodes: boxes and squared radii
+            float r2[2][32];
+        };
+    };
+    union {
+        struct {                     // until the masses are known
+            uint2 eval[kEvals];      // node, lanes inside
+            float coef[2][kSide * kSide];  // the expansion being evaluated and the next one, in whole blocks of
+                                           // 4 x 4, padded with zeros
+            float hermite[12][kSide];      // Hermite functions of the tile's columns, then of its rows
+        };
+        struct {                     // afterwards
+            float path[kPathRows][32];         // per-lane records of the levels below the stem
+            float series[kMaxDegree + 1][32];  // Hermite functions of a lane's own series (lane_series)
+        };
+    };
+    int owner[32];                   // warp_child_masses
+};
+
+// Blocks of four coefficients per side of a degree-p expansion.
+__device__ __forceinline__ int coef_blocks(int p) { return (p + 4) >> 2; }
+
+// Starts the copy of an expansion's coefficients to dst, a square of 4 nb per
+// side: (p + 1) x (p + 1) coefficients, zeros past them.
+__device__ __forceinline__ void stage(float* dst, const float* __restrict__ C, int p, int nb, int lane) {
+    const int S = 4 * nb, P1 = p + 1;
+    const unsigned rec = kReciprocal[S];
+    unsigned to = (unsigned)__cvta_generic_to_shared(dst) + 4u * (unsigned)lane;
+#pragma unroll 1
+    for (int e = lane; e < S * S; e += 32, to += 128u) {
+        const int row = (int)((unsigned)e * rec >> 16), col = e - row * S;
+        const bool ok = row < P1 && col < P1;
+        const float* from = ok ? C + row * P1 + col : C;
+        asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"(to), "l"(from), "r"(ok ? 4 : 0));
+    }
+    asm volatile("cp.async.commit_group;");
 }
-__device__ __forceinline__ float rec_mass(int2 r) { return __int_as_float(r.x); }
-__device__ __forceinline__ int rec_left(int2 r) { return (int)(short)(r.y & 0xffff); }
-__device__ __forceinline__ int rec_right(int2 r) { return r.y >> 16; }
-// the record of a node the cache does not hold
-__device__ __forceinline__ int2 no_record() { return mass_rec(0.0f, kNotWalked, kNotWalked); }
 
-struct MassCache {
-    int2 rec[kTable];
-    int m;
-    bool ok;
-};
+// The Hermite series of the staged expansion at the 32 pixels of a warp tile
+// of G rows and 32 / G columns (lane % (32 / G) is the column).  Pixels of
+// one column have the same y, hence the same Hermite functions h_b(y) and row
+// sums r_a = sum_b C_ab h_b(y), and pixels of one row the same h_a(x).  So
+// one lane per column and row computes the functions; each of a column's G
+// lanes sums one of G rows at a time, four coefficients per shared-memory
+// read; and the lanes exchange the sums.  Every recursion, every row's chain
+// and the outer sum keep their order; the padding adds zeros at the end of
+// each, so the value is hermite_eval's.  Loops stay rolled: with the descent
+// around it the kernel is bound by instruction fetch once its code outgrows
+// the instruction cache.  (q, centre): this lane's coordinate and the
+// expansion's along it, see warp_tables.
+__device__ __forceinline__ float hermite_tile(WarpTables& wt, const float* coef, int nb, int cols, float q,
+                                              float centre, float isq, int lane) {
+    const unsigned full = 0xffffffffu;
+    const int G = 32 / cols, S = 4 * nb;
+    {
+        float t = fmul(fsub(q, centre), isq);
+        float e = det_expf_neg(-fmul(t, t));
+        float t2 = fmul(2.0f, t);
+        float4 h;
+        h.x = e;
+        h.y = fmul(t2, e);
+        h.z = fsub(fmul(t2, h.y), fmul(2.0f, h.x));
+        h.w = fsub(fmul(t2, h.z), fmul(4.0f, h.y));
+        float4* row = reinterpret_cast<float4*>(wt.hermite[min(lane, 11)]);  // cols + G = 12
+        const bool writes = lane < 12;
+        if (writes) row[0] = h;
+        float k2 = 6.0f;  // 2 (k - 1): small whole numbers, exact
+#pragma unroll 1
+        for (int b = 1; b < nb; ++b, k2 += 8.0f) {
+            float u = h.z, v = h.w;
+            h.x = fsub(fmul(t2, v), fmul(k2, u));
+            h.y = fsub(fmul(t2, h.x), fmul(k2 + 2.0f, v));
+            h.z = fsub(fmul(t2, h.y), fmul(k2 + 4.0f, h.x));
+            h.w = fsub(fmul(t2, h.z), fmul(k2 + 6.0f, h.y));
+            if (writes) row[b] = h;
+        }
+    }
+    __syncwarp();
+    const int col = lane & (cols - 1), mine = lane / cols;
+    const float4* hy = reinterpret_cast<const float4*>(wt.hermite[col]);
+    const float4* hx = reinterpret_cast<const float4*>(wt.hermite[cols + mine]);
+    float w = 0.0f;
+#pragma unroll 1
+    for (int a0 = 0; a0 < S; a0 += G) {
+        const float4* C = reinterpret_cast<const float4*>(coef + min(a0 + mine, S - 1) * S);
+        float r = 0.0f;
+#pragma unroll 1
+        for (int b = 0; b < nb; ++b) {
+            const float4 c = C[b], h = hy[b];
+            r = __fmaf_rn(c.x, h.x, r);
+            r = __fmaf_rn(c.y, h.y, r);
+            r = __fmaf_rn(c.z, h.z, r);
+            r = __fmaf_rn(c.w, h.w, r);
+        }
+#pragma unroll 1
+        for (int s = 0; s < G && a0 + s < S; s += 4) {
+            const float4 h = hx[(a0 + s) >> 2];
+            const int from = col + cols * s;
+            w = __fmaf_rn(h.x, __shfl_sync(full, r, from), w);
+            w = __fmaf_rn(h.y, __shfl_sync(full, r, from + cols), w);
+            w = __fmaf_rn(h.z, __shfl_sync(full, r, from + 2 * cols), w);
+            w = __fmaf_rn(h.w, __shfl_sync(full, r, from + 3 * cols), w);
+        }
+    }
+    return w;
+}
 
-// Warp-cooperative walk.  The 32 pixels of a warp (an 8 x 4 tile) walk the
-// union of their trees in lock-step.  At a node, every lane inside tests its
-// own truncation circle; lanes that open the node continue into its children,
-// the others leave that subtree.  Restricted to one lane, the union walk
-// visits exactly that lane's nodes in its own depth-first order, so the
-// running sums are unchanged; but expansion coefficients are now loaded once
-// per warp and the Hermite loops run with warp-uniform bounds.
-//
-// Each iteration enters one node (its centre, box and links in one round
-// trip to memory); the stack in shared memory holds the opened ancestors
-// (lanes that opened each, its right child), and whether an ancestor's right
-// subtree is under way is one bit of a register.  After a node that is not
-// descended into, finished ancestors are closed in the same iteration.
-//
-// The running sums of a lane's opened ancestors live in shared memory,
-// acc[depth][lane]: every lane inside a node has opened the same ancestors,
-// so the update loop over them has one trip count per warp and touches one
-// bank per lane; each sum is written to the lane's cache once, when its node
-// is closed.  The stack holds kWalkDepth levels (the trees built here are
-// about 20-30 deep; a smaller block leaves more of the SM's L1 to the
-// per-lane caches).  A lane whose walk would go deeper gives up its cache
-// (the descent then evaluates masses directly) and takes its total from a
-// direct subtree walk.
-constexpr int kWalkDepth = 40;
-struct WalkStack {
-    unsigned mask[kWalkDepth];  // lanes that opened the ancestor at this depth
-    int right[kWalkDepth];      // its right child
-    float acc[kWalkDepth][32];
-};
+// node_weight of one lane's own node, the case of an expansion in few
+// instructions: Hermite functions of y in the lane's column of wt.series,
+// rows four at a time (independent chains); hermite_eval's operations in its
+// order.  Nodes without one (rare here) go out of line.
+__device__ __forceinline__ float lane_series(const Tree& T, WarpTables& wt, int lane, int v, float qx, float qy) {
+    const float4 c = T.cen[v];
+    const int p = meta_degree(c.w);
+    if (p < 0) return node_weight_out_of_line(T, v, qx, qy);
+    float tx = fmul(fsub(qx, c.x), T.isq);
+    float ty = fmul(fsub(qy, c.y), T.isq);
+    float ex = det_expf_neg(-fmul(tx, tx));
+    float ey = det_expf_neg(-fmul(ty, ty));
+    if (v >= T.n - 1) return fadd(0.0f, fmul(fmul(1.0f, ex), ey));
+    const float* C = T.coef + meta_offset(c.w);
+    {
+        const float t2 = fmul(2.0f, ty);
+        float h0 = ey, h1 = fmul(t2, ey), k2 = 2.0f;
+        wt.series[0][lane] = h0;
+#pragma unroll 1
+        for (int k = 1; k <= p; ++k, k2 += 2.0f) {
+            wt.series[k][lane] = h1;
+            float h = fsub(fmul(t2, h1), fmul(k2, h0));
+            h0 = h1;
+            h1 = h;
+        }
+    }
+    const float t2 = fmul(2.0f, tx);
+    float hx = ex, hxm = 0.0f, k2 = 0.0f;  // h_a and h_(a-1) of x
+    float w = 0.0f;
+    const int P1 = p + 1;
+#pragma unroll 1
+    for (int a = 0; a < P1; a += 4, C += 4 * P1) {
+        const int n1 = a + 1 < P1 ? P1 : 0, n2 = a + 2 < P1 ? 2 * P1 : 0, n3 = a + 3 < P1 ? 3 * P1 : 0;
+        float r[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+#pragma unroll 2
+        for (int b = 0; b < P1; ++b) {
+            const float h = wt.series[b][lane];
+            r[0] = __fmaf_rn(C[b], h, r[0]);
+            r[1] = __fmaf_rn(C[n1 + b], h, r[1]);
+            r[2] = __fmaf_rn(C[n2 + b], h, r[2]);
+            r[3] = __fmaf_rn(C[n3 + b], h, r[3]);
+        }
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+            if (a + q <= p) w = __fmaf_rn(hx, r[q], w);
+            float h = fsub(fmul(t2, hx), fmul(k2, hxm));
+            hxm = hx;
+            hx = h;
+            k2 += 2.0f;
+        }
+    }
+    return w;
+}
 
-__device__ void warp_root_walk(const Tree& T, float qx, float qy, bool live, MassCache& mc, float& total,
-                               WalkStack& ws) {
+// !truncated_box, the radius squared beforehand.
+__device__ __forceinline__ bool within(float4 b, float r2, float qx, float qy) {
+    float dx = fsub(qx, fminf(fmaxf(qx, b.x), b.z)), dy = fsub(qy, fminf(fmaxf(qy, b.y), b.w));
+    return fadd(fmul(dx, dx), fmul(dy, dy)) < r2;
+}
+
+// Fills the tables for the lanes of `lanes` (all 32 lanes call this).
+// Returns the number of expansions listed (opened node 0 is the root), 0
+// when there are no tables (the root carries an expansion, or no lane
+// reaches it), -1 when they are full (nothing computed).  total is getWeight
+// of the root for the lanes inside.
+__device__ int warp_tables(const Tree& T, float qx, float qy, unsigned lanes, int M, int cols, WarpTables& wt,
+                           float* val_hi, float& total) {
     const unsigned full = 0xffffffffu;
     const int lane = (threadIdx.x + blockDim.x * threadIdx.y) & 31;
-    mc.m = 0;
-    mc.ok = true;
+    const unsigned lt = (1u << lane) - 1u;
     total = 0.0f;
-    unsigned liveMask = __ballot_sync(full, live);
-    float4 c = T.cen[0];
-    if (meta_degree(c.w) >= 0) {
-        if (live) total = hermite_eval(T, 0, c, qx, qy);
-        return;
-    }
-    if (!liveMask) return;
-    // per opened ancestor (same index in every lane inside): its entry, its
-    // left child's entry and where its right child's entry would start
-    int ostack[kWalkDepth], lstack[kWalkDepth], rstack[kWalkDepth];
-    int osp = 0;
-    int sp = -1;                    // deepest opened ancestor of v
-    unsigned long long onright = 0; // bit k: ancestor k's right subtree is under way
-    int v = 0;                      // node entered next, and the lanes inside it
-    unsigned in = liveMask;
-    bool deep = false;  // a subtree was not walked: total is incomplete
-    int budget = 4 * T.n + 64;
-    while (true) {
-        if (--budget < 0) { mc.ok = false; deep = true; break; }
-        bool mine = (in >> lane) & 1u;
-        c = T.cen[v];
-        float4 bx = T.box[v];
-        int4 Lv = T.lnk[v];
-        bool descend = false;
+    const bool live = (lanes >> lane) & 1u;
+    {
+        float4 c = T.cen[0];
         if (meta_degree(c.w) >= 0) {
-            if (mine) {
-                float val = hermite_eval(T, v, c, qx, qy);
-                total = fadd(total, val);
-                if (mc.ok) {
-                    for (int q = 0; q < osp; ++q) ws.acc[q][lane] = fadd(ws.acc[q][lane], val);
-                    if (mc.m < kTable) {
-                        mc.rec[mc.m] = mass_rec(val, kNotWalked, kNotWalked);
-                        ++mc.m;
-                    } else {
-                        mc.ok = false;
-                    }
-                }
+            if (live) total = node_weight_out_of_line(T, 0, qx, qy);
+            return 0;
+        }
+        lanes = __ballot_sync(full, live && !truncated(T, 0, c.z, qx, qy));
+        if (!lanes) return 0;
+    }
+    __syncwarp();
+    if (lane == 0) {
+        int4 L = T.lnk[0];
+        wt.open[0] = make_uint4(0u, (unsigned)L.x, (unsigned)L.y, lanes);
+        wt.level[0] = 0;
+    }
+    __syncwarp();
+    // ---- topology
+    int lo = 0, hi = 1, levels = 0;  // opened nodes of this level
+    while (lo < hi) {
+        if (levels >= kLevels) return -1;
+        int next = hi;
+        for (int base = lo; base < hi; base += 32) {
+            const int cnt = min(32, hi - base);
+            const int o = base + min(lane, cnt - 1);
+            const uint4 E = wt.open[o];
+            const int a = (int)E.y, b = (int)E.z;
+            const float4 ca = T.cen[a], cb = T.cen[b];
+            const float4 ba = T.box[a], bb = T.box[b];
+            const int4 La = T.lnk[a], Lb = T.lnk[b];
+            unsigned ma = 0u, mb = 0u;  // lanes whose circle reaches the children of this lane's node
+            wt.box[0][lane] = ba;
+            wt.box[1][lane] = bb;
+            wt.r2[0][lane] = fmul(ca.z, ca.z);
+            wt.r2[1][lane] = fmul(cb.z, cb.z);
+            __syncwarp();
+#pragma unroll 1
+            for (int k = 0; k < cnt; ++k) {
+                const bool inside = (wt.open[base + k].w >> lane) & 1u;
+                unsigned hit = __ballot_sync(full, inside && within(wt.box[0][k], wt.r2[0][k], qx, qy));
+                if (lane == k) ma = hit;
+                hit = __ballot_sync(full, inside && within(wt.box[1][k], wt.r2[1][k], qx, qy));
+                if (lane == k) mb = hit;
             }
-        } else {
-            bool op = mine && !truncated_box(bx, c.z, qx, qy);
-            unsigned opened = __ballot_sync(full, op);
-            // v sits at depth sp + 1; its children would be at sp + 2
-            if (opened && sp + 2 >= kWalkDepth) {
-                if (op) {  // this lane's subtree below v is not walked
-                    mc.ok = false;
-                    deep = true;
+            __syncwarp();
+            const bool ea = meta_degree(ca.w) >= 0, eb = meta_degree(cb.w) >= 0;
+            const bool oa = lane < cnt && !ea && ma, ob = lane < cnt && !eb && mb;
+            const unsigned Ba = __ballot_sync(full, oa), Bb = __ballot_sync(full, ob);
+            const int pa = next + __popc(Ba & lt) + __popc(Bb & lt), pb = pa + (oa ? 1 : 0);
+            next += __popc(Ba) + __popc(Bb);
+            if (next > kOpen) return -1;
+            if (lane < cnt) {
+                unsigned la = ea ? kLinkEval : kLinkNone, lb = eb ? kLinkEval : kLinkNone;
+                if (oa) {
+                    la = kLinkOpen | (La.w <= M ? kLinkStop : 0u) | (unsigned)pa;
+                    wt.open[pa] = make_uint4(0u, (unsigned)La.x, (unsigned)La.y, ma);
                 }
-            } else if (opened) {
-                if (op && mc.ok) {
-                    if (mc.m < kTable && osp < kWalkDepth) {
-                        ws.acc[osp][lane] = 0.0f;
-                        ostack[osp++] = mc.m++;
-                    } else {
-                        mc.ok = false;
-                    }
+                if (ob) {
+                    lb = kLinkOpen | (Lb.w <= M ? kLinkStop : 0u) | (unsigned)pb;
+                    wt.open[pb] = make_uint4(0u, (unsigned)Lb.x, (unsigned)Lb.y, mb);
                 }
-                ++sp;
-                onright &= ~(1ull << sp);
-                if (lane == 0) {
-                    ws.mask[sp] = opened;
-                    ws.right[sp] = Lv.y;
-                }
-                v = Lv.x;
-                in = opened;
-                descend = true;
+                wt.open[o].x = la | (lb << 16);
             }
+        }
+        ++levels;
+        if (lane == 0) wt.level[levels] = (unsigned short)hi;
+        lo = hi;
+        hi = next;
+        __syncwarp();
+    }
+    // ---- expansions below each opened node, up the levels
+    auto children = [&](uint4 E, int& na, int& nb) {
+        unsigned la = E.x & 0xffffu, lb = E.x >> 16;
+        na = (la & kLinkKind) == kLinkOpen ? wt.count[la & kLinkEntry] : (la == kLinkEval ? 1 : 0);
+        nb = (lb & kLinkKind) == kLinkOpen ? wt.count[lb & kLinkEntry] : (lb == kLinkEval ? 1 : 0);
+    };
+#pragma unroll 1
+    for (int l = levels - 1; l >= 0; --l) {
+#pragma unroll 1
+        for (int o = wt.level[l] + lane; o < wt.level[l + 1]; o += 32) {
+            int na, nb;
+            children(wt.open[o], na, nb);
+            wt.count[o] = (unsigned short)(na + nb);
         }
         __syncwarp();
-        if (descend) continue;
-        // climb: close ancestors whose right subtree is done; at the first
-        // one whose left subtree is done, continue with its right child
-        bool more = false;
-        while (sp >= 0) {
-            unsigned pin = ws.mask[sp];
-            bool pm = (pin >> lane) & 1u;
-            if (!((onright >> sp) & 1ull)) {
-                // the left child, if recorded, directly follows its parent
-                if (pm && mc.ok) {
-                    int q = ostack[osp - 1];
-                    lstack[osp - 1] = mc.m > q + 1 ? q + 1 : -1;
-                    rstack[osp - 1] = mc.m;
-                }
-                onright |= 1ull << sp;
-                v = ws.right[sp];
-                in = pin;
-                more = true;
-                break;
-            }
-            if (pm && mc.ok) {
-                int q = ostack[--osp];
-                int rs = rstack[osp];
-                mc.rec[q] = mass_rec(ws.acc[osp][lane], lstack[osp], mc.m > rs ? rs : -1);
-            }
-            --sp;
-        }
-        if (!more) break;
-        __syncwarp();  // the stack slots read above may be rewritten next
     }
-    // the same running sum in the same order, by a direct walk (rare: out of
-    // line)
-    if (deep && live) total = node_weight_out_of_line(T, 0, qx, qy);
+    const int nV = wt.count[0];
+    if (nV > kEvals) return -1;
+    // ---- and their places in depth-first order, down the levels
+    if (lane == 0) wt.first[0] = 0;
+    __syncwarp();
+#pragma unroll 1
+    for (int l = 0; l < levels; ++l) {
+#pragma unroll 1
+        for (int o = wt.level[l] + lane; o < wt.level[l + 1]; o += 32) {
+            uint4 E = wt.open[o];
+            int na, nb, s = wt.first[o];
+            children(E, na, nb);
+            unsigned la = E.x & 0xffffu, lb = E.x >> 16;
+            wt.split[o] = (unsigned short)(s + na);
+            if ((la & kLinkKind) == kLinkOpen) wt.first[la & kLinkEntry] = (unsigned short)s;
+            else if (la == kLinkEval) wt.eval[s] = make_uint2(E.y, E.w);
+            if ((lb & kLinkKind) == kLinkOpen) wt.first[lb & kLinkEntry] = (unsigned short)(s + na);
+            else if (lb == kLinkEval) wt.eval[s + na] = make_uint2(E.z, E.w);
+        }
+        __syncwarp();
+    }
+    // ---- masses.  Lane l < cols computes the Hermite functions of column l,
+    // lane cols + g those of row g; the next expansion's coefficients are
+    // copied meanwhile.
+    const bool columns = lane < cols;
+    const float qx0 = __shfl_sync(full, qx, 0);
+    const float q = columns ? qy : qx0 + (float)min(lane - cols, 32 / cols - 1);
+#pragma unroll 1
+    for (int v0 = 0; v0 < nV; v0 += 32) {
+        const int cnt = min(32, nV - v0);
+        const uint2 ev = wt.eval[v0 + min(lane, cnt - 1)];
+        float4 c = T.cen[ev.x];
+        const bool leaf = (int)ev.x >= T.n - 1;
+        const int p = meta_degree(c.w);
+        if (lane < cnt && !leaf) {  // each lane asks for its expansion's lines
+            const float* C = T.coef + meta_offset(c.w);
+#pragma unroll 1
+            for (int e = 0; e < (p + 1) * (p + 1); e += 32) asm volatile("prefetch.global.L2 [%0];" ::"l"(C + e));
+        }
+        if (leaf) c.w = make_meta(0, -1);  // no coefficients
+#pragma unroll 1
+        for (int k = -1; k < cnt; ++k) {
+            if (k + 1 < cnt) {
+                const float next = __shfl_sync(full, c.w, k + 1);
+                const int pn = meta_degree(next);
+                stage(wt.coef[(k + 1) & 1], T.coef + meta_offset(next), pn, (pn + 4) >> 2, lane);
+            }
+            if (k < 0) continue;
+            const unsigned m = __shfl_sync(full, ev.y, k);
+            const float cx = __shfl_sync(full, c.x, k), cy = __shfl_sync(full, c.y, k);
+            const int nb = (meta_degree(__shfl_sync(full, c.w, k)) + 4) >> 2;
+            if (k + 1 < cnt) asm volatile("cp.async.wait_group 1;" ::: "memory");
+            else asm volatile("cp.async.wait_group 0;" ::: "memory");
+            __syncwarp();
+            float w = nb == 0 ? leaf_mass(T, make_float4(cx, cy, 0.0f, 0.0f), qx, qy)
+                              : hermite_tile(wt, wt.coef[k & 1], nb, cols, q, columns ? cy : cx, T.isq, lane);
+            w = ((m >> lane) & 1u) ? w : 0.0f;
+            if (v0 + k < kRows) wt.val[v0 + k][lane] = w;
+            else val_hi[v0 + k - kRows] = w;
+            total = fadd(total, w);
+            __syncwarp();  // the expansion has been read
+        }
+    }
+    __syncwarp();
+    return nV;
+}
+
+// Sum of the listed masses [s, t) of this lane, in order.
+__device__ __forceinline__ float range_sum(const WarpTables& wt, const float* val_hi, int lane, int s, int t) {
+    float acc = 0.0f;
+    int i = s;
+    const int top = min(t, kRows);
+#pragma unroll 1
+    for (; i + 4 <= top; i += 4) {
+        float x0 = wt.val[i][lane], x1 = wt.val[i + 1][lane], x2 = wt.val[i + 2][lane], x3 = wt.val[i + 3][lane];
+        acc = fadd(fadd(fadd(fadd(acc, x0), x1), x2), x3);
+    }
+#pragma unroll 1
+    for (; i < t; ++i) acc = fadd(acc, i < kRows ? wt.val[i][lane] : val_hi[i - kRows]);
+    return acc;
+}
+
+// A lane's place in the tables: an opened node, the range of its expansions
+// and their sum.
+struct Place {
+    int o, s, t;
+    float sum;
+};
+
+// The opened nodes above the first one with two children in the tables: every
+// lane with a mass has the root's mass in each of them and goes through them
+// all.  node: that first one; depth: its depth; path: the choices to it.
+struct Stem {
+    int node, depth;
+    unsigned long long path;
+};
+
+__device__ __forceinline__ Stem find_stem(const WarpTables& wt) {
+    Stem s{0, 0, 0ull};
+#pragma unroll 1
+    while (s.depth < kTrace - 2) {  // uniform over the warp
+        const unsigned links = wt.open[s.node].x, la = links & 0xffffu, lb = links >> 16;
+        const bool left = lb == kLinkNone, right = la == kLinkNone;
+        const unsigned link = left ? la : lb;
+        if (left == right || (link & kLinkKind) != kLinkOpen || (link & kLinkStop)) break;
+        if (right) s.path |= 1ull << s.depth;
+        ++s.depth;
+        s.node = (int)(link & kLinkEntry);
+    }
+    return s;
+}
+
+// The sums of the children's ranges (getWeight of both children); E: the
+// node's entry, m: its split.  A child that holds the whole range has the
+// node's own sum.
+__device__ __forceinline__ void child_sums(const WarpTables& wt, const float* val_hi, int lane, const Place& at, int m,
+                                           float& w0, float& w1) {
+    if (m == at.t) { w0 = at.sum; w1 = 0.0f; }
+    else if (m == at.s) { w0 = 0.0f; w1 = at.sum; }
+    else {
+#pragma unroll 1
+        for (int side = 0; side < 2; ++side) {
+            w0 = w1;
+            w1 = range_sum(wt, val_hi, lane, side ? m : at.s, side ? at.t : m);
+        }
+    }
+}
+
+// The lanes of the next pass: the group of `width` lanes around the first
+// lane of todo.
+__device__ __forceinline__ unsigned lane_group(unsigned todo, int width) {
+    if (width == 32) return todo;
+    return todo & (((1u << width) - 1u) << ((__ffs(todo) - 1) & ~(width - 1)));
 }
 
 // Child masses (w0, w1) = getWeight of the children (a, b) for every lane
@@ -1044,13 +1312,15 @@ __device__ void warp_root_walk(const Tree& T, float qx, float qy, bool live, Mas
 //   instead of two while c <= 16.  `owner`: 32 ints of the warp's shared
 //   memory.
 template <bool SPREAD>
-__device__ __forceinline__ void warp_child_masses(const Tree& T, bool need, int a, int b, float qx, float qy,
-                                                  float& w0, float& w1, int* owner) {
+__device__ __forceinline__ void warp_child_masses(const Tree& T, WarpTables& wt, bool need, int a, int b, float qx,
+                                                  float qy, float& w0, float& w1) {
+    int* owner = wt.owner;
+    const int lane = (threadIdx.x + blockDim.x * threadIdx.y) & 31;
     if (!SPREAD) {
         if (need) {
 #pragma unroll 1
             for (int ch = 0; ch < 2; ++ch) {
-                float x = fmaxf(0.0f, node_weight(T, ch ? b : a, qx, qy));
+                float x = fmaxf(0.0f, lane_series(T, wt, lane, ch ? b : a, qx, qy));
                 if (ch) w1 = x; else w0 = x;
             }
         }
@@ -1059,7 +1329,6 @@ __device__ __forceinline__ void warp_child_masses(const Tree& T, bool need, int 
     const unsigned full = 0xffffffffu;
     unsigned nm = __ballot_sync(full, need);
     if (!nm) return;
-    const int lane = (threadIdx.x + blockDim.x * threadIdx.y) & 31;
     int c = __popc(nm), c2 = 2 * c;
     int rank = __popc(nm & ((1u << lane) - 1u));
     if (need) owner[rank] = lane;
@@ -1072,7 +1341,7 @@ __device__ __forceinline__ void warp_child_masses(const Tree& T, bool need, int 
         float oqx = __shfl_sync(full, qx, o), oqy = __shfl_sync(full, qy, o);
         int oa = __shfl_sync(full, a, o), ob = __shfl_sync(full, b, o);
         float x = 0.0f;
-        if (e < c2) x = fmaxf(0.0f, node_weight(T, right ? ob : oa, oqx, oqy));
+        if (e < c2) x = fmaxf(0.0f, lane_series(T, wt, lane, right ? ob : oa, oqx, oqy));
         int s0 = rank - e0, s1 = c + rank - e0;  // lanes holding this lane's children in this pass
         float x0 = __shfl_sync(full, x, s0 & 31), x1 = __shfl_sync(full, x, s1 & 31);
         if (need && s0 >= 0 && s0 < 32) w0 = x0;
@@ -1080,6 +1349,19 @@ __device__ __forceinline__ void warp_child_masses(const Tree& T, bool need, int 
     }
     __syncwarp();  // owner is rewritten by the next call
 }
+
+constexpr int kKnown = 3;  // nodes outside the tables whose child masses a lane keeps
+
+// Two warps per block: their tables fit the 48 KB of static shared memory,
+// and a block's slot is free again when two tiles are done.  Six blocks per
+// SM fill its shared memory (168 registers per thread).  What bounds the
+// descent is the length of its instruction stream (620 million warp
+// instructions at 500k splats / 1024^2, 0.43 per cycle and scheduler, mostly
+// waiting for the previous instruction); the same algorithm with unrolled
+// loops ran 516 million but took 2.6 ms instead of 1.34, fetching them (187
+// KB of code instead of 54).  500k / 1024^2 / K = 8: 2.7-3.3 ms before these
+// tables, 11 ms where one pixel's cache of 160 nodes overflowed; 1.3 ms now.
+constexpr int kDescentThreads = 64, kDescentBlocks = 6;
 
 // Views of different sizes in one descent launch: blocks [first[v],
 // first[v+1]) of the one-dimensional grid cover view v, bx[v] blocks along
@@ -1093,13 +1375,18 @@ struct UnevenViews {
     long long ioff[kMaxUneven];
 };
 
+// Warps per block: two; one where the lists of more than 16 keys take shared
+// memory (dynamic, 256 K bytes per warp).
+template <int KM>
+constexpr int kDescentWarps = KM <= 16 ? kDescentThreads / 32 : 1;
+
 template <int R, int KM, bool UNEVEN, bool SPREAD>
-__global__ void __launch_bounds__(128, 4) k_sample(Tree T, const ViewState* vs, int W, int H, int K,
-                                                int M, float precision, const float* __restrict__ uniforms,
-                                                uint64_t seed, const uint64_t* __restrict__ seed_ptr,
-                                                uint32_t view, int* __restrict__ indices, uds_view_stats* st,
-                                                size_t vstride, size_t ustride, size_t istride, UnevenViews uv) {
-    // block tile_x (y) x 128 / tile_x (x).  blockIdx.z selects the
+__global__ void __launch_bounds__(32 * kDescentWarps<KM>, KM <= 16 ? kDescentBlocks : 8)
+    k_sample(Tree T, const ViewState* vs, int W, int H, int K, int M, float precision,
+             const float* __restrict__ uniforms, uint64_t seed, const uint64_t* __restrict__ seed_ptr, uint32_t view,
+             int* __restrict__ indices, uds_view_stats* st, size_t vstride, size_t ustride, size_t istride,
+             UnevenViews uv) {
+    // block tile_x (y) x threads / tile_x (x).  blockIdx.z selects the
     // view: its tree lives vstride bytes after the previous view's, its
     // uniforms ustride floats and its indices istride entries further on.
     // With UNEVEN the view and the block's place in it come from uv
@@ -1134,7 +1421,8 @@ __global__ void __launch_bounds__(128, 4) k_sample(Tree T, const ViewState* vs, 
         }
         st += vz;
     }
-    __shared__ WalkStack s_walk[4];
+    __shared__ WarpTables s_tables[kDescentWarps<KM>];
+    extern __shared__ uint2 list[];  // K > 16: (key, id) in order, one column per lane
     const unsigned full = 0xffffffffu;
     int j = bxi * blockDim.x + threadIdx.x;
     int i = byi * blockDim.y + threadIdx.y;
@@ -1147,164 +1435,287 @@ __global__ void __launch_bounds__(128, 4) k_sample(Tree T, const ViewState* vs, 
     if (T.n == 0) return;  // indices were preset to -1 (uniform over the grid)
     size_t pixel = (size_t)j + (size_t)H * i;
     float qx = (float)i, qy = (float)j;
-    MassCache mc;
-    float total;
-    warp_root_walk(T, qx, qy, live, mc, total, s_walk[warp]);
-    int* ws_owner = s_walk[warp].right;  // free once the walk is done
-    total = fmaxf(0.0f, total);
-    bool act = live && !(total < precision);
-    if (!__any_sync(full, act)) return;
+    WarpTables& wt = s_tables[warp];
+    float val_hi[kEvals - kRows];
     // K-sized arrays stay in registers for K <= 16 (loops fully unrolled)
     constexpr int UK = KM <= 16 ? KM : 1;
-    int ids[KM];
-    float keys[KM];
+    unsigned todo = __ballot_sync(full, live);
+    int width = 32;
+    while (todo) {
+        const unsigned group = lane_group(todo, width);
+        float total;
+        const int state = warp_tables(T, qx, qy, group, M, blockDim.x, wt, val_hi, total);
+        if (state < 0 && width > 1) {
+            width >>= 1;
+            continue;
+        }
+        todo &= ~group;
+        const bool mine = (group >> lane) & 1u;
+        if (state < 0 && mine) total = node_weight_out_of_line(T, 0, qx, qy);
+        const Place root{0, 0, state, total};
+        total = fmaxf(0.0f, total);
+        bool act = mine && !(total < precision);
+        if (!__any_sync(full, act)) continue;
+        constexpr int KR = KM <= 16 ? KM : 1;
+        int ids[KR];
+        float keys[KR];
+        float last = __int_as_float(0x7f800000);  // K > 16: the list's largest key once it is full
+        int have = 0;                             // and its length
+        if (KM <= 16) {
 #pragma unroll UK
-    for (int k = 0; k < KM; ++k) { ids[k] = -1; keys[k] = __int_as_float(0x7f800000); }
-    // each round's path is kept as its choice bits (bit m: right child taken
-    // at depth m) and its length, in registers: two rounds meet the same node
-    // at depth m iff their first m choices agree (node ids are unique)
-    unsigned long long pb[R];
-    float tc[R][kTrace];
-    float tp[kTrace];
-    int tl[R];
+            for (int k = 0; k < KR; ++k) { ids[k] = -1; keys[k] = __int_as_float(0x7f800000); }
+        }
+        // each round's path as its choice bits (bit m: right child taken at depth
+        // m): two rounds meet the same node at depth m iff their first m choices
+        // agree (node ids are unique)
+        unsigned long long pb[R];
 #pragma unroll
-    for (int rr = 0; rr < R; ++rr) { pb[rr] = 0ull; tl[rr] = 0; }
-    // child masses of the node met at each depth by the latest round; slots
-    // [0, cvn) are valid (depths are reached in order, so no clearing needed)
-    int cv[kTrace];
-    float cw0[kTrace], cw1[kTrace];
-    int cvn = 0;
-    bool overflow = false;
-    for (int r = 0; r < R; ++r) {
-        int v = 0, d = 0;
-        const int2 no_rec = no_record();
-        int2 rc = (mc.ok && mc.m > 0) ? mc.rec[0] : no_rec;  // cache record of v
-        unsigned long long cur = 0ull;                        // this round's choice bits so far
-        tp[0] = 1.0f;
-        int4 L = T.lnk[0];
-        bool going = act && L.w > M;
-        while (__any_sync(full, going)) {
-            int a = L.x, b = L.y;
-            float w0 = 0.0f, w1 = 0.0f;
-            int2 ra = no_rec, rb = no_rec;  // the children's records
-            bool need = false;
-            if (going) {
-                int ia = rec_left(rc), ib = rec_right(rc);
-                if (ia != kNotWalked) {
-                    if (ia >= 0) { ra = mc.rec[ia]; w0 = fmaxf(0.0f, rec_mass(ra)); }
-                    if (ib >= 0) { rb = mc.rec[ib]; w1 = fmaxf(0.0f, rec_mass(rb)); }
-                } else if (d < cvn && cv[d] == v) {
-                    w0 = cw0[d];
-                    w1 = cw1[d];
-                } else {
-                    need = true;
-                }
+        for (int rr = 0; rr < R; ++rr) pb[rr] = 0ull;
+        // per depth >= 1 the path's node's share of its parent's mass and, by
+        // round, its capacity: the first levels below the stem in wt.path, the
+        // others in local memory
+        float far_rows[R * kTrace];
+        float* far = far_rows;
+        asm volatile("" : "+l"(far));  // stays an array in memory
+        constexpr int kNear = kPathRows / R;  // levels in wt.path, R rows each: the share, R - 1 capacities
+        // child masses of the last nodes met outside the tables
+        int kv[kKnown];
+        float kw0[kKnown], kw1[kKnown];
+#pragma unroll
+        for (int q = 0; q < kKnown; ++q) { kv[q] = -1; kw0[q] = 0.0f; kw1[q] = 0.0f; }
+        bool overflow = false;
+        // A node of the stem gives its one child its whole mass, so the child's
+        // capacity is always the node's: one number, cap, for the whole stem, and
+        // a round starts at the stem's end.  Once it is used up (cap = 0) a round
+        // starts at the root instead: where neither child has anything left it
+        // goes left, off the stem if need be.  The rounds below `quick` started
+        // at the stem's end.
+        const Stem stem = state > 0 ? find_stem(wt) : Stem{0, 0, 0ull};
+        float cap = 1.0f;
+        int quick = 0;
+        const int near0 = stem.depth + 1;
+        auto capacity = [&](int rr, int d) {
+            const int q = d - near0;
+            return q >= 0 && q < kNear ? wt.path[R * q + 1 + rr][lane] : far[R * d + 1 + rr];
+        };
+        auto set_capacity = [&](int rr, int d, float x) {
+            const int q = d - near0;
+            if (q >= 0 && q < kNear) wt.path[R * q + 1 + rr][lane] = x;
+            else far[R * d + 1 + rr] = x;
+        };
+#pragma unroll 1
+        for (int r = 0; r < R; ++r) {
+            int d = 0;
+            Place at = root;                // place in the tables (o < 0: outside), or
+            if (state <= 0) at.o = -1;
+            int v = 0;                      // the node itself and its links
+            int4 L = T.lnk[0];
+            unsigned long long cur = 0ull;  // this round's choice bits so far
+            unsigned with = (1u << r) - 1u; // earlier rounds that have come the same way so far
+            bool going = act && L.w > M, pend = false;
+            const bool skip = state > 0 && cap > 0.0f && total < __int_as_float(0x7f800000);
+            if (skip) {
+                d = stem.depth;
+                cur = stem.path;
+                at.o = stem.node;
+                quick = r + 1;
             }
-            // every lane that needs its node's child masses gets them in the
-            // same pass, whatever node it is at (below the expansion frontier
-            // a child is one expansion, so the divergence is only in the
-            // series' trip counts); one call site keeps the walk inlined once,
-            // small enough for the instruction cache
-            warp_child_masses<SPREAD>(T, need, a, b, qx, qy, w0, w1, ws_owner);
-            if (going) {
-                // (re)write unconditionally: a hit stores the same masses, and
-                // a store does not wait on the per-thread memory like a load
-                cv[d] = v;
-                cw0[d] = w0;
-                cw1[d] = w1;
-                if (d >= cvn) cvn = d + 1;
-                float sum = fadd(fadd(0.0f, w0), w1);
-                w0 = fdiv(w0, sum);
-                w1 = fdiv(w1, sum);
-                // capacities of a and b: from the latest earlier round whose
-                // path passed through v (same first d choices) into that child
-                float c0 = 1.0f, c1 = 1.0f;
-                bool f0 = false, f1 = false;
-                unsigned long long pre = (1ull << d) - 1ull;
+            // lanes go down the tables on their own; a lane that needs child
+            // masses evaluated waits until no other lane can go on, so that the
+            // evaluations of a round are made in as few passes as possible
+            while (true) {
+                float w0 = 0.0f, w1 = 0.0f, sum0 = 0.0f, sum1 = 0.0f;
+                uint4 E = make_uint4(0u, 0u, 0u, 0u);
+                int split = 0;
+                if (going && !pend) {
+                    if (at.o >= 0) {
+                        E = wt.open[at.o];
+                        split = wt.split[at.o];
+                        child_sums(wt, val_hi, lane, at, split, sum0, sum1);
+                        w0 = fmaxf(0.0f, sum0);
+                        w1 = fmaxf(0.0f, sum1);
+                    } else {
+                        pend = true;
 #pragma unroll
-                for (int rr = R - 1; rr >= 0; --rr) {
-                    if (rr < r && d + 1 < tl[rr] && ((pb[rr] ^ cur) & pre) == 0ull) {
-                        bool right = (pb[rr] >> d) & 1ull;
-                        if (!right && !f0) { c0 = tc[rr][d + 1]; f0 = true; }
-                        if (right && !f1) { c1 = tc[rr][d + 1]; f1 = true; }
+                        for (int q = 0; q < kKnown; ++q)
+                            if (kv[q] == v) { w0 = kw0[q]; w1 = kw1[q]; pend = false; }
                     }
                 }
-                float s0 = fmul(w0, c0), s1 = fmul(w1, c1);
-                ++d;
-                if (d >= kTrace) {
-                    overflow = true;
-                    going = false;
-                    act = false;
-                } else {
-                    if (s0 < s1) { cur |= 1ull << (d - 1); tp[d] = w1; v = b; rc = rb; }
-                    else { tp[d] = w0; v = a; rc = ra; }
-                    L = T.lnk[v];
-                    going = L.w > M;
+                bool can = going && !pend;
+                if (!__any_sync(full, can)) {
+                    if (!__any_sync(full, pend)) break;
+                    warp_child_masses<SPREAD>(T, wt, pend, L.x, L.y, qx, qy, w0, w1);
+                    can = pend;
+                    pend = false;
+                    if (can) {
+#pragma unroll
+                        for (int q = kKnown - 1; q > 0; --q) {
+                            kv[q] = kv[q - 1];
+                            kw0[q] = kw0[q - 1];
+                            kw1[q] = kw1[q - 1];
+                        }
+                        kv[0] = v;
+                        kw0[0] = w0;
+                        kw1[0] = w1;
+                    }
+                }
+                if (can) {
+                    // the children's shares; w / w = 1: many nodes above the
+                    // pixel have one child that its circle reaches
+                    float sum = fadd(fadd(0.0f, w0), w1);
+                    if ((w0 == 0.0f) != (w1 == 0.0f) && sum < __int_as_float(0x7f800000)) {
+                        w0 = w0 == 0.0f ? 0.0f : 1.0f;
+                        w1 = w1 == 0.0f ? 0.0f : 1.0f;
+                    } else {
+                        w0 = fdiv(w0, sum);
+                        w1 = fdiv(w1, sum);
+                    }
+                    // capacities of the children: from the latest earlier round
+                    // whose path passed through this node into that child
+                    float c0 = 1.0f, c1 = 1.0f;
+                    unsigned into0 = 0u, into1 = 0u;
+                    if (with) {
+#pragma unroll
+                        for (int rr = 0; rr < R - 1; ++rr) into1 |= (unsigned)((pb[rr] >> d) & 1ull) << rr;
+                        into1 &= with;
+                        into0 = with & ~into1;
+                        if (into0 && d + 1 < kTrace) {
+                            const int rr = 31 - __clz(into0);
+                            c0 = rr < quick && d < stem.depth ? cap : capacity(rr, d + 1);
+                        }
+                        if (into1 && d + 1 < kTrace) {
+                            const int rr = 31 - __clz(into1);
+                            c1 = rr < quick && d < stem.depth ? cap : capacity(rr, d + 1);
+                        }
+                    }
+                    const bool right = fmul(w0, c0) < fmul(w1, c1);
+                    with = right ? into1 : into0;
+                    ++d;
+                    if (d >= kTrace) {
+                        overflow = true;
+                        going = false;
+                        act = false;
+                    } else {
+                        if (right) cur |= 1ull << (d - 1);
+                        if (r < R - 1) {
+                            const int q = d - near0;
+                            if (q >= 0 && q < kNear) wt.path[R * q][lane] = right ? w1 : w0;
+                            else far[R * d] = right ? w1 : w0;
+                            set_capacity(r, d, right ? c1 : c0);
+                        }
+                        bool through = false;  // on to an opened child of the tables
+                        unsigned link = 0u;
+                        if (at.o >= 0) {
+                            v = (int)(right ? E.z : E.y);
+                            link = right ? E.x >> 16 : E.x & 0xffffu;
+                            through = (link & kLinkKind) == kLinkOpen &&
+                                      ((wt.open[link & kLinkEntry].w >> lane) & 1u);
+                        } else {
+                            v = right ? L.y : L.x;
+                        }
+                        if (through && !(link & kLinkStop)) {
+                            at.o = (int)(link & kLinkEntry);
+                            at.sum = right ? sum1 : sum0;
+                            if (right) at.s = split; else at.t = split;
+                        } else {
+                            at.o = -1;
+                            L = T.lnk[v];
+                            going = L.w > M;
+                        }
+                    }
                 }
             }
-        }
-        if (!act) continue;
+            if (!act) continue;
 #pragma unroll
-        for (int rr = 0; rr < R; ++rr)
-            if (rr == r) { pb[rr] = cur; tl[rr] = d + 1; }
-        float prob = 1.0f;
-        for (int m = d; m >= 0; --m) {
-            float cap = 1.0f;
-            bool found = false;
-            unsigned long long pre = (1ull << m) - 1ull;
-#pragma unroll
-            for (int rr = R - 1; rr >= 0; --rr)
-                if (rr < r && !found && m < tl[rr] && ((pb[rr] ^ cur) & pre) == 0ull) { cap = tc[rr][m]; found = true; }
-            tc[r][m] = fmaxf(0.0f, fsub(cap, prob));
-            prob = fmul(prob, tp[m]);
-        }
-        // order sampling over the subtree's leaves (insertSample,
-        // sequentialPoissonRadixTree.cuh:15-41); a leaf's mass is its own
-        // Gaussian (degree 0, coefficient 1).  The subtree holds at most M
-        // leaves: K, or the leaf size when that is larger.
-        int f0 = L.z, cnt = L.w;
-        // the round's uniforms, drawn as the leaves use them (after the
-        // descent, so they hold no registers there): Philox block
-        // (pixel, view, r * ceil(M / 4) + k / 4), or the caller's tensor
-        const float* up = uniforms ? uniforms + ((size_t)pixel * R + r) * M : nullptr;
-        const int G = (M + 3) >> 2;
-        uint32_t c4[4];
+            for (int rr = 0; rr < R; ++rr)
+                if (rr == r) pb[rr] = cur;
+            // the path's capacities shrink by the probability of the part below
+            // (no later round looks at the last one's)
+            if (r < R - 1) {
+                float prob = 1.0f;
+                const int top = skip ? stem.depth : 0;
 #pragma unroll 1
-        for (int k0 = 0; k0 < cnt; k0 += 4) {
-            if (!up) {
-                c4[0] = (uint32_t)pixel; c4[1] = view; c4[2] = (uint32_t)(r * G + (k0 >> 2)); c4[3] = 0u;
-                philox4x32_10(c4, (uint32_t)seed, (uint32_t)(seed >> 32));
+                for (int m = d; m > top; --m) {
+                    const int q = m - near0;
+                    set_capacity(r, m, fmaxf(0.0f, fsub(capacity(r, m), prob)));
+                    prob = fmul(prob, q >= 0 && q < kNear ? wt.path[R * q][lane] : far[R * m]);
+                }
+                if (skip) cap = fmaxf(0.0f, fsub(cap, prob));
             }
-#pragma unroll
-            for (int k4 = 0; k4 < 4; ++k4) {
-                int k = k0 + k4;
-                if (k < cnt) {
-                    float uk = up ? up[k] : bits_to_uniform(c4[k4]);
-                    int leafNode = T.n - 1 + f0 + k;
-                    float pw = fmaxf(0.0f, leaf_mass(T, T.cen[leafNode], qx, qy));
-                    float key = fdiv(uk, pw);
-                    int index = T.leaf_id[f0 + k];
-                    bool done = false;
+            // order sampling over the subtree's leaves (insertSample,
+            // sequentialPoissonRadixTree.cuh:15-41); a leaf's mass is its own
+            // Gaussian (degree 0, coefficient 1).  The subtree holds at most M
+            // leaves: K, or the leaf size when that is larger.
+            int f0 = L.z, cnt = L.w;
+            // the round's uniforms, drawn as the leaves use them (after the
+            // descent, so they hold no registers there): Philox block
+            // (pixel, view, r * ceil(M / 4) + k / 4), or the caller's tensor
+            const float* up = uniforms ? uniforms + ((size_t)pixel * R + r) * M : nullptr;
+            const int G = (M + 3) >> 2;
+            uint32_t c4[4];
+            float2 xy = T.leaf_xy[f0];
+            int id = T.leaf_id[f0];
+#pragma unroll 1
+            for (int k = 0; k < cnt; ++k) {
+                if (!up && (k & 3) == 0) {
+                    c4[0] = (uint32_t)pixel; c4[1] = view; c4[2] = (uint32_t)(r * G + (k >> 2)); c4[3] = 0u;
+                    philox4x32_10(c4, (uint32_t)seed, (uint32_t)(seed >> 32));
+                }
+                const uint32_t bits = (k & 2) ? ((k & 1) ? c4[3] : c4[2]) : ((k & 1) ? c4[1] : c4[0]);
+                float uk = up ? up[k] : bits_to_uniform(bits);
+                float pw = fmaxf(0.0f, leaf_mass(T, make_float4(xy.x, xy.y, 0.0f, 0.0f), qx, qy));
+                float key = fdiv(uk, pw);
+                int index = id;
+                if (k + 1 < cnt) {  // the next leaf's record on its way
+                    xy = T.leaf_xy[f0 + k + 1];
+                    id = T.leaf_id[f0 + k + 1];
+                }
+                {
+                    {
+                        // the K smallest keys in order, the earlier candidate
+                        // first among equals (an infinite or NaN key never enters)
+                        if (KM <= 16) {
+                            if (key < keys[KR - 1]) {
 #pragma unroll UK
-                    for (int q = 0; q < KM; ++q) {
-                        if (!done && q < K) {
-                            if (key < keys[q]) {
-                                int ti = ids[q]; ids[q] = index; index = ti;
-                                float tk = keys[q]; keys[q] = key; key = tk;
+                                for (int q = 0; q < KR; ++q) {
+                                    bool lt = key < keys[q];
+                                    float tk = keys[q];
+                                    int ti = ids[q];
+                                    keys[q] = lt ? key : tk;
+                                    ids[q] = lt ? index : ti;
+                                    key = lt ? tk : key;
+                                    index = lt ? ti : index;
+                                }
                             }
-                            if (index == -1) done = true;
+                        } else if (key < last) {
+                            int q = have < K ? have++ : K - 1;
+#pragma unroll 1
+                            while (q > 0) {
+                                uint2 x = list[(q - 1) * 32 + lane];
+                                if (!(__uint_as_float(x.x) > key)) break;
+                                list[q * 32 + lane] = x;
+                                --q;
+                            }
+                            list[q * 32 + lane] = make_uint2(__float_as_uint(key), (unsigned)index);
+                            if (have == K) last = __uint_as_float(list[(K - 1) * 32 + lane].x);
                         }
                     }
                 }
             }
         }
-    }
-    if (overflow) atomicAdd(&st->overflow, 1);
-    if (!live) return;
-    int* out = indices + (size_t)K * pixel;
+        if (overflow) atomicAdd(&st->overflow, 1);
+        if (mine) {
+            int* out = indices + (size_t)K * pixel;
+            if (KM <= 16) {
 #pragma unroll UK
-    for (int k = 0; k < KM; ++k)
-        if (k < K) out[k] = ids[k];
+                for (int k = 0; k < KR; ++k)
+                    if (k < K) out[k] = ids[k];
+            } else {
+#pragma unroll 1
+                for (int k = 0; k < K; ++k) out[k] = k < have ? (int)list[k * 32 + lane].y : -1;
+            }
+        }
+    }
 }
 
 // Stochastic mode (no reference counterpart).  Each of the K draws of a
@@ -1317,7 +1728,7 @@ __global__ void __launch_bounds__(128, 4) k_sample(Tree T, const ViewState* vs, 
 // their upper paths, so the child masses of the last path are kept per depth
 // (node ids are unique, so a hit is exact).  A draw that meets two zero
 // masses, or is still above the leaves after kTrace levels, stays -1 / 0.
-__global__ void __launch_bounds__(128, 4) k_stochastic(Tree T, const ViewState* vs, int W, int H, int K,
+__global__ void __launch_bounds__(kDescentThreads, kDescentBlocks) k_stochastic(Tree T, const ViewState* vs, int W, int H, int K,
                                                        float precision, uint64_t seed,
                                                        const uint64_t* __restrict__ seed_ptr, uint32_t view,
                                                        int* __restrict__ indices, float* __restrict__ probs,
@@ -1329,12 +1740,12 @@ __global__ void __launch_bounds__(128, 4) k_stochastic(Tree T, const ViewState* 
     // direct evaluation by each lane that needs them (all bit-identical to
     // separate getWeight calls)
     if (seed_ptr) seed = *seed_ptr;
-    __shared__ WalkStack s_walk[4];
+    __shared__ WarpTables s_tables[kDescentThreads / 32];
     const unsigned full = 0xffffffffu;
     int j = blockIdx.x * blockDim.x + threadIdx.x;
     int i = blockIdx.y * blockDim.y + threadIdx.y;
     int tid = threadIdx.x + blockDim.x * threadIdx.y;
-    int warp = tid >> 5;
+    int warp = tid >> 5, lane = tid & 31;
     size_t pixel = (size_t)j + (size_t)H * i;
     bool live = (i < W && j < H) && (!mask || mask[pixel]);
     T.n = vs->n;
@@ -1343,84 +1754,147 @@ __global__ void __launch_bounds__(128, 4) k_stochastic(Tree T, const ViewState* 
     int n = T.n;
     if (n == 0) return;
     float qx = (float)i, qy = (float)j;
-    MassCache mc;
-    float m0;
-    warp_root_walk(T, qx, qy, live, mc, m0, s_walk[warp]);
-    m0 = fmaxf(0.0f, m0);
-    bool act = live && !(m0 < precision);
-    if (!__any_sync(full, act)) return;
-    int cv[kTrace];
-    float cw0[kTrace], cw1[kTrace];
-    int cvn = 0;
+    WarpTables& wt = s_tables[warp];
+    float val_hi[kEvals - kRows];
     bool overflow = false;
-    for (int k = 0; k < K; ++k) {
-        int v = 0, d = 0;
-        const int2 no_rec = no_record();
-        int2 rc = (mc.ok && mc.m > 0) ? mc.rec[0] : no_rec;
-        float prob = 1.0f;
-        uint32_t c[4];
-        bool ok = act;
-        int4 L = T.lnk[0];
-        bool going = act && v < n - 1;
-        while (__any_sync(full, going)) {
-            int a = L.x, b = L.y;
-            float w0 = 0.0f, w1 = 0.0f;
-            int2 ra = no_rec, rb = no_rec;  // the children's records
-            int4 La = L, Lb = L;            // and links, loaded with them
-            bool need = false;
-            if (going) {
-                La = T.lnk[a];
-                Lb = T.lnk[b];
-                int ia = rec_left(rc), ib = rec_right(rc);
-                if (ia != kNotWalked) {
-                    if (ia >= 0) { ra = mc.rec[ia]; w0 = fmaxf(0.0f, rec_mass(ra)); }
-                    if (ib >= 0) { rb = mc.rec[ib]; w1 = fmaxf(0.0f, rec_mass(rb)); }
-                } else if (d < cvn && cv[d] == v) {
-                    w0 = cw0[d];
-                    w1 = cw1[d];
-                } else {
-                    need = true;
-                }
+    unsigned todo = __ballot_sync(full, live);
+    int width = 32;
+    while (todo) {
+        const unsigned group = lane_group(todo, width);
+        float m0;
+        const int state = warp_tables(T, qx, qy, group, 1, blockDim.x, wt, val_hi, m0);
+        if (state < 0 && width > 1) {
+            width >>= 1;
+            continue;
+        }
+        todo &= ~group;
+        const bool mine = (group >> lane) & 1u;
+        if (state < 0 && mine) m0 = node_weight_out_of_line(T, 0, qx, qy);
+        const Place root{0, 0, state, m0};
+        m0 = fmaxf(0.0f, m0);
+        bool act = mine && !(m0 < precision);
+        if (!__any_sync(full, act)) continue;
+        // child masses of the node last met at each depth outside the tables
+        // (bit d of cvalid: slot d is set): the first levels from the stem on in
+        // wt.path, three rows each, the others in local memory
+        constexpr int kNear = kPathRows / 3;
+        int cv_far[kTrace];
+        float cw0_far[kTrace], cw1_far[kTrace];
+        unsigned long long cvalid = 0ull;
+        const Stem stem = state > 0 ? find_stem(wt) : Stem{0, 0, 0ull};
+        for (int k = 0; k < K; ++k) {
+            int d = 0;
+            Place at = root;
+            if (state <= 0) at.o = -1;
+            int v = 0;
+            int4 L = T.lnk[0];
+            float prob = 1.0f;
+            uint32_t c[4];
+            bool ok = act;
+            bool going = act && n > 1, pend = false, first = true;
+            // on the stem the branch with the mass has probability 1
+            if (state > 0 && m0 < __int_as_float(0x7f800000)) {
+                d = stem.depth;
+                at.o = stem.node;
             }
-            // every lane that needs its node's child masses gets them in the
-            // same pass (one call site: the walk is inlined once)
-            warp_child_masses<false>(T, need, a, b, qx, qy, w0, w1, s_walk[warp].right);
-            if (going) {
-                cv[d] = v;
-                cw0[d] = w0;
-                cw1[d] = w1;
-                if (d >= cvn) cvn = d + 1;
-                if ((d & 3) == 0) {
-                    c[0] = (uint32_t)pixel; c[1] = view; c[2] = 0x80000000u | ((uint32_t)k << 8) | (uint32_t)(d >> 2);
-                    c[3] = 0;
-                    philox4x32_10(c, (uint32_t)seed, (uint32_t)(seed >> 32));
+            while (true) {
+                float w0 = 0.0f, w1 = 0.0f, sum0 = 0.0f, sum1 = 0.0f;
+                uint4 E = make_uint4(0u, 0u, 0u, 0u);
+                int split = 0;
+                if (going && !pend) {
+                    if (at.o >= 0) {
+                        E = wt.open[at.o];
+                        split = wt.split[at.o];
+                        child_sums(wt, val_hi, lane, at, split, sum0, sum1);
+                        w0 = fmaxf(0.0f, sum0);
+                        w1 = fmaxf(0.0f, sum1);
+                    } else {
+                        pend = true;
+                        const int q = d - stem.depth;
+                        if ((cvalid >> d) & 1ull) {
+                            if (q >= 0 && q < kNear) {
+                                pend = __float_as_int(wt.path[3 * q][lane]) != v;
+                                w0 = wt.path[3 * q + 1][lane];
+                                w1 = wt.path[3 * q + 2][lane];
+                            } else {
+                                pend = cv_far[d] != v;
+                                w0 = cw0_far[d];
+                                w1 = cw1_far[d];
+                            }
+                        }
+                    }
                 }
-                float u = bits_to_uniform(c[d & 3]);
-                float sum = fadd(fadd(0.0f, w0), w1);
-                if (!(sum > 0.0f)) {
-                    ok = false;
-                    going = false;
-                } else {
-                    float r0 = fdiv(w0, sum);
-                    if (u <= r0) { prob = fmul(prob, r0); v = a; rc = ra; L = La; }
-                    else { prob = fmul(prob, fdiv(w1, sum)); v = b; rc = rb; L = Lb; }
-                    ++d;
-                    if (d >= kTrace && v < n - 1) {
+                bool can = going && !pend;
+                if (!__any_sync(full, can)) {
+                    if (!__any_sync(full, pend)) break;
+                    warp_child_masses<false>(T, wt, pend, L.x, L.y, qx, qy, w0, w1);
+                    can = pend;
+                    pend = false;
+                    if (can) {
+                        const int q = d - stem.depth;
+                        if (q >= 0 && q < kNear) {
+                            wt.path[3 * q][lane] = __int_as_float(v);
+                            wt.path[3 * q + 1][lane] = w0;
+                            wt.path[3 * q + 2][lane] = w1;
+                        } else {
+                            cv_far[d] = v;
+                            cw0_far[d] = w0;
+                            cw1_far[d] = w1;
+                        }
+                        cvalid |= 1ull << d;
+                    }
+                }
+                if (can) {
+                    if ((d & 3) == 0 || first) {
+                        first = false;
+                        c[0] = (uint32_t)pixel; c[1] = view; c[2] = 0x80000000u | ((uint32_t)k << 8) | (uint32_t)(d >> 2);
+                        c[3] = 0;
+                        philox4x32_10(c, (uint32_t)seed, (uint32_t)(seed >> 32));
+                    }
+                    float u = bits_to_uniform(c[d & 3]);
+                    float sum = fadd(fadd(0.0f, w0), w1);
+                    if (!(sum > 0.0f)) {
                         ok = false;
-                        overflow = true;
                         going = false;
                     } else {
-                        going = v < n - 1;
+                        float r0 = fdiv(w0, sum);
+                        bool right = !(u <= r0);
+                        prob = fmul(prob, right ? fdiv(w1, sum) : r0);
+                        bool through = false;
+                        unsigned link = 0u;
+                        if (at.o >= 0) {
+                            v = (int)(right ? E.z : E.y);
+                            link = right ? E.x >> 16 : E.x & 0xffffu;
+                            through = (link & kLinkKind) == kLinkOpen &&
+                                      ((wt.open[link & kLinkEntry].w >> lane) & 1u);
+                        } else {
+                            v = right ? L.y : L.x;
+                        }
+                        if (through) {  // an opened node is not a leaf
+                            at.o = (int)(link & kLinkEntry);
+                            at.sum = right ? sum1 : sum0;
+                            if (right) at.s = split; else at.t = split;
+                        } else {
+                            at.o = -1;
+                            going = v < n - 1;
+                            if (going) L = T.lnk[v];
+                        }
+                        ++d;
+                        if (d >= kTrace && going) {
+                            ok = false;
+                            overflow = true;
+                            going = false;
+                        }
                     }
                 }
             }
-        }
-        if (ok) {
-            size_t o = (size_t)K * pixel + k;
-            indices[o] = T.leaf_id[v - (n - 1)];
-            probs[o] = prob;
-            // importance weight of the draw: (leaf mass / root mass) / q
-            if (weights) weights[o] = leaf_mass(T, T.cen[v], qx, qy) / m0 / prob;
+            if (ok) {
+                size_t o = (size_t)K * pixel + k;
+                indices[o] = T.leaf_id[v - (n - 1)];
+                probs[o] = prob;
+                // importance weight of the draw: (leaf mass / root mass) / q
+                if (weights) weights[o] = leaf_mass(T, T.cen[v], qx, qy) / m0 / prob;
+            }
         }
     }
     if (overflow) atomicAdd(&st->overflow, 1);
@@ -1532,16 +2006,17 @@ __global__ void __launch_bounds__(128) k_prop_dataset(Tree T, const ViewState* v
 }
 
 // Per pixel: root mass; active pixels put their K draws on the list.
-__global__ void k_prop_init(Tree T, const ViewState* vs, int W, int H, int K, float precision,
+__global__ void __launch_bounds__(kDescentThreads, kDescentBlocks) k_prop_init(Tree T, const ViewState* vs, int W, int H, int K, float precision,
                             float* __restrict__ root_mass, int* __restrict__ node_out, int* __restrict__ draw_out,
                             float* __restrict__ logq_out, int* __restrict__ count_out, int* __restrict__ indices,
                             float* __restrict__ weights) {
-    // root masses by the warp-cooperative walk of k_sample (128-thread
-    // blocks, warps of consecutive threads)
-    __shared__ WalkStack s_walk[4];
+    // root masses from the tables of k_sample (warps of consecutive
+    // threads)
+    __shared__ WarpTables s_tables[kDescentThreads / 32];
     int j = blockIdx.x * blockDim.x + threadIdx.x;
     int i = blockIdx.y * blockDim.y + threadIdx.y;
-    int warp = (threadIdx.x + blockDim.x * threadIdx.y) >> 5;
+    int tid = threadIdx.x + blockDim.x * threadIdx.y;
+    int warp = tid >> 5, lane = tid & 31;
     bool live = i < W && j < H;
     T.n = vs->n;
     T.sq = vs->sq;
@@ -1550,8 +2025,20 @@ __global__ void k_prop_init(Tree T, const ViewState* vs, int W, int H, int K, fl
     float qx = (float)i, qy = (float)j;
     float m0 = 0.0f;
     if (T.n > 0) {
-        MassCache mc;
-        warp_root_walk(T, qx, qy, live, mc, m0, s_walk[warp]);
+        float val_hi[kEvals - kRows];
+        unsigned todo = __ballot_sync(0xffffffffu, live);
+        int width = 32;
+        while (todo) {
+            const unsigned group = lane_group(todo, width);
+            float total;
+            const int state = warp_tables(T, qx, qy, group, 1, blockDim.x, s_tables[warp], val_hi, total);
+            if (state < 0 && width > 1) {
+                width >>= 1;
+                continue;
+            }
+            todo &= ~group;
+            if ((group >> lane) & 1u) m0 = state < 0 ? node_weight_out_of_line(T, 0, qx, qy) : total;
+        }
         m0 = fmaxf(0.0f, m0);
     }
     if (!live) return;
@@ -1763,6 +2250,10 @@ static int build_view(const uds_sample_params* p, const Ws& w, int view, const f
 // node holding at most max(K, leaf_size) splats.
 static int candidates(const uds_sample_params* p) { return p->leaf_size > p->K ? p->leaf_size : p->K; }
 
+// Columns of the warp tile: 4 or 8 (wider tiles share fewer row sums: at 16
+// the descent took a third longer, so 16 and 32 run as 8).
+static int tile_of(const uds_sample_params* p) { return p->tile_x == 4 ? 4 : 8; }
+
 static Tree tree_of(const Ws& w) {
     Tree T;
     T.lnk = w.lnk; T.par = w.par; T.box = w.box; T.cen = w.cen; T.coef = w.coef;
@@ -1773,13 +2264,13 @@ static Tree tree_of(const Ws& w) {
 template <int R>
 // Descent for views view .. view + nviews - 1 in one launch (grid.z = view),
 // their trees vstride bytes apart in the workspace.
-// Block: 128 threads, tile_x (y) by 128 / tile_x (x) pixels; each warp is a
+// Block: tile_x (y) by kDescentThreads / tile_x (x) pixels; each warp is a
 // tile_x by 32 / tile_x pixel tile.  Every lane's walk is its own, so the
 // indices do not depend on the tile shape, only the speed does.
 static void launch_sample(const Tree& T, const Ws& w, const uds_sample_params* p, const float* u, int view,
                           int* idx, cudaStream_t s, int nviews = 1, size_t vstride = 0) {
-    int tx = p->tile_x > 0 ? p->tile_x : 8;
-    dim3 block(tx, 128 / tx);
+    int tx = tile_of(p);
+    dim3 block(tx, kDescentThreads / tx);
     dim3 grid(cdiv(p->H, block.x), cdiv(p->W, block.y), nviews);
     size_t istride = (size_t)p->W * p->H * p->K;
     const int M = candidates(p);
@@ -1796,7 +2287,11 @@ static void launch_sample(const Tree& T, const Ws& w, const uds_sample_params* p
                                                                  p->seed, p->seed_dev, (uint32_t)view, idx,
                                                                  w.stats + view, vstride, ustride, istride, none);
     } else {
-        k_sample<(R >= 3 ? R : 3), kMaxK, false, false><<<grid, block, 0, s>>>(
+        // the K smallest keys in registers up to 16, in shared memory above
+        constexpr int RR = R >= 3 ? R : 3, KM = RR <= 4 ? 16 : kMaxK;
+        dim3 block(tx, 32 * kDescentWarps<KM> / tx);
+        dim3 grid(cdiv(p->H, block.x), cdiv(p->W, block.y), nviews);
+        k_sample<RR, KM, false, true><<<grid, block, KM <= 16 ? 0 : 256 * (size_t)p->K, s>>>(
             T, w.vs, p->W, p->H, p->K, M, p->precision, u, p->seed, p->seed_dev, (uint32_t)view, idx,
             w.stats + view, vstride, ustride, istride, none);
     }
@@ -1807,8 +2302,8 @@ static void launch_sample(const Tree& T, const Ws& w, const uds_sample_params* p
 template <int R>
 static void launch_sample_uneven(const Tree& T, const Ws& w, const uds_sample_params* p, const UnevenViews& uv,
                                  int* idx, cudaStream_t s, size_t vstride) {
-    int tx = p->tile_x > 0 ? p->tile_x : 8;
-    dim3 block(tx, 128 / tx);
+    int tx = tile_of(p);
+    dim3 block(tx, kDescentThreads / tx);
     if (p->spread)
         k_sample<R, 8, true, true><<<uv.first[uv.nv], block, 0, s>>>(T, w.vs, 0, 0, p->K, candidates(p), p->precision,
                                                                      nullptr, p->seed, p->seed_dev, 0u, idx, w.stats,
@@ -2001,7 +2496,7 @@ extern "C" int uds_sample_views(const uds_sample_params* prm, const uds_view_des
     if (prm->N > 0) {
         Tree T = tree_of(w);
         int R = num_rounds(prm->K);
-        int tx = prm->tile_x > 0 ? prm->tile_x : 8;
+        int tx = tile_of(prm);
         if (prm->K <= 8 && prm->B <= kMaxUneven) {
             UnevenViews uv{};
             uv.nv = prm->B;
@@ -2013,7 +2508,7 @@ extern "C" int uds_sample_views(const uds_sample_params* prm, const uds_view_des
                 uv.W[b] = views[b].W;
                 uv.H[b] = views[b].H;
                 uv.ioff[b] = off;
-                blocks += uv.bx[b] * (int)cdiv(views[b].W, 128 / tx);
+                blocks += uv.bx[b] * (int)cdiv(views[b].W, kDescentThreads / tx);
                 off += (long long)views[b].W * views[b].H * prm->K;
             }
             uv.first[prm->B] = blocks;
@@ -2069,7 +2564,7 @@ extern "C" int uds_sample_stochastic(const uds_sample_params* prm, const float* 
     if (e == cudaSuccess) e = cudaMemsetAsync(probs, 0, sizeof(float) * per_view * prm->B, s);
     if (e != cudaSuccess) { set_last_error(e); return UDS_ERR_CUDA; }
     Tree T = tree_of(w);
-    dim3 block(8, 16);
+    dim3 block(8, kDescentThreads / 8);
     dim3 grid(cdiv(prm->H, block.x), cdiv(prm->W, block.y));
     for (int b = 0; b < prm->B; ++b) {
         if ((st = build_view(prm, w, b, points, normals, std_devs, h_override, s))) return st;
@@ -2237,7 +2732,7 @@ extern "C" int uds_sample_proposal(const uds_sample_params* prm, const float* po
     if (e == cudaSuccess && n_fallback) e = cudaMemsetAsync(n_fallback, 0, sizeof(int32_t) * prm->B, s);
     if (e != cudaSuccess) { set_last_error(e); return UDS_ERR_CUDA; }
     Tree T = tree_of(w);
-    dim3 block(16, 8);
+    dim3 block(8, kDescentThreads / 8);
     dim3 grid(cdiv(prm->H, block.x), cdiv(prm->W, block.y));
     for (int b = 0; b < prm->B; ++b) {
         if ((st = build_view(prm, w, b, points, normals, std_devs, h_override, s))) return st;
@@ -2248,7 +2743,7 @@ extern "C" int uds_sample_proposal(const uds_sample_params* prm, const float* po
         if (mlp_params) {
             e = cudaMemsetAsync(q.counts, 0, 16, s);
             if (e != cudaSuccess) { set_last_error(e); return UDS_ERR_CUDA; }
-            k_prop_init<<<dim3(cdiv(prm->H, 8), cdiv(prm->W, 16)), dim3(8, 16), 0, s>>>(T, w.vs, prm->W, prm->H, prm->K, prm->precision, q.root_mass,
+            k_prop_init<<<grid, block, 0, s>>>(T, w.vs, prm->W, prm->H, prm->K, prm->precision, q.root_mass,
                                                q.node[0], q.draw[0], q.logq[0], q.counts, idx, wt);
             if ((st = launch_status())) return st;
             unsigned nb = cdiv(per_view, 256);
