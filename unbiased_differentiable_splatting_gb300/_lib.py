@@ -158,6 +158,22 @@ def load(build_if_missing: bool = True):
     return _lib
 
 
+_ops_loaded = False
+
+
+def load_ops() -> None:
+    """Load libuds_torch.so (the native CUDA implementations of torch.ops.uds),
+    building it in-tree first when it is missing."""
+    global _ops_loaded
+    load()
+    with _lock:
+        if not _ops_loaded:
+            if not os.path.exists(_build.OPS_LIB):
+                _build.build()
+            torch.ops.load_library(_build.OPS_LIB)
+            _ops_loaded = True
+
+
 class UdsError(RuntimeError):
     pass
 

@@ -12,6 +12,10 @@ the reference's post-processing of their gradient (norm clamp, NaN scrub,
 dropped normal gradient), which ``extensions.EWASplatting`` and the renderer
 use.
 
+For CUDA tensors the implementations and autograd formulas of most ops are
+replaced by the same ones in native code (csrc/uds_torch.cpp, loaded at the
+end of this module): an eager call then runs no Python below the op.
+
 Schemas use the reference's argument order; names are snake_case
 (``splat_forward`` for ``splatting.forward``).
 """
@@ -22,6 +26,7 @@ from typing import List, Optional, Tuple
 import torch
 from torch import Tensor
 
+from . import _lib, training
 from .cudaExtensions import (filtering, interpolation, nearestsamples, pixelgather, sampling, shading, splatting,
                              transform)
 
@@ -545,8 +550,62 @@ def _(nearest, points, normals, sigma, mean):
     return points.new_empty((2,)), torch.empty_like(points), torch.empty_like(normals)
 
 
+# ------------------------------------- losses with their gradients inside
+@_op("uds::nearest_losses", mutates_args=())
+def nearest_losses(points: Tensor, normals: Tensor, nearest: Tensor, sigma: float,
+                   mean: bool) -> Tuple[Tensor, Tensor, Tensor, Tensor]:
+    """(normal loss, plane loss) of nearest_regularizer and their gradients
+    w.r.t. points and normals; differentiable, the gradients are constants."""
+    losses, gp, gn = nearestsamples.regularizer(nearest, points, normals, sigma, mean)
+    return losses[0], losses[1].clone(), gp, gn
+
+
+@nearest_losses.register_fake
+def _(points, normals, nearest, sigma, mean):
+    return points.new_empty(()), points.new_empty(()), torch.empty_like(points), torch.empty_like(normals)
+
+
+def _nearest_losses_setup(ctx, inputs, output):
+    ctx.mark_non_differentiable(output[2], output[3])
+    ctx.save_for_backward(output[2], output[3])
+
+
+def _nearest_losses_grad(ctx, g_normal, g_plane, _gp, _gn):
+    gp, gn = ctx.saved_tensors
+    return gp * g_plane, gn * g_normal, None, None, None
+
+
+nearest_losses.register_autograd(_nearest_losses_grad, setup_context=_nearest_losses_setup)
+
+
+@_op("uds::image_loss", mutates_args=())
+def image_loss(image: Tensor, target: Tensor, kind: int, scale: float) -> Tuple[Tensor, Tensor]:
+    """L1 (kind 0) or L2 (kind 1) image loss and its gradient w.r.t. the
+    image; differentiable, the gradient is a constant."""
+    return training.image_loss(image, target, kind, scale)
+
+
+@image_loss.register_fake
+def _(image, target, kind, scale):
+    return image.new_empty(()), torch.empty_like(image)
+
+
+def _image_loss_setup(ctx, inputs, output):
+    ctx.mark_non_differentiable(output[1])
+    ctx.save_for_backward(output[1])
+
+
+def _image_loss_grad(ctx, g, _grad):
+    return ctx.saved_tensors[0] * g, None, None, None
+
+
+image_loss.register_autograd(_image_loss_grad, setup_context=_image_loss_setup)
+
+
 OPS = ("sample", "sample_views", "splat_forward", "splat_backward", "ewa_weights", "render_splats", "render_splats_backward", "filter_forward", "filter_backward", "interp_forward",
        "interp_backward", "affine_forward", "affine_backward", "linear_forward", "linear_backward",
        "view_matrix_forward", "view_matrix_backward", "backface", "backface_backward", "shade_forward", "shade_backward", "shade_sh_forward",
        "shade_sh_backward", "lambert_forward", "lambert_backward", "pixel_scatter", "pixel_gather", "nearest",
-       "nearest_regularizer")
+       "nearest_regularizer", "nearest_losses", "image_loss")
+
+_lib.load_ops()

@@ -16,23 +16,10 @@ from __future__ import annotations
 
 import torch as th
 
+from . import library  # noqa: F401  (registers torch.ops.uds)
 from .cudaExtensions import nearestsamples
 
 REDUCTIONS = ("sum", "mean")
-
-
-class _NearestLosses(th.autograd.Function):
-    @staticmethod
-    def forward(ctx, points, normals, nearest, sigma, mean):
-        losses, gp, gn = nearestsamples.regularizer(nearest, points.detach().contiguous(),
-                                                    normals.detach().contiguous(), sigma, mean)
-        ctx.save_for_backward(gp, gn)
-        return losses[0], losses[1]
-
-    @staticmethod
-    def backward(ctx, g_normal, g_plane):
-        gp, gn = ctx.saved_tensors
-        return gp * g_plane, gn * g_normal, None, None, None
 
 
 class NearestSamplesRegularizer(th.nn.Module):
@@ -52,4 +39,6 @@ class NearestSamplesRegularizer(th.nn.Module):
         with th.no_grad():
             nearest = self.nearest(indices, weights.detach().contiguous(), points.detach().contiguous(),
                                    self.num_nearest)
-        return _NearestLosses.apply(points, normals, nearest, float(self.sigma), self.reduction == "mean")
+        normal, plane, _, _ = th.ops.uds.nearest_losses(points.contiguous(), normals.contiguous(), nearest,
+                                                        float(self.sigma), self.reduction == "mean")
+        return normal, plane

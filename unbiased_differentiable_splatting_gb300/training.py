@@ -11,22 +11,15 @@ import torch as th
 from ._lib import check, load, need, ptr, stream_ptr
 
 
-class _FusedImageLoss(th.autograd.Function):
-    @staticmethod
-    def forward(ctx, kind, scale, x, y):
-        x = need(x.contiguous(), "image")
-        y = need(y.contiguous(), "target", device=x.device)
-        loss = th.empty((), device=x.device)
-        grad = th.empty_like(x)
-        check(load().uds_image_loss(kind, x.numel(), ptr(x), ptr(y), float(scale), ptr(loss), ptr(grad),
-                                    stream_ptr(x.device)), "image loss")
-        ctx.save_for_backward(grad)
-        return loss
-
-    @staticmethod
-    def backward(ctx, g):
-        (grad,) = ctx.saved_tensors
-        return None, None, grad * g, None
+def image_loss(x, y, kind, scale):
+    """(loss, gradient w.r.t. x) of the L1 (kind 0) or L2 (kind 1) image loss."""
+    x = need(x, "image")
+    y = need(y, "target", device=x.device)
+    loss = th.empty((), device=x.device)
+    grad = th.empty_like(x)
+    check(load().uds_image_loss(kind, x.numel(), ptr(x), ptr(y), float(scale), ptr(loss), ptr(grad),
+                                stream_ptr(x.device)), "image loss")
+    return loss, grad
 
 
 class _ImageLoss(th.nn.Module):
@@ -36,11 +29,12 @@ class _ImageLoss(th.nn.Module):
         super().__init__()
         if reduction not in ("mean", "sum"):
             raise ValueError("Unkown reduction mode")
+        from . import library  # noqa: F401  (registers torch.ops.uds; it imports this module)
         self.reduction = reduction
 
     def forward(self, x, y):
         scale = 1.0 / x.numel() if self.reduction == "mean" else 1.0
-        return _FusedImageLoss.apply(self.kind, scale, x, y), None
+        return th.ops.uds.image_loss(x.contiguous(), y.contiguous(), self.kind, scale)[0], None
 
 
 class L1ImageLoss(_ImageLoss):
