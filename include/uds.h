@@ -333,6 +333,13 @@ int uds_splat_backward(int B, int W, int H, int K, float focal, const float* gra
                        int std_batch, int N, const float* std_devs, float smoothing,
                        float* grad_points, float* grad_normals, float* grad_std_devs,
                        void* workspace, size_t workspace_bytes, void* stream);
+/* The same with the reference's post-processing of point and std-dev
+ * gradients (see uds_render_fused_gradients), none of the normals. */
+int uds_splat_gradients(int B, int W, int H, int K, float focal, const float* grad,
+                       const int32_t* indices, const float* points, const float* normals,
+                       int std_batch, int N, const float* std_devs, float smoothing,
+                       float* grad_points, float* grad_std_devs,
+                       void* workspace, size_t workspace_bytes, void* stream);
 
 /* ---- The shading pass of Splatting.forward (render.py:268-376, the chain
  *      splattingCuda.cu:18-66 -> zSortingCuda.cu:11-62 ->
@@ -356,6 +363,16 @@ int uds_render_fused_backward(int B, int W, int H, int K, float focal, const flo
                               const float* weights, const float* points, const float* normals, int std_batch, int N,
                               const float* std_devs, float smoothing, int aB, int C, const float* attribute,
                               float* grad_points, float* grad_normals, float* grad_std_devs, float* grad_attribute,
+                              void* workspace, size_t workspace_bytes, void* stream);
+/* The same for an optimiser: gradients of points and std-devs with the
+ * reference's post-processing (rows scaled to norm <= 1, NaNs 0:
+ * conditionalNormalization, splatting/extensions/utils.py:147-150), none of
+ * the normals. */
+int uds_render_fused_gradients(int B, int W, int H, int K, float focal, const float* grad_image,
+                              const float* grad_depth_weights, const float* grad_weights, const int32_t* indices,
+                              const float* weights, const float* points, const float* normals, int std_batch, int N,
+                              const float* std_devs, float smoothing, int aB, int C, const float* attribute,
+                              float* grad_points, float* grad_std_devs, float* grad_attribute,
                               void* workspace, size_t workspace_bytes, void* stream);
 
 /* splatting.forward without a workspace, for callers that cannot allocate

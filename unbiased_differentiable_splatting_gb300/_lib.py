@@ -60,6 +60,10 @@ _SIGS = {
                                           c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_void_p, c_float,
                                           c_int, c_int, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p,
                                           c_size_t, c_void_p]),
+    "uds_render_fused_gradients": (c_int, [c_int, c_int, c_int, c_int, c_float, c_void_p, c_void_p, c_void_p,
+                                           c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_void_p, c_float,
+                                           c_int, c_int, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_size_t,
+                                           c_void_p]),
     "uds_sample_workspace_size": (c_size_t, [ctypes.POINTER(SampleParams)]),
     "uds_sample": (c_int, [ctypes.POINTER(SampleParams), c_void_p, c_void_p, c_void_p, c_void_p, c_void_p,
                            c_void_p, c_void_p, c_void_p, c_size_t, c_void_p]),
@@ -110,6 +114,9 @@ _SIGS = {
     "uds_splat_backward": (c_int, [c_int, c_int, c_int, c_int, c_float, c_void_p, c_void_p, c_void_p,
                                    c_void_p, c_int, c_int, c_void_p, c_float, c_void_p, c_void_p, c_void_p,
                                    c_void_p, c_size_t, c_void_p]),
+    "uds_splat_gradients": (c_int, [c_int, c_int, c_int, c_int, c_float, c_void_p, c_void_p, c_void_p,
+                                    c_void_p, c_int, c_int, c_void_p, c_float, c_void_p, c_void_p, c_void_p, c_size_t,
+                                    c_void_p]),
     "uds_splat_forward_static": (c_int, [c_int, c_int, c_int, c_int, c_float, c_void_p, c_void_p, c_void_p,
                                          c_int, c_int, c_void_p, c_float, c_void_p, c_void_p]),
     "uds_filter_forward": (c_int, [c_int, c_int, c_int, c_int, c_void_p, c_void_p, c_float, c_int, c_int,

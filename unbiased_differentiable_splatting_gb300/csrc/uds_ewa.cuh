@@ -4,6 +4,7 @@
 #pragma once
 #include "uds_common.cuh"
 #include "uds_backproject.cuh"
+#include "uds_nearfloat.cuh"
 
 namespace uds {
 
@@ -17,14 +18,23 @@ __device__ __forceinline__ void screen_point(float W, float H, float f, const fl
     s[1] = add_via_double(fdiv(fmul(p[1], f), p[2]), fmul(H, 0.5f));
 }
 
-// backproject (double arithmetic, rounded to float): the same numbers from
-// the exact integer quotient where it applies, else the double sequence
-__device__ __forceinline__ void back_project(float W, float H, float f, const float* s, float* x) {
+// backproject (double arithmetic, rounded to float): the same numbers in
+// float arithmetic, or near a rounding boundary from the exact integer
+// quotient, or else from the double sequence
+__device__ __forceinline__ float back_project_one(float W, float s, float f, float rf) {
     float q;
-    if (bp_quotient(fmul(W, 0.5f), s[0], f, &q)) x[0] = q;
-    else x[0] = (float)ddiv(dsub((double)W, dmul(2.0, (double)s[0])), dmul(2.0, (double)f));
-    if (bp_quotient(fmul(H, 0.5f), s[1], f, &q)) x[1] = -q;
-    else x[1] = (float)ddiv(-dsub((double)H, dmul(2.0, (double)s[1])), dmul(2.0, (double)f));
+    const float a = fmul(W, 0.5f);
+    if (near_quotient(a, s, f, rf, &q) || bp_quotient(a, s, f, &q)) return q;
+    return (float)ddiv(dsub((double)W, dmul(2.0, (double)s)), dmul(2.0, (double)f));
+}
+__device__ __forceinline__ void back_project(float W, float H, float f, const float* s, float* x) {
+    const float rf = fdiv(1.0f, f);
+#pragma unroll 1
+    for (int i = 0; i < 2; ++i) {
+        const float q = back_project_one(i ? H : W, s[i], f, rf);
+        if (i) x[1] = -q;
+        else x[0] = q;
+    }
     x[2] = 1.0f;
 }
 

@@ -34,7 +34,8 @@ using OptTensor = std::optional<Tensor>;
 // ------------------------------------------------------------------ checks
 const Tensor& need(const Tensor& t, const char* name, const Tensor* like = nullptr, at::ScalarType type = at::kFloat) {
     TORCH_CHECK_VALUE(t.is_cuda(), name, " must be a CUDA tensor");
-    if (like) TORCH_CHECK_VALUE(t.device() == like->device(), name, " is on ", t.device(), ", expected ", like->device());
+    if (like)
+        TORCH_CHECK_VALUE(t.device() == like->device(), name, " is on ", t.device(), ", expected ", like->device());
     TORCH_CHECK_TYPE(t.scalar_type() == type, name, " must be ", type == at::kInt ? "torch.int32" : "torch.float32",
                      ", got ", t.scalar_type());
     TORCH_CHECK_VALUE(t.is_contiguous(), name, " must be contiguous");
@@ -255,6 +256,11 @@ using RenderFwd = std::tuple<Tensor, Tensor, Tensor>(SymInt, SymInt, double, con
 using RenderBwd = std::vector<Tensor>(SymInt, SymInt, double, const Tensor&, const OptTensor&, const OptTensor&,
                                       const Tensor&, const Tensor&, const Tensor&, const Tensor&, const Tensor&, double,
                                       const Tensor&);
+using SplatGrads = std::tuple<Tensor, Tensor>(SymInt, SymInt, double, const Tensor&, const Tensor&, const Tensor&,
+                                              const Tensor&, const Tensor&, double);
+using RenderGrads = std::tuple<Tensor, Tensor, Tensor>(SymInt, SymInt, double, const Tensor&, const OptTensor&,
+                                                       const OptTensor&, const Tensor&, const Tensor&, const Tensor&,
+                                                       const Tensor&, const Tensor&, double, const Tensor&);
 
 void check_splats(const Tensor& ids, const Tensor& pts, const Tensor& nrm, const Tensor& sd) {
     need(ids, "indices", nullptr, at::kInt);
@@ -297,6 +303,22 @@ std::tuple<Tensor, Tensor, Tensor> splat_backward_cuda(int64_t, int64_t, double 
           "splatting backward");
     return {gp, gn, gs};
 }
+std::tuple<Tensor, Tensor> splat_gradients_cuda(int64_t, int64_t, double focal, const Tensor& g, const Tensor& ids,
+                                                const Tensor& pts, const Tensor& nrm, const Tensor& sd,
+                                                double smoothing) {
+    check_splats(ids, pts, nrm, sd);
+    need(g, "gradIn", &pts);
+    TORCH_CHECK_VALUE(g.sizes() == ids.sizes(), "gradIn must match indices");
+    const int B = i32(ids.size(0)), N = i32(pts.size(1));
+    On on(pts);
+    Tensor ws = scratch(uds_splat_workspace_size(B, N), pts);
+    Tensor gp = at::empty_like(pts), gs = at::empty_like(sd);
+    check(uds_splat_gradients(B, i32(ids.size(1)), i32(ids.size(2)), i32(ids.size(3)), (float)focal, f(g), idx(ids),
+                              f(pts), f(nrm), i32(sd.size(0)), N, f(sd), (float)smoothing, fm(gp), fm(gs),
+                              ws.mutable_data_ptr(), (size_t)ws.numel(), on.stream()),
+          "splatting backward");
+    return {gp, gs};
+}
 std::tuple<Tensor, Tensor, Tensor> render_forward_cuda(int64_t width, int64_t height, double focal, const Tensor& ids,
                                                        const Tensor& pts, const Tensor& nrm, const Tensor& sd,
                                                        double smoothing, const Tensor& attr) {
@@ -317,9 +339,12 @@ std::tuple<Tensor, Tensor, Tensor> render_forward_cuda(int64_t width, int64_t he
           "render forward");
     return {img, depth, w};
 }
-std::vector<Tensor> render_backward_cuda(int64_t, int64_t, double focal, const Tensor& gimg, const OptTensor& gdepth,
-                                         const OptTensor& gw, const Tensor& ids, const Tensor& w, const Tensor& pts,
-                                         const Tensor& nrm, const Tensor& sd, double smoothing, const Tensor& attr) {
+// CLAMP: render_splats_gradients ({points, std-devs, attribute} with the
+// reference's post-processing), else the raw gradients.
+template <bool CLAMP>
+std::vector<Tensor> render_gradients(double focal, const Tensor& gimg, const OptTensor& gdepth, const OptTensor& gw,
+                                     const Tensor& ids, const Tensor& w, const Tensor& pts, const Tensor& nrm,
+                                     const Tensor& sd, double smoothing, const Tensor& attr) {
     check_splats(ids, pts, nrm, sd);
     need(gimg, "gradImage", &pts);
     need(w, "weights", &pts);
@@ -336,21 +361,38 @@ std::vector<Tensor> render_backward_cuda(int64_t, int64_t, double focal, const T
                       "gradImage must be (B,W,H,C) and weights (B,W,H,K)");
     On on(pts);
     Tensor ws = scratch(uds_splat_workspace_size(B, N), pts);
-    Tensor gp = at::empty_like(pts), gn = at::empty_like(nrm), gs = at::empty_like(sd), ga = at::empty_like(attr);
-    check(uds_render_fused_backward(B, i32(ids.size(1)), i32(ids.size(2)), i32(ids.size(3)), (float)focal, f(gimg),
-                                    fo(gdepth), fo(gw), idx(ids), f(w), f(pts), f(nrm), i32(sd.size(0)), N, f(sd),
-                                    (float)smoothing, i32(attr.size(0)), C, f(attr), fm(gp), fm(gn), fm(gs), fm(ga),
-                                    ws.mutable_data_ptr(), (size_t)ws.numel(), on.stream()),
-          "render backward");
-    return {gp, gn, gs, ga};
+    Tensor gp = at::empty_like(pts), gs = at::empty_like(sd), ga = at::empty_like(attr);
+    if constexpr (CLAMP) {
+        check(uds_render_fused_gradients(B, i32(ids.size(1)), i32(ids.size(2)), i32(ids.size(3)), (float)focal, f(gimg),
+                                         fo(gdepth), fo(gw), idx(ids), f(w), f(pts), f(nrm), i32(sd.size(0)), N, f(sd),
+                                         (float)smoothing, i32(attr.size(0)), C, f(attr), fm(gp), fm(gs), fm(ga),
+                                         ws.mutable_data_ptr(), (size_t)ws.numel(), on.stream()),
+              "render backward");
+        return {gp, gs, ga};
+    } else {
+        Tensor gn = at::empty_like(nrm);
+        check(uds_render_fused_backward(B, i32(ids.size(1)), i32(ids.size(2)), i32(ids.size(3)), (float)focal, f(gimg),
+                                        fo(gdepth), fo(gw), idx(ids), f(w), f(pts), f(nrm), i32(sd.size(0)), N, f(sd),
+                                        (float)smoothing, i32(attr.size(0)), C, f(attr), fm(gp), fm(gn), fm(gs), fm(ga),
+                                        ws.mutable_data_ptr(), (size_t)ws.numel(), on.stream()),
+              "render backward");
+        return {gp, gn, gs, ga};
+    }
+}
+std::vector<Tensor> render_backward_cuda(int64_t, int64_t, double focal, const Tensor& gimg, const OptTensor& gdepth,
+                                         const OptTensor& gw, const Tensor& ids, const Tensor& w, const Tensor& pts,
+                                         const Tensor& nrm, const Tensor& sd, double smoothing, const Tensor& attr) {
+    return render_gradients<false>(focal, gimg, gdepth, gw, ids, w, pts, nrm, sd, smoothing, attr);
+}
+std::tuple<Tensor, Tensor, Tensor> render_gradients_cuda(int64_t, int64_t, double focal, const Tensor& gimg,
+                                                         const OptTensor& gdepth, const OptTensor& gw,
+                                                         const Tensor& ids, const Tensor& w, const Tensor& pts,
+                                                         const Tensor& nrm, const Tensor& sd, double smoothing,
+                                                         const Tensor& attr) {
+    auto r = render_gradients<true>(focal, gimg, gdepth, gw, ids, w, pts, nrm, sd, smoothing, attr);
+    return {r[0], r[1], r[2]};
 }
 
-// The reference's post-processing of the EWA gradients (conditionalNormali-
-// zation and the NaN scrub), see ewa_weights in library.py.
-Tensor post(const Tensor& g) {
-    const double inf = std::numeric_limits<double>::infinity();
-    return at::nan_to_num(g / at::clamp_min(g.norm(2, {-1}, true) + 1e-4, 1.0), 0.0, inf, -inf);
-}
 void save_view(AutogradContext* ctx, const SymInt& width, const SymInt& height, double focal, double smoothing) {
     ctx->saved_data["width"] = width;
     ctx->saved_data["height"] = height;
@@ -373,11 +415,17 @@ struct SplatFn : Function<SplatFn<RAW>> {
     static variable_list backward(AutogradContext* ctx, variable_list g) {
         auto s = ctx->get_saved_variables();
         auto& d = ctx->saved_data;
-        static auto call = op<SplatBwd>("uds::splat_backward");
-        auto [gp, gn, gs] = call.call(d["width"].toSymInt(), d["height"].toSymInt(), d["focal"].toDouble(),
+        if constexpr (RAW) {
+            static auto call = op<SplatBwd>("uds::splat_backward");
+            auto [gp, gn, gs] = call.call(d["width"].toSymInt(), d["height"].toSymInt(), d["focal"].toDouble(),
+                                          g[0].contiguous(), s[0], s[1], s[2], s[3], d["smoothing"].toDouble());
+            return {Tensor(), Tensor(), Tensor(), Tensor(), gp, gn, gs, Tensor()};
+        } else {
+            static auto call = op<SplatGrads>("uds::splat_gradients");
+            auto [gp, gs] = call.call(d["width"].toSymInt(), d["height"].toSymInt(), d["focal"].toDouble(),
                                       g[0].contiguous(), s[0], s[1], s[2], s[3], d["smoothing"].toDouble());
-        if (RAW) return {Tensor(), Tensor(), Tensor(), Tensor(), gp, gn, gs, Tensor()};
-        return {Tensor(), Tensor(), Tensor(), Tensor(), post(gp), Tensor(), post(gs), Tensor()};
+            return {Tensor(), Tensor(), Tensor(), Tensor(), gp, Tensor(), gs, Tensor()};
+        }
     }
     static Tensor autograd(SymInt width, SymInt height, double focal, const Tensor& ids, const Tensor& pts,
                            const Tensor& nrm, const Tensor& sd, double smoothing) {
@@ -408,10 +456,11 @@ struct RenderFn : Function<RenderFn> {
         Tensor gimg = g[0].defined() ? g[0].contiguous()
                                      : at::zeros_symint({s[0].sym_size(0), s[0].sym_size(1), s[0].sym_size(2),
                                                          s[4].sym_size(2)}, s[5].options());
-        static auto call = op<RenderBwd>("uds::render_splats_backward");
-        auto r = call.call(d["width"].toSymInt(), d["height"].toSymInt(), d["focal"].toDouble(), gimg, opt(g[1]),
-                           opt(g[2]), s[0], s[5], s[1], s[2], s[3], d["smoothing"].toDouble(), s[4]);
-        return {Tensor(), Tensor(), Tensor(), Tensor(), post(r[0]), Tensor(), post(r[2]), Tensor(), r[3]};
+        static auto call = op<RenderGrads>("uds::render_splats_gradients");
+        auto [gp, gs, ga] = call.call(d["width"].toSymInt(), d["height"].toSymInt(), d["focal"].toDouble(), gimg,
+                                      opt(g[1]), opt(g[2]), s[0], s[5], s[1], s[2], s[3], d["smoothing"].toDouble(),
+                                      s[4]);
+        return {Tensor(), Tensor(), Tensor(), Tensor(), gp, Tensor(), gs, Tensor(), ga};
     }
 };
 std::tuple<Tensor, Tensor, Tensor> render_autograd(SymInt width, SymInt height, double focal, const Tensor& ids,
@@ -816,7 +865,9 @@ TORCH_LIBRARY_IMPL(uds, CUDA, m) {
     m.impl("splat_forward", splat_forward_cuda);
     m.impl("ewa_weights", splat_forward_cuda);
     m.impl("splat_backward", splat_backward_cuda);
+    m.impl("splat_gradients", splat_gradients_cuda);
     m.impl("render_splats", render_forward_cuda);
+    m.impl("render_splats_gradients", render_gradients_cuda);
     m.impl("render_splats_backward", render_backward_cuda);
     m.impl("filter_forward", filter_forward_cuda);
     m.impl("filter_backward", filter_backward_cuda);
@@ -852,7 +903,8 @@ TORCH_LIBRARY_IMPL(uds, AutogradCUDA, m) {
     // no formula: a graph through these fails in its backward pass, as with
     // the Python definitions
     for (const char* name : {"sample", "sample_views", "affine_backward", "linear_backward", "view_matrix_backward",
-                             "backface_backward", "splat_backward", "render_splats_backward", "filter_backward",
+                             "backface_backward", "splat_backward", "splat_gradients", "render_splats_backward",
+                             "render_splats_gradients", "filter_backward",
                              "interp_backward", "shade_backward", "shade_sh_backward", "lambert_backward",
                              "pixel_gather", "nearest", "nearest_regularizer"})
         m.impl(name, torch::autograd::autogradNotImplementedFallback());

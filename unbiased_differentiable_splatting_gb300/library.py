@@ -130,13 +130,29 @@ def _clamp_rows(dx: Tensor, eps: float = 1e-4) -> Tensor:
     return dx / torch.clamp(dx.norm(dim=-1, keepdim=True) + eps, 1.0)
 
 
+def _post(g: Tensor) -> Tensor:
+    return torch.nan_to_num(_clamp_rows(g), nan=0.0, posinf=float("inf"), neginf=float("-inf"))
+
+
+@_op("uds::splat_gradients", mutates_args=())
+def splat_gradients(width: int, height: int, focallength: float, gradIn: Tensor, indices: Tensor, points: Tensor,
+                    normals: Tensor, stdDevs: Tensor, smoothing: float) -> Tuple[Tensor, Tensor]:
+    """Gradients of ewa_weights: points and std-devs of splat_backward with
+    the reference's post-processing."""
+    gp, _, gs = splatting.backward(width, height, focallength, gradIn, indices, points, normals, stdDevs, smoothing)
+    return _post(gp), _post(gs)
+
+
+@splat_gradients.register_fake
+def _(width, height, focallength, gradIn, indices, points, normals, stdDevs, smoothing):
+    return torch.empty_like(points), torch.empty_like(stdDevs)
+
+
 def _ewa_grad(ctx, grad):
     indices, points, normals, stdDevs = ctx.saved_tensors
     width, height, focallength, smoothing = ctx.args
-    gp, _, gs = torch.ops.uds.splat_backward(width, height, focallength, grad.contiguous(), indices, points, normals,
-                                             stdDevs, smoothing)
-    gp = torch.nan_to_num(_clamp_rows(gp), nan=0.0, posinf=float("inf"), neginf=float("-inf"))
-    gs = torch.nan_to_num(_clamp_rows(gs), nan=0.0, posinf=float("inf"), neginf=float("-inf"))
+    gp, gs = torch.ops.uds.splat_gradients(width, height, focallength, grad.contiguous(), indices, points, normals,
+                                           stdDevs, smoothing)
     return None, None, None, None, gp, None, gs, None
 
 
@@ -179,6 +195,24 @@ def _(width, height, focallength, gradImage, gradDepthWeights, gradWeights, indi
     return [torch.empty_like(t) for t in (points, normals, stdDevs, attribute)]
 
 
+@_op("uds::render_splats_gradients", mutates_args=())
+def render_splats_gradients(width: int, height: int, focallength: float, gradImage: Tensor,
+                            gradDepthWeights: Optional[Tensor], gradWeights: Optional[Tensor], indices: Tensor,
+                            weights: Tensor, points: Tensor, normals: Tensor, stdDevs: Tensor, smoothing: float,
+                            attribute: Tensor) -> Tuple[Tensor, Tensor, Tensor]:
+    """Gradients of render_splats: points and std-devs with the reference's
+    post-processing, attribute."""
+    gp, _, gs, ga = splatting.renderBackward(width, height, focallength, gradImage, gradDepthWeights, gradWeights,
+                                             indices, weights, points, normals, stdDevs, smoothing, attribute)
+    return _post(gp), _post(gs), ga
+
+
+@render_splats_gradients.register_fake
+def _(width, height, focallength, gradImage, gradDepthWeights, gradWeights, indices, weights, points, normals,
+      stdDevs, smoothing, attribute):
+    return torch.empty_like(points), torch.empty_like(stdDevs), torch.empty_like(attribute)
+
+
 def _render_setup(ctx, inputs, output):
     width, height, focallength, indices, points, normals, stdDevs, smoothing, attribute = inputs
     ctx.save_for_backward(indices, points, normals, stdDevs, attribute, output[2])
@@ -192,11 +226,9 @@ def _render_grad(ctx, g_image, g_depth, g_weights):
     if g_image is None:
         g_image = weights.new_zeros(ctx.image_shape)
     c = lambda t: None if t is None else t.contiguous()  # noqa: E731
-    gp, _, gs, ga = torch.ops.uds.render_splats_backward(width, height, focallength, g_image.contiguous(),
-                                                         c(g_depth), c(g_weights), indices, weights, points,
-                                                         normals, stdDevs, smoothing, attribute)
-    gp = torch.nan_to_num(_clamp_rows(gp), nan=0.0, posinf=float("inf"), neginf=float("-inf"))
-    gs = torch.nan_to_num(_clamp_rows(gs), nan=0.0, posinf=float("inf"), neginf=float("-inf"))
+    gp, gs, ga = torch.ops.uds.render_splats_gradients(width, height, focallength, g_image.contiguous(), c(g_depth),
+                                                       c(g_weights), indices, weights, points, normals, stdDevs,
+                                                       smoothing, attribute)
     return None, None, None, None, gp, None, gs, None, ga
 
 
@@ -606,6 +638,6 @@ OPS = ("sample", "sample_views", "splat_forward", "splat_backward", "ewa_weights
        "interp_backward", "affine_forward", "affine_backward", "linear_forward", "linear_backward",
        "view_matrix_forward", "view_matrix_backward", "backface", "backface_backward", "shade_forward", "shade_backward", "shade_sh_forward",
        "shade_sh_backward", "lambert_forward", "lambert_backward", "pixel_scatter", "pixel_gather", "nearest",
-       "nearest_regularizer", "nearest_losses", "image_loss")
+       "nearest_regularizer", "nearest_losses", "image_loss", "splat_gradients", "render_splats_gradients")
 
 _lib.load_ops()
