@@ -882,9 +882,6 @@ constexpr int kLevels = 64;               // a radix tree over 62-bit keys is at
 // Per-lane records of the descent in shared memory: local memory that is
 // written and read back costs an L2 round trip here (about 700 cycles).
 constexpr int kPathRows = 32;
-// 65536 / S rounded up: e * kReciprocal[S] >> 16 = e / S for e < S * S
-__constant__ unsigned kReciprocal[21] = {0,    65536, 32768, 21846, 16384, 13108, 10923, 9363, 8192, 7282, 6554,
-                                         5958, 5462,  5042,  4682,  4370,  4096,  3856,  3641, 3450, 3277};
 constexpr int kSide = 20;                 // Hermite functions and coefficients per side (17, in blocks of four)
 
 // A child's link: kind, stop bit (the child holds at most M splats), entry
@@ -921,18 +918,33 @@ struct WarpTables {
 // Blocks of four coefficients per side of a degree-p expansion.
 __device__ __forceinline__ int coef_blocks(int p) { return (p + 4) >> 2; }
 
-// Starts the copy of an expansion's coefficients to dst, a square of 4 nb per
-// side: (p + 1) x (p + 1) coefficients, zeros past them.
-__device__ __forceinline__ void stage(float* dst, const float* __restrict__ C, int p, int nb, int lane) {
-    const int S = 4 * nb, P1 = p + 1;
-    const unsigned rec = kReciprocal[S];
-    unsigned to = (unsigned)__cvta_generic_to_shared(dst) + 4u * (unsigned)lane;
-#pragma unroll 1
-    for (int e = lane; e < S * S; e += 32, to += 128u) {
-        const int row = (int)((unsigned)e * rec >> 16), col = e - row * S;
-        const bool ok = row < P1 && col < P1;
-        const float* from = ok ? C + row * P1 + col : C;
-        asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"(to), "l"(from), "r"(ok ? 4 : 0));
+// Row stride of a staged expansion of NB blocks per side.
+template <int NB>
+constexpr int kCoefStride = NB == 3 ? 16 : 4 * NB;
+
+// Starts the copy of an expansion's P1 x P1 coefficients to dst, rows of 4 NB
+// with zeros past column P1.  Whole rows per warp instruction (two of 16,
+// four of 8), so that a lane's column is fixed.
+template <int NB>
+__device__ __forceinline__ void stage_blocks(float* dst, const float* __restrict__ C, int P1, int lane) {
+    constexpr int S = kCoefStride<NB>, ROWS = NB < 5 ? 32 / S : 1;
+    const int row = NB < 5 ? lane / S : 0, col = NB < 5 ? lane % S : lane;
+    const float* from = C + row * P1 + min(col, P1 - 1);
+    unsigned to = (unsigned)__cvta_generic_to_shared(dst) + 4u * (unsigned)(row * S + col);
+    const int size = col < P1 ? 4 : 0;
+    if (NB == 5 && lane >= S) return;
+#pragma unroll 2
+    for (int r = row; r < P1; r += ROWS, from += ROWS * P1, to += 4u * ROWS * S)
+        asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"(to), "l"(from), "r"(size));
+}
+__device__ __forceinline__ void stage(float* dst, const float* __restrict__ C, int p, int lane) {
+    switch (coef_blocks(p)) {  // uniform over the warp
+        case 0: break;
+        case 1: stage_blocks<1>(dst, C, p + 1, lane); break;
+        case 2: stage_blocks<2>(dst, C, p + 1, lane); break;
+        case 3: stage_blocks<3>(dst, C, p + 1, lane); break;
+        case 4: stage_blocks<4>(dst, C, p + 1, lane); break;
+        default: stage_blocks<5>(dst, C, p + 1, lane); break;
     }
     asm volatile("cp.async.commit_group;");
 }
@@ -945,65 +957,83 @@ __device__ __forceinline__ void stage(float* dst, const float* __restrict__ C, i
 // lanes sums one of G rows at a time, four coefficients per shared-memory
 // read; and the lanes exchange the sums.  Every recursion, every row's chain
 // and the outer sum keep their order; the padding adds zeros at the end of
-// each, so the value is hermite_eval's.  Loops stay rolled: with the descent
-// around it the kernel is bound by instruction fetch once its code outgrows
-// the instruction cache.  (q, centre): this lane's coordinate and the
-// expansion's along it, see warp_tables.
-__device__ __forceinline__ float hermite_tile(WarpTables& wt, const float* coef, int nb, int cols, float q,
-                                              float centre, float isq, int lane) {
+// each, so the value is hermite_eval's.  One form per number of blocks: a
+// row's reads are in flight together and the column's functions stay in
+// registers; the loop over rows stays rolled (with the descent around it the
+// kernel is bound by instruction fetch once its code outgrows the instruction
+// cache).  (t2, e): 2 t and exp(-t^2), t this lane's coordinate relative to
+// the expansion's centre.
+template <int NB>
+__device__ __forceinline__ float hermite_blocks(WarpTables& wt, const float* coef, int P1, int cols, float t2, float e,
+                                                int lane) {
     const unsigned full = 0xffffffffu;
-    const int G = 32 / cols, S = 4 * nb;
+    constexpr int S = kCoefStride<NB>;
+    const int G = 32 / cols;
     {
-        float t = fmul(fsub(q, centre), isq);
-        float e = det_expf_neg(-fmul(t, t));
-        float t2 = fmul(2.0f, t);
+        float4* row = reinterpret_cast<float4*>(wt.hermite[min(lane, 11)]);  // cols + G = 12
+        const bool writes = lane < 12;
         float4 h;
         h.x = e;
         h.y = fmul(t2, e);
         h.z = fsub(fmul(t2, h.y), fmul(2.0f, h.x));
         h.w = fsub(fmul(t2, h.z), fmul(4.0f, h.y));
-        float4* row = reinterpret_cast<float4*>(wt.hermite[min(lane, 11)]);  // cols + G = 12
-        const bool writes = lane < 12;
         if (writes) row[0] = h;
-        float k2 = 6.0f;  // 2 (k - 1): small whole numbers, exact
-#pragma unroll 1
-        for (int b = 1; b < nb; ++b, k2 += 8.0f) {
-            float u = h.z, v = h.w;
-            h.x = fsub(fmul(t2, v), fmul(k2, u));
-            h.y = fsub(fmul(t2, h.x), fmul(k2 + 2.0f, v));
-            h.z = fsub(fmul(t2, h.y), fmul(k2 + 4.0f, h.x));
-            h.w = fsub(fmul(t2, h.z), fmul(k2 + 6.0f, h.y));
+#pragma unroll
+        for (int b = 1; b < NB; ++b) {  // 2 (k - 1): small whole numbers, exact
+            h.x = fsub(fmul(t2, h.w), fmul(8.0f * b - 2.0f, h.z));
+            h.y = fsub(fmul(t2, h.x), fmul(8.0f * b, h.w));
+            h.z = fsub(fmul(t2, h.y), fmul(8.0f * b + 2.0f, h.x));
+            h.w = fsub(fmul(t2, h.z), fmul(8.0f * b + 4.0f, h.y));
             if (writes) row[b] = h;
         }
     }
     __syncwarp();
     const int col = lane & (cols - 1), mine = lane / cols;
-    const float4* hy = reinterpret_cast<const float4*>(wt.hermite[col]);
+    float4 hy[NB];
+#pragma unroll
+    for (int b = 0; b < NB; ++b) hy[b] = reinterpret_cast<const float4*>(wt.hermite[col])[b];
     const float4* hx = reinterpret_cast<const float4*>(wt.hermite[cols + mine]);
     float w = 0.0f;
 #pragma unroll 1
-    for (int a0 = 0; a0 < S; a0 += G) {
-        const float4* C = reinterpret_cast<const float4*>(coef + min(a0 + mine, S - 1) * S);
+    for (int a0 = 0; a0 < P1; a0 += G) {
+        const float4* C = reinterpret_cast<const float4*>(coef + min(a0 + mine, P1 - 1) * S);
         float r = 0.0f;
-#pragma unroll 1
-        for (int b = 0; b < nb; ++b) {
-            const float4 c = C[b], h = hy[b];
-            r = __fmaf_rn(c.x, h.x, r);
-            r = __fmaf_rn(c.y, h.y, r);
-            r = __fmaf_rn(c.z, h.z, r);
-            r = __fmaf_rn(c.w, h.w, r);
+#pragma unroll
+        for (int b = 0; b < NB; ++b) {
+            const float4 c = C[b];
+            r = __fmaf_rn(c.x, hy[b].x, r);
+            r = __fmaf_rn(c.y, hy[b].y, r);
+            r = __fmaf_rn(c.z, hy[b].z, r);
+            r = __fmaf_rn(c.w, hy[b].w, r);
         }
+        if (a0 + mine >= P1) r = 0.0f;
 #pragma unroll 1
-        for (int s = 0; s < G && a0 + s < S; s += 4) {
+        for (int s = 0; s < G && a0 + s < P1; s += 4) {
             const float4 h = hx[(a0 + s) >> 2];
             const int from = col + cols * s;
-            w = __fmaf_rn(h.x, __shfl_sync(full, r, from), w);
-            w = __fmaf_rn(h.y, __shfl_sync(full, r, from + cols), w);
-            w = __fmaf_rn(h.z, __shfl_sync(full, r, from + 2 * cols), w);
-            w = __fmaf_rn(h.w, __shfl_sync(full, r, from + 3 * cols), w);
+            const float r0 = __shfl_sync(full, r, from), r1 = __shfl_sync(full, r, from + cols);
+            const float r2 = __shfl_sync(full, r, from + 2 * cols), r3 = __shfl_sync(full, r, from + 3 * cols);
+            w = __fmaf_rn(h.x, r0, w);
+            w = __fmaf_rn(h.y, r1, w);
+            w = __fmaf_rn(h.z, r2, w);
+            w = __fmaf_rn(h.w, r3, w);
         }
     }
     return w;
+}
+// (q, centre): this lane's coordinate and the expansion's along it, see
+// warp_tables; P1 >= 1 coefficients per side.
+__device__ __forceinline__ float hermite_tile(WarpTables& wt, const float* coef, int P1, int cols, float q,
+                                              float centre, float isq, int lane) {
+    const float t = fmul(fsub(q, centre), isq);
+    const float e = det_expf_neg(-fmul(t, t)), t2 = fmul(2.0f, t);
+    switch ((P1 + 3) >> 2) {  // uniform over the warp
+        case 1: return hermite_blocks<1>(wt, coef, P1, cols, t2, e, lane);
+        case 2: return hermite_blocks<2>(wt, coef, P1, cols, t2, e, lane);
+        case 3: return hermite_blocks<3>(wt, coef, P1, cols, t2, e, lane);
+        case 4: return hermite_blocks<4>(wt, coef, P1, cols, t2, e, lane);
+        default: return hermite_blocks<5>(wt, coef, P1, cols, t2, e, lane);
+    }
 }
 
 // node_weight of one lane's own node, the case of an expansion in few
@@ -1207,18 +1237,17 @@ __device__ int warp_tables(const Tree& T, float qx, float qy, unsigned lanes, in
         for (int k = -1; k < cnt; ++k) {
             if (k + 1 < cnt) {
                 const float next = __shfl_sync(full, c.w, k + 1);
-                const int pn = meta_degree(next);
-                stage(wt.coef[(k + 1) & 1], T.coef + meta_offset(next), pn, (pn + 4) >> 2, lane);
+                stage(wt.coef[(k + 1) & 1], T.coef + meta_offset(next), meta_degree(next), lane);
             }
             if (k < 0) continue;
             const unsigned m = __shfl_sync(full, ev.y, k);
             const float cx = __shfl_sync(full, c.x, k), cy = __shfl_sync(full, c.y, k);
-            const int nb = (meta_degree(__shfl_sync(full, c.w, k)) + 4) >> 2;
+            const int P1 = meta_degree(__shfl_sync(full, c.w, k)) + 1;
             if (k + 1 < cnt) asm volatile("cp.async.wait_group 1;" ::: "memory");
             else asm volatile("cp.async.wait_group 0;" ::: "memory");
             __syncwarp();
-            float w = nb == 0 ? leaf_mass(T, make_float4(cx, cy, 0.0f, 0.0f), qx, qy)
-                              : hermite_tile(wt, wt.coef[k & 1], nb, cols, q, columns ? cy : cx, T.isq, lane);
+            float w = P1 == 0 ? leaf_mass(T, make_float4(cx, cy, 0.0f, 0.0f), qx, qy)
+                              : hermite_tile(wt, wt.coef[k & 1], P1, cols, q, columns ? cy : cx, T.isq, lane);
             w = ((m >> lane) & 1u) ? w : 0.0f;
             if (v0 + k < kRows) wt.val[v0 + k][lane] = w;
             else val_hi[v0 + k - kRows] = w;
@@ -1360,7 +1389,8 @@ constexpr int kKnown = 3;  // nodes outside the tables whose child masses a lane
 // waiting for the previous instruction); the same algorithm with unrolled
 // loops ran 516 million but took 2.6 ms instead of 1.34, fetching them (187
 // KB of code instead of 54).  500k / 1024^2 / K = 8: 2.7-3.3 ms before these
-// tables, 11 ms where one pixel's cache of 160 nodes overflowed; 1.3 ms now.
+// tables, 11 ms where one pixel's cache of 160 nodes overflowed; 1.34 with
+// rolled series, 1.22 with one form of the series per number of blocks.
 constexpr int kDescentThreads = 64, kDescentBlocks = 6;
 
 // Views of different sizes in one descent launch: blocks [first[v],
