@@ -49,9 +49,45 @@ struct ViewState {            // per-view device scalars (lives in the workspace
     int pad[4];
 };
 
+// ----------------------------------------------------- order of the tiles
+// Pixels take very different times to sample: one at a silhouette, where
+// many splats project onto a few pixels, takes ten times the mean, and most
+// images are partly empty.  Blocks started in raster order left a third of
+// the GPU's slots idle (500k splats at 1024^2: 1.22 ms, stochastic 2.93).  So
+// the image is cut into cells of 16 x 16 pixels (larger ones from 2^20 pixels
+// on, for at most kCells of them), the visible splats of each cell are
+// counted, and the descent's blocks take the cells in order of falling count
+// in the cell and its neighbours, to a quarter of a power of two: 0.96 ms,
+// stochastic 2.28.  (Cells of 32 x 32 without the neighbours 1.12 and 2.66;
+// of 16 x 16 without them 1.10 and 2.56: what is started late and takes long
+// sits next to a silhouette.)
+constexpr int kCells = 4096;
+__host__ __device__ inline int cell_shift(int W, int H) {
+    int sh = 4;
+    while ((((long long)W - 1) >> sh) + 1 > kCells / ((((long long)H - 1) >> sh) + 1)) ++sh;
+    return sh;
+}
+__host__ __device__ inline int cell_columns(int H, int sh) { return ((H - 1) >> sh) + 1; }
+static unsigned cell_blocks(int W, int H, dim3 block) {  // blocks that cover every cell
+    const int sh = cell_shift(W, H);
+    return (unsigned)(cell_columns(W, sh) * cell_columns(H, sh)) * ((1u << sh) / block.x) * ((1u << sh) / block.y);
+}
+// The first pixel (row i along W, column j along H) of a block of a view, its
+// place among the view's blocks given.
+__device__ __forceinline__ void cell_block(const unsigned short* __restrict__ order, int W, int H, unsigned at, int& i,
+                                           int& j) {
+    const int sh = cell_shift(W, H);
+    const unsigned across = (1u << sh) / blockDim.x, per = across * ((1u << sh) / blockDim.y);
+    const int cell = order[at / per], columns = cell_columns(H, sh);
+    i = ((cell / columns) << sh) + (int)(at % per / across * blockDim.y);
+    j = ((cell % columns) << sh) + (int)(at % across * blockDim.x);
+}
+
 // ----------------------------------------------------------- workspace
 struct Ws {
     ViewState* vs;
+    uint32_t* cells;          // visible splats of each cell (zeroed with vs: it follows it)
+    unsigned short* order;    // the cells in order of falling count
     uds_view_stats* stats;
     uint32_t *keysA, *idsA, *keysB, *idsB;
     uint32_t* hist;
@@ -90,6 +126,8 @@ static Ws layout(const uds_sample_params* p, char* base) {
     size_t off = 0;
     auto take = [&](size_t bytes) { size_t o = off; off += a256(bytes); return base ? base + o : nullptr; };
     w.vs = (ViewState*)take(sizeof(ViewState));
+    w.cells = (uint32_t*)take(4 * kCells);
+    w.order = (unsigned short*)take(2 * kCells);
     w.stats = (uds_view_stats*)take(sizeof(uds_view_stats) * (size_t)(p->B > 0 ? p->B : 1));
     w.keysA = (uint32_t*)take(4 * N);
     w.idsA = (uint32_t*)take(4 * N);
@@ -340,8 +378,8 @@ __device__ __forceinline__ float trunc_radius(float h, float precision, int coun
     return fsqrt(fmul(fmul(-2.0f, fmul(h, h)), det_logf(fdiv(precision, (float)(unsigned)count))));
 }
 
-__global__ void k_leaves(int N, float W, float H, float f, const float* __restrict__ pts,
-                         const ViewState* vs, float precision, const uint32_t* __restrict__ ids,
+__global__ void k_leaves(int N, int W, int H, float f, const float* __restrict__ pts, const ViewState* vs,
+                         float precision, uint32_t* __restrict__ cells, const uint32_t* __restrict__ ids,
                          float2* __restrict__ leaf_xy, int* __restrict__ leaf_id, int4* __restrict__ lnk,
                          int* __restrict__ par, float4* __restrict__ box, float4* __restrict__ cen) {
     int i = blockIdx.x * blockDim.x + threadIdx.x;
@@ -350,7 +388,14 @@ __global__ void k_leaves(int N, float W, float H, float f, const float* __restri
     int id = (int)ids[i];
     float p[3] = {pts[3 * (size_t)id], pts[3 * (size_t)id + 1], pts[3 * (size_t)id + 2]};
     float s[2];
-    screen_point(W, H, f, p, s);
+    screen_point((float)W, (float)H, f, p, s);
+    {  // neighbours in Morton order share their cell: one addition for each group of a warp
+        const int sh = cell_shift(W, H);
+        const int row = min(max((int)s[0], 0), W - 1) >> sh, column = min(max((int)s[1], 0), H - 1) >> sh;
+        const int cell = row * cell_columns(H, sh) + column;
+        const unsigned group = __match_any_sync(__activemask(), cell);
+        if ((threadIdx.x & 31) == __ffs(group) - 1) atomicAdd(&cells[cell], __popc(group));
+    }
     int v = n - 1 + i;
     leaf_xy[i] = make_float2(s[0], s[1]);
     leaf_id[i] = id;
@@ -728,6 +773,7 @@ struct Tree {
     const float* coef;
     const float2* leaf_xy;
     const int* leaf_id;
+    const unsigned short* order;
     int n;
     float sq;
     float isq;
@@ -1390,17 +1436,17 @@ constexpr int kKnown = 3;  // nodes outside the tables whose child masses a lane
 // loops ran 516 million but took 2.6 ms instead of 1.34, fetching them (187
 // KB of code instead of 54).  500k / 1024^2 / K = 8: 2.7-3.3 ms before these
 // tables, 11 ms where one pixel's cache of 160 nodes overflowed; 1.34 with
-// rolled series, 1.22 with one form of the series per number of blocks.
+// rolled series, 1.22 with one form of the series per number of blocks, 0.96
+// with the tiles in order of the work they hold (kCells).
 constexpr int kDescentThreads = 64, kDescentBlocks = 6;
 
 // Views of different sizes in one descent launch: blocks [first[v],
-// first[v+1]) of the one-dimensional grid cover view v, bx[v] blocks along
-// y per block row; its indices start at entry ioff[v] of the packed output.
+// first[v+1]) of the one-dimensional grid cover view v; its indices start at
+// entry ioff[v] of the packed output.
 constexpr int kMaxUneven = 32;
 struct UnevenViews {
     int nv;
     int first[kMaxUneven + 1];
-    int bx[kMaxUneven];
     int W[kMaxUneven], H[kMaxUneven];
     long long ioff[kMaxUneven];
 };
@@ -1416,19 +1462,17 @@ __global__ void __launch_bounds__(32 * kDescentWarps<KM>, KM <= 16 ? kDescentBlo
              const float* __restrict__ uniforms, uint64_t seed, const uint64_t* __restrict__ seed_ptr, uint32_t view,
              int* __restrict__ indices, uds_view_stats* st, size_t vstride, size_t ustride, size_t istride,
              UnevenViews uv) {
-    // block tile_x (y) x threads / tile_x (x).  blockIdx.z selects the
-    // view: its tree lives vstride bytes after the previous view's, its
-    // uniforms ustride floats and its indices istride entries further on.
-    // With UNEVEN the view and the block's place in it come from uv
-    // (blockIdx.x only; no uniforms tensor).
+    // block tile_x (y) x threads / tile_x (x), blockIdx.x its place among
+    // the view's (cell_block).  blockIdx.y selects the view: its tree lives
+    // vstride bytes after the previous view's, its uniforms ustride floats and
+    // its indices istride entries further on.  With UNEVEN the view and the
+    // block's place in it come from uv (blockIdx.x only; no uniforms tensor).
     if (seed_ptr) seed = *seed_ptr;
-    unsigned bxi = blockIdx.x, byi = blockIdx.y, vz = blockIdx.z;
+    unsigned at_block = blockIdx.x, vz = blockIdx.y;
     if (UNEVEN) {
         int b = 0;
         while (b + 1 < uv.nv && uv.first[b + 1] <= (int)blockIdx.x) ++b;
-        int local = (int)blockIdx.x - uv.first[b];
-        bxi = (unsigned)(local % uv.bx[b]);
-        byi = (unsigned)(local / uv.bx[b]);
+        at_block = blockIdx.x - (unsigned)uv.first[b];
         vz = (unsigned)b;
         W = uv.W[b];
         H = uv.H[b];
@@ -1443,6 +1487,7 @@ __global__ void __launch_bounds__(32 * kDescentWarps<KM>, KM <= 16 ? kDescentBlo
         T.coef = shifted(T.coef, off);
         T.leaf_xy = shifted(T.leaf_xy, off);
         T.leaf_id = shifted(T.leaf_id, off);
+        T.order = shifted(T.order, off);
         vs = shifted(vs, off);
         view += vz;
         if (!UNEVEN) {
@@ -1454,8 +1499,11 @@ __global__ void __launch_bounds__(32 * kDescentWarps<KM>, KM <= 16 ? kDescentBlo
     __shared__ WarpTables s_tables[kDescentWarps<KM>];
     extern __shared__ uint2 list[];  // K > 16: (key, id) in order, one column per lane
     const unsigned full = 0xffffffffu;
-    int j = bxi * blockDim.x + threadIdx.x;
-    int i = byi * blockDim.y + threadIdx.y;
+    int i, j;
+    cell_block(T.order, W, H, at_block, i, j);
+    if (i >= W || j >= H) return;  // (uniform over the block)
+    i += threadIdx.y;
+    j += threadIdx.x;
     int tid = threadIdx.x + blockDim.x * threadIdx.y;
     int warp = tid >> 5, lane = tid & 31;
     bool live = (i < W && j < H);
@@ -1758,12 +1806,11 @@ __global__ void __launch_bounds__(32 * kDescentWarps<KM>, KM <= 16 ? kDescentBlo
 // their upper paths, so the child masses of the last path are kept per depth
 // (node ids are unique, so a hit is exact).  A draw that meets two zero
 // masses, or is still above the leaves after kTrace levels, stays -1 / 0.
-__global__ void __launch_bounds__(kDescentThreads, kDescentBlocks) k_stochastic(Tree T, const ViewState* vs, int W, int H, int K,
-                                                       float precision, uint64_t seed,
-                                                       const uint64_t* __restrict__ seed_ptr, uint32_t view,
-                                                       int* __restrict__ indices, float* __restrict__ probs,
-                                                       uds_view_stats* st, const unsigned char* __restrict__ mask,
-                                                       float* __restrict__ weights) {
+__global__ void __launch_bounds__(kDescentThreads, kDescentBlocks)
+    k_stochastic(Tree T, const ViewState* vs, int W, int H, int K, float precision, uint64_t seed,
+                 const uint64_t* __restrict__ seed_ptr, uint32_t view, int* __restrict__ indices,
+                 float* __restrict__ probs, uds_view_stats* st, const unsigned char* __restrict__ mask,
+                 float* __restrict__ weights) {
     // same warp layout and per-pixel mass cache as k_sample: one warp walks
     // its 32 pixels' trees together, then every lane draws its K paths; the
     // masses come from the cache, the per-depth cache of earlier draws, or a
@@ -1772,8 +1819,11 @@ __global__ void __launch_bounds__(kDescentThreads, kDescentBlocks) k_stochastic(
     if (seed_ptr) seed = *seed_ptr;
     __shared__ WarpTables s_tables[kDescentThreads / 32];
     const unsigned full = 0xffffffffu;
-    int j = blockIdx.x * blockDim.x + threadIdx.x;
-    int i = blockIdx.y * blockDim.y + threadIdx.y;
+    int i, j;
+    cell_block(T.order, W, H, blockIdx.x, i, j);
+    if (i >= W || j >= H) return;  // (uniform over the block)
+    i += threadIdx.y;
+    j += threadIdx.x;
     int tid = threadIdx.x + blockDim.x * threadIdx.y;
     int warp = tid >> 5, lane = tid & 31;
     size_t pixel = (size_t)j + (size_t)H * i;
@@ -2186,9 +2236,53 @@ __global__ void k_prop_clear(size_t P, int K, const unsigned char* __restrict__ 
     }
 }
 
-__global__ void k_finish_view(const ViewState* vs, uds_view_stats* st) {
-    st->n_visible = vs->n;
-    st->n_coefs = (int)vs->coef_used;
+// One block: the view's statistics, and its cells in order of falling count
+// (counting sort; cells of about the same count in any order).
+constexpr int kFinishThreads = 1024, kBuckets = 128;
+__global__ void __launch_bounds__(kFinishThreads) k_finish_view(const ViewState* vs, uds_view_stats* st, int W, int H,
+                                                                const uint32_t* __restrict__ cells,
+                                                                unsigned short* __restrict__ order) {
+    __shared__ int place[kBuckets];
+    __shared__ uint32_t count[kCells];
+    const int t = threadIdx.x, sh = cell_shift(W, H), rows = cell_columns(W, sh), columns = cell_columns(H, sh);
+    const int n = rows * columns;
+    for (int c = t; c < n; c += kFinishThreads) count[c] = cells[c];
+    if (t == 0) {
+        st->n_visible = vs->n;
+        st->n_coefs = (int)vs->coef_used;
+    }
+    if (t < kBuckets) place[t] = 0;
+    __syncthreads();
+    // bucket 127: empty; below, four per power of two, larger counts first.  A
+    // pixel sees splats up to a few bandwidths away: the neighbours count too.
+    auto bucket = [&](int c) {
+        const int i = c / columns, j = c % columns;
+        unsigned x = 0;
+        for (int a = max(i - 1, 0); a <= min(i + 1, rows - 1); ++a)
+            for (int b = max(j - 1, 0); b <= min(j + 1, columns - 1); ++b) x += count[a * columns + b];
+        return x ? (int)(kBuckets - 2 - ((__float_as_uint((float)x) >> 21) - (127u << 2))) : kBuckets - 1;
+    };
+    for (int c = t; c < n; c += kFinishThreads) atomicAdd(&place[bucket(c)], 1);
+    __syncthreads();
+    if (t < 32) {  // exclusive sums, four buckets per lane
+        int x[kBuckets / 32], sum = 0;
+#pragma unroll
+        for (int q = 0; q < kBuckets / 32; ++q) {
+            x[q] = sum;
+            sum += place[t * (kBuckets / 32) + q];
+        }
+        int before = sum;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const int y = __shfl_up_sync(0xffffffffu, before, o);
+            if (t >= o) before += y;
+        }
+        before -= sum;
+#pragma unroll
+        for (int q = 0; q < kBuckets / 32; ++q) place[t * (kBuckets / 32) + q] = before + x[q];
+    }
+    __syncthreads();
+    for (int c = t; c < n; c += kFinishThreads) order[atomicAdd(&place[bucket(c)], 1)] = (unsigned short)c;
 }
 
 // Evaluate getWeight for (node, query) pairs (debug entry point).
@@ -2210,7 +2304,7 @@ static int build_view(const uds_sample_params* p, const Ws& w, int view, const f
     const float* vp = pts + 3 * (size_t)N * view;
     const float* vn = nrm + 3 * (size_t)N * view;
     const float* vsd = sd + (p->std_batch > 1 ? 2 * (size_t)N * view : 0);
-    cudaError_t e = cudaMemsetAsync(w.vs, 0, sizeof(ViewState), s);
+    cudaError_t e = cudaMemsetAsync(w.vs, 0, (size_t)((char*)(w.cells + kCells) - (char*)w.vs), s);
     if (e == cudaSuccess) e = cudaMemsetAsync(w.fanin, 0, 4 * (size_t)(N > 0 ? N : 1), s);
     if (e != cudaSuccess) { set_last_error(e); return UDS_ERR_CUDA; }
     int st;
@@ -2246,8 +2340,8 @@ static int build_view(const uds_sample_params* p, const Ws& w, int view, const f
         t = vi; vi = vo; vo = t;
     }
     // after an even number of passes the sorted data is back in A
-    k_leaves<<<nbN, 128, 0, s>>>(N, W, H, f, vp, w.vs, p->precision, vi, w.leaf_xy, w.leaf_id, w.lnk, w.par,
-                                 w.box, w.cen);
+    k_leaves<<<nbN, 128, 0, s>>>(N, p->W, p->H, f, vp, w.vs, p->precision, w.cells, vi, w.leaf_xy, w.leaf_id, w.lnk,
+                                 w.par, w.box, w.cen);
     k_karras<<<nbN, 128, 0, s>>>(w.vs, ki, w.lnk, w.par);
     if (p->fixed_degree > 0) {
         int P = p->fixed_degree;
@@ -2260,7 +2354,7 @@ static int build_view(const uds_sample_params* p, const Ws& w, int view, const f
             case 6: k_m2m<6><<<nbN, 128, 0, s>>>(w.vs, w.lnk, w.par, w.cen, w.coef, w.fanin); break;
             default: k_m2m<8><<<nbN, 128, 0, s>>>(w.vs, w.lnk, w.par, w.cen, w.coef, w.fanin); break;
         }
-        k_finish_view<<<1, 1, 0, s>>>(w.vs, w.stats + view);
+        k_finish_view<<<1, kFinishThreads, 0, s>>>(w.vs, w.stats + view, p->W, p->H, w.cells, w.order);
         return launch_status(6);
     }
     k_bottomup<<<nbN, 128, 0, s>>>(w.vs, p->precision, p->max_degree, w.lnk, w.par, w.box, w.cen, w.fanin);
@@ -2272,7 +2366,7 @@ static int build_view(const uds_sample_params* p, const Ws& w, int view, const f
     k_scan_down<<<sb, kScanThreads, 0, s>>>(w.sizes, w.vs, 1, 0, w.scanTmp, w.offsets);
     k_assign<<<nbN, 128, 0, s>>>(w.vs, w.cen, w.sizes, w.offsets, w.coef_cap, w.stats + view);
     k_p2m<<<cdiv((size_t)N, 32 * kP2MWarps), 32 * kP2MWarps, 0, s>>>(w.vs, w.lnk, w.cen, w.leaf_xy, w.coef);
-    k_finish_view<<<1, 1, 0, s>>>(w.vs, w.stats + view);
+    k_finish_view<<<1, kFinishThreads, 0, s>>>(w.vs, w.stats + view, p->W, p->H, w.cells, w.order);
     return launch_status(6);
 }
 
@@ -2287,12 +2381,12 @@ static int tile_of(const uds_sample_params* p) { return p->tile_x == 4 ? 4 : 8; 
 static Tree tree_of(const Ws& w) {
     Tree T;
     T.lnk = w.lnk; T.par = w.par; T.box = w.box; T.cen = w.cen; T.coef = w.coef;
-    T.leaf_xy = w.leaf_xy; T.leaf_id = w.leaf_id; T.n = 0; T.sq = 0.0f; T.isq = 0.0f;
+    T.leaf_xy = w.leaf_xy; T.leaf_id = w.leaf_id; T.order = w.order; T.n = 0; T.sq = 0.0f; T.isq = 0.0f;
     return T;
 }
 
 template <int R>
-// Descent for views view .. view + nviews - 1 in one launch (grid.z = view),
+// Descent for views view .. view + nviews - 1 in one launch (grid.y = view),
 // their trees vstride bytes apart in the workspace.
 // Block: tile_x (y) by kDescentThreads / tile_x (x) pixels; each warp is a
 // tile_x by 32 / tile_x pixel tile.  Every lane's walk is its own, so the
@@ -2301,7 +2395,7 @@ static void launch_sample(const Tree& T, const Ws& w, const uds_sample_params* p
                           int* idx, cudaStream_t s, int nviews = 1, size_t vstride = 0) {
     int tx = tile_of(p);
     dim3 block(tx, kDescentThreads / tx);
-    dim3 grid(cdiv(p->H, block.x), cdiv(p->W, block.y), nviews);
+    dim3 grid(cell_blocks(p->W, p->H, block), nviews);
     size_t istride = (size_t)p->W * p->H * p->K;
     const int M = candidates(p);
     size_t ustride = (size_t)p->W * p->H * R * M;
@@ -2320,7 +2414,7 @@ static void launch_sample(const Tree& T, const Ws& w, const uds_sample_params* p
         // the K smallest keys in registers up to 16, in shared memory above
         constexpr int RR = R >= 3 ? R : 3, KM = RR <= 4 ? 16 : kMaxK;
         dim3 block(tx, 32 * kDescentWarps<KM> / tx);
-        dim3 grid(cdiv(p->H, block.x), cdiv(p->W, block.y), nviews);
+        dim3 grid(cell_blocks(p->W, p->H, block), nviews);
         k_sample<RR, KM, false, true><<<grid, block, KM <= 16 ? 0 : 256 * (size_t)p->K, s>>>(
             T, w.vs, p->W, p->H, p->K, M, p->precision, u, p->seed, p->seed_dev, (uint32_t)view, idx,
             w.stats + view, vstride, ustride, istride, none);
@@ -2534,11 +2628,10 @@ extern "C" int uds_sample_views(const uds_sample_params* prm, const uds_view_des
             int blocks = 0;
             for (int b = 0; b < prm->B; ++b) {
                 uv.first[b] = blocks;
-                uv.bx[b] = (int)cdiv(views[b].H, tx);
                 uv.W[b] = views[b].W;
                 uv.H[b] = views[b].H;
                 uv.ioff[b] = off;
-                blocks += uv.bx[b] * (int)cdiv(views[b].W, kDescentThreads / tx);
+                blocks += (int)cell_blocks(views[b].W, views[b].H, dim3(tx, kDescentThreads / tx));
                 off += (long long)views[b].W * views[b].H * prm->K;
             }
             uv.first[prm->B] = blocks;
@@ -2595,12 +2688,13 @@ extern "C" int uds_sample_stochastic(const uds_sample_params* prm, const float* 
     if (e != cudaSuccess) { set_last_error(e); return UDS_ERR_CUDA; }
     Tree T = tree_of(w);
     dim3 block(8, kDescentThreads / 8);
-    dim3 grid(cdiv(prm->H, block.x), cdiv(prm->W, block.y));
+    const unsigned grid = cell_blocks(prm->W, prm->H, block);
     for (int b = 0; b < prm->B; ++b) {
         if ((st = build_view(prm, w, b, points, normals, std_devs, h_override, s))) return st;
         if (prm->N == 0) continue;
-        k_stochastic<<<grid, block, 0, s>>>(T, w.vs, prm->W, prm->H, prm->K, prm->precision, prm->seed, prm->seed_dev, (uint32_t)b,
-                                            indices + per_view * b, probs + per_view * b, w.stats + b, nullptr, nullptr);
+        k_stochastic<<<grid, block, 0, s>>>(T, w.vs, prm->W, prm->H, prm->K, prm->precision, prm->seed, prm->seed_dev,
+                                            (uint32_t)b, indices + per_view * b, probs + per_view * b, w.stats + b,
+                                            nullptr, nullptr);
         if ((st = launch_status())) return st;
     }
     if (stats) {
@@ -2815,8 +2909,9 @@ extern "C" int uds_sample_proposal(const uds_sample_params* prm, const float* po
         }
         // the plain stochastic sampler: every pixel, or the fallback pixels
         float* probs = q.logits;  // scratch for the path probabilities
-        k_stochastic<<<grid, block, 0, s>>>(T, w.vs, prm->W, prm->H, prm->K, prm->precision, prm->seed,
-                                            prm->seed_dev, (uint32_t)b, idx, probs, w.stats + b, mask, wt);
+        const unsigned cells = cell_blocks(prm->W, prm->H, block);
+        k_stochastic<<<cells, block, 0, s>>>(T, w.vs, prm->W, prm->H, prm->K, prm->precision, prm->seed,
+                                             prm->seed_dev, (uint32_t)b, idx, probs, w.stats + b, mask, wt);
         if ((st = launch_status())) return st;
     }
     if (stats) {
