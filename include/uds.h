@@ -51,7 +51,7 @@ typedef struct {
     int32_t n_coefs;  /* Hermite coefficients stored for internal nodes */
     int32_t demoted;  /* nodes whose expansion did not fit the coefficient pool */
     int32_t overflow; /* pixels whose descent exceeded the 64-entry trace */
-    int32_t reserved[2];
+    int32_t reserved[2]; /* [0]: 1 where a wait of the tree build ran out (the view samples nothing) */
 } uds_view_stats;
 
 /* Sampling parameters (sampling.cpp:48-94 plus the uniforms interface). */
@@ -147,7 +147,7 @@ typedef struct {
 
 /* ---- sampling.sample for B views of different sizes in one call (no
  *      counterpart in the reference, whose host loop runs one view at a time,
- *      samplingCuda.cu:216-289): every view's tree built (side streams), then
+ *      samplingCuda.cu:216-289): all views' trees built together, then
  *      one descent launch over all views' pixels for K <= 8 and B <= 32 (one
  *      launch per view otherwise).  views: host array of B descriptors (prm's
  *      W, H and focal are ignored); indices packed view after view, view b's
