@@ -9,32 +9,57 @@
 //   atomic mode: lanes of a warp that hold the same splat first combine their
 //     values (__match_any_sync + shuffles), then one atomic per group and
 //     channel; the order of additions is not fixed (like the reference).
-//   deterministic mode: the valid samples are compacted in sample order and
+//   deterministic mode: the valid samples are packed in sample order and
 //     stably radix-sorted by splat (so each splat's samples stay in sample
-//     order, however many there are), bucket offsets come from per-splat
-//     counts, and one thread sums its splat's values in that order: the
-//     result is bit-identical to a sequential sum in sample order.
+//     order, however many there are), and one thread sums its splat's values
+//     in that order: the result is bit-identical to a sequential sum in
+//     sample order.
 #include "uds_common.cuh"
 #include "uds_radix.cuh"
-#include "uds_scan.cuh"
 
 namespace uds {
 
-// one thread per (sample, channel) would re-read the index C times; one
-// thread per sample copies C contiguous floats
+// One thread per sample copies its splat's C values, four (16 bytes) at a time
+// where WIDE (C a multiple of four, both arrays aligned).
+template <bool WIDE>
 __global__ void k_pixel_scatter(size_t S, size_t per_view, int N, int C, const int* __restrict__ idx,
-                                 const float* __restrict__ values, float* __restrict__ out) {
-    size_t t = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
+                                const float* __restrict__ values, float* __restrict__ out) {
+    const size_t t = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (t >= S) return;
-    size_t b = t / per_view;
-    int id = idx[t];
+    const int id = idx[t];
+    const bool ok = id >= 0 && id < N;
+    const float* v = values + (ok ? ((size_t)id + (size_t)N * (t / per_view)) * C : 0);
     float* o = out + t * (size_t)C;
-    if (id < 0 || id >= N) {
-        for (int c = 0; c < C; ++c) o[c] = 0.0f;
-        return;
+    if (WIDE) {
+        for (int c = 0; c < C; c += 4)
+            *reinterpret_cast<float4*>(o + c) =
+                ok ? *reinterpret_cast<const float4*>(v + c) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    } else {
+        for (int c = 0; c < C; ++c) o[c] = ok ? v[c] : 0.0f;
     }
-    const float* v = values + ((size_t)id + (size_t)N * b) * C;
-    for (int c = 0; c < C; ++c) o[c] = v[c];
+}
+
+// Fewer than four channels: one thread per four samples, whose 4 C values are
+// C 16-byte stores (idx and out aligned, per_view a multiple of four).  Bound
+// by the writes: 1024 x 768, K = 8, C = 3 25 us, 37 with one sample
+// per thread.
+template <int C>
+__global__ void k_pixel_scatter4(size_t S, size_t per_view, int N, const int* __restrict__ idx,
+                                 const float* __restrict__ values, float* __restrict__ out) {
+    const size_t t = 4 * ((size_t)blockIdx.x * blockDim.x + threadIdx.x);
+    if (t >= S) return;
+    const int4 i4 = *reinterpret_cast<const int4*>(idx + t);
+    const int id[4] = {i4.x, i4.y, i4.z, i4.w};
+    const float* view = values + (size_t)N * (t / per_view) * C;
+    __align__(16) float x[4 * C];
+#pragma unroll
+    for (int q = 0; q < 4; ++q)
+#pragma unroll
+        for (int c = 0; c < C; ++c)
+            x[q * C + c] = id[q] >= 0 && id[q] < N ? view[(size_t)id[q] * C + c] : 0.0f;
+#pragma unroll
+    for (int c = 0; c < C; ++c)
+        reinterpret_cast<float4*>(out + t * C)[c] = make_float4(x[4 * c], x[4 * c + 1], x[4 * c + 2], x[4 * c + 3]);
 }
 
 __global__ void k_pixel_gather_atomic(size_t S, size_t per_view, int N, int C, const int* __restrict__ idx,
@@ -60,40 +85,130 @@ __global__ void k_pixel_gather_atomic(size_t S, size_t per_view, int N, int C, c
     }
 }
 
-// deterministic mode: per-splat counts and the valid-sample flags in one pass
-__global__ void k_pixel_count(size_t S, size_t per_view, int N, const int* __restrict__ idx,
-                              unsigned* __restrict__ count, unsigned* __restrict__ flag) {
-    size_t t = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= S) return;
-    int id = idx[t];
-    bool ok = id >= 0 && id < N;
-    flag[t] = ok ? 1u : 0u;
-    if (ok) atomicAdd(&count[(size_t)id + (size_t)N * (t / per_view)], 1u);
+// Deterministic mode.
+struct GatherState {
+    unsigned n;       // valid samples
+    unsigned failed;  // a wait ran out (see look_back): the sums are left at 0
+    unsigned ticket[6];
+};
+constexpr int kGatherPasses = 4;  // of 10 bits at most: 32-bit splat keys
+
+// Samples per thread of the packing and of the sort's passes.  Larger tiles
+// than the tree build's: there are more of them than the GPU holds blocks, and
+// the words of tiles that are looked back at are most of the sort's traffic.
+constexpr int kPackItems = 32, kPackTile = kPackItems * kTileThreads;
+constexpr int kSortItems = 16, kSortTile = kSortItems * kTileThreads;
+
+// The valid samples of a tile, packed behind those of the tiles before it:
+// (splat key, sample) pairs, and the digits of their keys.  The indices are
+// read twice (the second time from the L1), which keeps no key in a register.
+__global__ void __launch_bounds__(kTileThreads) k_pixel_pack(size_t S, size_t per_view, int N, int passes,
+                                                             const int* __restrict__ idx, GatherState* gs,
+                                                             unsigned long long* status, unsigned* hist,
+                                                             unsigned* __restrict__ keys,
+                                                             unsigned* __restrict__ samples) {
+    constexpr int kWarps = kTileThreads / 32;
+    __shared__ unsigned digits[kGatherPasses * kDigits];
+    __shared__ unsigned before[kPackItems * kWarps];
+    __shared__ unsigned s_first;
+    __shared__ int s_tile, s_failed;
+    const unsigned full = 0xffffffffu;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    if (threadIdx.x == 0) s_tile = (int)atomicAdd(&gs->ticket[kGatherPasses], 1u);
+    for (int d = threadIdx.x; d < passes * kDigits; d += kTileThreads) digits[d] = 0;
+    __syncthreads();
+    const size_t first = (size_t)s_tile * kPackTile + threadIdx.x;
+    auto sample = [&](int r) {
+        const size_t t = first + r * kTileThreads;
+        return t < S ? idx[t] : -1;
+    };
+    auto key_of = [&](int id, int r) {
+        return (unsigned)((size_t)id + (size_t)N * ((first + r * kTileThreads) / per_view));
+    };
+#pragma unroll 8
+    for (int r = 0; r < kPackItems; ++r) {
+        const int id = sample(r);
+        const bool ok = id >= 0 && id < N;
+        if (ok) {
+            const unsigned key = key_of(id, r);
+            for (int q = 0; q < passes; ++q)
+                atomicAdd(&digits[q * kDigits + ((key >> (q * kDigitBits)) & (kDigits - 1))], 1u);
+        }
+        const unsigned ball = __ballot_sync(full, ok);
+        if (lane == 0) before[r * kWarps + warp] = __popc(ball);
+    }
+    __syncthreads();
+    if (warp == 0) {
+        unsigned long long at;
+        unsigned total;
+        const bool ok = tile_places<kPackItems * kWarps>(before, status, s_tile, at, total);
+        if (lane == 0) {
+            s_first = (unsigned)at;
+            s_failed = !ok;
+            if (!ok) gs->failed = 1;
+            else if (s_tile == (int)gridDim.x - 1) gs->n = (unsigned)at + total;
+        }
+    }
+    __syncthreads();
+    if (s_failed) return;
+#pragma unroll 8
+    for (int r = 0; r < kPackItems; ++r) {
+        const int id = sample(r);
+        const bool ok = id >= 0 && id < N;
+        const unsigned ball = __ballot_sync(full, ok);
+        if (ok) {
+            const unsigned at = s_first + before[r * kWarps + warp] + __popc(ball & ((1u << lane) - 1u));
+            keys[at] = key_of(id, r);
+            samples[at] = (unsigned)(first + r * kTileThreads);
+        }
+    }
+    for (int d = threadIdx.x; d < passes * kDigits; d += kTileThreads)
+        if (digits[d]) atomicAdd(&hist[d], digits[d]);
 }
 
-// the valid samples in sample order: (splat key, sample offset) pairs
-__global__ void k_pixel_compact(size_t S, size_t per_view, int N, const int* __restrict__ idx,
-                                const unsigned* __restrict__ pos, unsigned* __restrict__ keys,
-                                unsigned* __restrict__ samples) {
-    size_t t = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= S) return;
-    int id = idx[t];
-    if (id < 0 || id >= N) return;
-    unsigned p = pos[t];
-    keys[p] = (unsigned)((size_t)id + (size_t)N * (t / per_view));
-    samples[p] = (unsigned)t;
+template <typename Word>
+__global__ void __launch_bounds__(kTileThreads) k_pixel_sort(int pass, GatherState* gs,
+                                                             const unsigned* __restrict__ hist, Word* status,
+                                                             const unsigned* __restrict__ kin,
+                                                             const unsigned* __restrict__ vin,
+                                                             unsigned* __restrict__ kout, unsigned* __restrict__ vout) {
+    const unsigned n = gs->failed ? 0u : gs->n;
+    if ((size_t)blockIdx.x * kSortTile >= n) return;
+    if (!sort_tile<kSortItems, Word>(n, pass * kDigitBits, &gs->ticket[pass], hist, status, kin, vin, kout, vout) &&
+        threadIdx.x == 0)
+        gs->failed = 1;
 }
 
-// one thread per splat sums its bucket (already in sample order)
-__global__ void k_pixel_sum(size_t M, int C, const unsigned* __restrict__ offs, const unsigned* __restrict__ slots,
+// First and one past the last of each splat's sorted samples (0, 0: none).
+__global__ void k_pixel_bounds(const GatherState* gs, const unsigned* __restrict__ keys, uint2* __restrict__ bounds) {
+    const size_t n = gs->failed ? 0 : gs->n, step = (size_t)gridDim.x * blockDim.x;
+    for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += step) {
+        const unsigned k = keys[i];
+        if (i == 0 || keys[i - 1] != k) bounds[k].x = (unsigned)i;
+        if (i + 1 == n || keys[i + 1] != k) bounds[k].y = (unsigned)i + 1u;
+    }
+}
+
+// One thread per splat sums its bucket (already in sample order), up to four
+// channels at a time, the next samples' values on their way.
+__global__ void k_pixel_sum(size_t M, int C, const uint2* __restrict__ bounds, const unsigned* __restrict__ slots,
                             const float* __restrict__ values, float* __restrict__ out) {
     size_t key = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (key >= M) return;
-    unsigned lo = offs[key], hi = offs[key + 1];
-    for (int c = 0; c < C; ++c) {
-        float s = 0.0f;
-        for (unsigned i = lo; i < hi; ++i) s = __fadd_rn(s, values[(size_t)slots[i] * C + c]);
-        out[key * (size_t)C + c] = s;
+    const uint2 range = bounds[key];
+    for (int c0 = 0; c0 < C; c0 += 4) {
+        const int cn = min(4, C - c0);
+        float s[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+#pragma unroll 4
+        for (unsigned i = range.x; i < range.y; ++i) {
+            const float* v = values + (size_t)slots[i] * C + c0;
+#pragma unroll
+            for (int c = 0; c < 4; ++c)
+                if (c < cn) s[c] = __fadd_rn(s[c], v[c]);
+        }
+#pragma unroll
+        for (int c = 0; c < 4; ++c)
+            if (c < cn) out[key * (size_t)C + c0 + c] = s[c];
     }
 }
 
@@ -106,41 +221,61 @@ extern "C" int uds_pixel_scatter(int B, int W, int H, int K, const int32_t* indi
     if (B <= 0 || W <= 0 || H <= 0 || K <= 0 || N < 0 || C <= 0 || !indices || !out || (N > 0 && !values))
         return UDS_ERR_ARGUMENT;
     size_t per_view = (size_t)W * H * K, S = per_view * B;
-    k_pixel_scatter<<<cdiv(S, 256), 256, 0, as_stream(stream)>>>(S, per_view, N, C, indices, values, out);
+    cudaStream_t s = as_stream(stream);
+    const bool aligned = ((reinterpret_cast<size_t>(indices) | reinterpret_cast<size_t>(values) |
+                           reinterpret_cast<size_t>(out)) & 15) == 0;
+    if (aligned && C < 4 && per_view % 4 == 0) {
+        if (C == 1) k_pixel_scatter4<1><<<cdiv(S / 4, 256), 256, 0, s>>>(S, per_view, N, indices, values, out);
+        else if (C == 2) k_pixel_scatter4<2><<<cdiv(S / 4, 256), 256, 0, s>>>(S, per_view, N, indices, values, out);
+        else k_pixel_scatter4<3><<<cdiv(S / 4, 256), 256, 0, s>>>(S, per_view, N, indices, values, out);
+    } else if (aligned && C % 4 == 0) {
+        k_pixel_scatter<true><<<cdiv(S, 256), 256, 0, s>>>(S, per_view, N, C, indices, values, out);
+    } else {
+        k_pixel_scatter<false><<<cdiv(S, 256), 256, 0, s>>>(S, per_view, N, C, indices, values, out);
+    }
     return launch_status();
 }
 
-// Deterministic-mode scratch: per-splat counts and offsets, sample flags and
-// positions, two (key, sample) pair buffers, the radix digit histograms and
-// their scan, and the scans' tile sums.
+// Deterministic-mode scratch: what is zeroed first (state, digit counts,
+// look-back words of the packing and of the sort's passes, the splats' bounds),
+// then two (key, sample) pair buffers.
 struct GatherWs {
-    unsigned *count, *offs, *flag, *pos, *ka, *va, *kb, *vb, *hist, *hscan, *part;
+    GatherState* state;
+    unsigned* hist;
+    unsigned long long* pack_status;
+    char* sort_status;
+    size_t sort_bytes;  // look-back words of one pass
+    uint2* bounds;
+    size_t zeroed;
+    unsigned *ka, *va, *kb, *vb;
+    int passes;
+    bool wide;  // 64-bit words: 2^30 samples or more
     size_t bytes;
 };
 
 static GatherWs gather_layout(size_t M, size_t S, char* base) {
-    auto a = [](size_t x) { return (x + 255) & ~(size_t)255; };
-    size_t nb = cdiv(S, kSortTile), nh = 256 * nb;
-    size_t longest = S > nh ? S : nh;
-    size_t parts = scan_part_entries(longest > M ? longest : M);
     GatherWs g{};
     size_t off = 0;
     auto take = [&](size_t n) {
-        unsigned* p = base ? reinterpret_cast<unsigned*>(base + off) : nullptr;
-        off += a(4 * n);
+        char* p = base ? base + off : nullptr;
+        off += (n + 255) & ~(size_t)255;
         return p;
     };
-    g.count = take(M);
-    g.offs = take(M + 1);
-    g.flag = take(S);
-    g.pos = take(S + 1);
-    g.ka = take(S);
-    g.va = take(S);
-    g.kb = take(S);
-    g.vb = take(S);
-    g.hist = take(nh);
-    g.hscan = take(nh + 1);
-    g.part = take(parts);
+    int bits = 1;
+    while (bits < 32 && M > 1 && (M - 1) >> bits) ++bits;
+    g.passes = (bits + kDigitBits - 1) / kDigitBits;
+    g.wide = S >= (1ull << 30);
+    g.sort_bytes = (g.wide ? 8 : 4) * (size_t)cdiv(S, kSortTile) * kDigits;
+    g.state = reinterpret_cast<GatherState*>(take(sizeof(GatherState)));
+    g.hist = reinterpret_cast<unsigned*>(take(4 * kGatherPasses * kDigits));
+    g.pack_status = reinterpret_cast<unsigned long long*>(take(8 * (size_t)cdiv(S, kPackTile)));
+    g.sort_status = take(g.sort_bytes * g.passes);
+    g.bounds = reinterpret_cast<uint2*>(take(8 * M));
+    g.zeroed = off;
+    g.ka = reinterpret_cast<unsigned*>(take(4 * S));
+    g.va = reinterpret_cast<unsigned*>(take(4 * S));
+    g.kb = reinterpret_cast<unsigned*>(take(4 * S));
+    g.vb = reinterpret_cast<unsigned*>(take(4 * S));
     g.bytes = off;
     return g;
 }
@@ -167,28 +302,26 @@ extern "C" int uds_pixel_gather(int B, int W, int H, int K, const int32_t* indic
     }
     if (!workspace || workspace_bytes < uds_pixel_gather_workspace_size(B, W, H, K, N)) return UDS_ERR_WORKSPACE;
     GatherWs g = gather_layout(M, S, reinterpret_cast<char*>(workspace));
-    cudaError_t e = cudaMemsetAsync(g.count, 0, 4 * M, s);
+    cudaError_t e = cudaMemsetAsync(g.state, 0, g.zeroed, s);
     if (e != cudaSuccess) { set_last_error(e); return UDS_ERR_CUDA; }
-    // bucket offsets from the per-splat counts; the valid samples in sample
-    // order, then a stable sort by splat; the number of valid samples
-    // (g.pos[S]) stays on the device
-    k_pixel_count<<<cdiv(S, 256), 256, 0, s>>>(S, per_view, N, indices, g.count, g.flag);
-    exclusive_scan(M, g.count, g.offs, g.part, s);
-    exclusive_scan(S, g.flag, g.pos, g.part, s);
-    k_pixel_compact<<<cdiv(S, 256), 256, 0, s>>>(S, per_view, N, indices, g.pos, g.ka, g.va);
-    int bits = 1;
-    while (bits < 32 && (M - 1) >> bits) ++bits;
-    unsigned nb = cdiv(S, kSortTile);
+    // the number of valid samples stays on the device
+    const unsigned tiles = cdiv(S, kSortTile);
+    k_pixel_pack<<<cdiv(S, kPackTile), kTileThreads, 0, s>>>(S, per_view, N, g.passes, indices, g.state, g.pack_status,
+                                                             g.hist, g.ka, g.va);
     unsigned *ki = g.ka, *vi = g.va, *ko = g.kb, *vo = g.vb;
-    int launched = 8;
-    for (int shift = 0; shift < bits; shift += 8) {
-        k_radix_hist<<<nb, kSortThreads, 0, s>>>((int)S, g.pos + S, ki, shift, g.hist);
-        exclusive_scan((size_t)256 * nb, g.hist, g.hscan, g.part, s);
-        k_radix_scatter<<<nb, kSortThreads, 0, s>>>((int)S, g.pos + S, ki, vi, ko, vo, shift, g.hscan);
+    for (int pass = 0; pass < g.passes; ++pass) {
+        const unsigned* hist = g.hist + pass * kDigits;
+        char* status = g.sort_status + g.sort_bytes * pass;
+        if (g.wide)
+            k_pixel_sort<unsigned long long><<<tiles, kTileThreads, 0, s>>>(
+                pass, g.state, hist, reinterpret_cast<unsigned long long*>(status), ki, vi, ko, vo);
+        else
+            k_pixel_sort<unsigned><<<tiles, kTileThreads, 0, s>>>(pass, g.state, hist,
+                                                                  reinterpret_cast<unsigned*>(status), ki, vi, ko, vo);
         unsigned* t = ki; ki = ko; ko = t;
         t = vi; vi = vo; vo = t;
-        launched += 5;
     }
-    k_pixel_sum<<<cdiv(M, 128), 128, 0, s>>>(M, C, g.offs, vi, values, out);
-    return launch_status(launched + 1);
+    k_pixel_bounds<<<cdiv(S, 256) < 1216 ? cdiv(S, 256) : 1216, 256, 0, s>>>(g.state, ki, g.bounds);
+    k_pixel_sum<<<cdiv(M, 128), 128, 0, s>>>(M, C, g.bounds, vi, values, out);
+    return launch_status(3 + g.passes);
 }

@@ -33,13 +33,14 @@
 #include <cuda_bf16.h>
 
 #include "uds_ewa.cuh"
+#include "uds_radix.cuh"
 #include "uds_tc.cuh"
 
 namespace uds {
 
 constexpr int kBatch = 32;  // views per launch of the build
-constexpr int kDigitBits = 10, kDigits = 1 << kDigitBits, kPasses = 3;  // 30-bit Morton keys
-constexpr int kTileThreads = 256, kTileItems = 8, kTile = kTileThreads * kTileItems;  // splats per block of a scan
+constexpr int kPasses = 3;  // of 10 bits: 30-bit Morton keys
+constexpr int kTileItems = 8, kTile = kTileItems * kTileThreads;  // splats per thread and block of a scan
 constexpr int kNodeTile = 128;  // nodes per block of k_p2m
 
 struct ViewState {            // per-view device scalars (lives in the workspace)
@@ -171,47 +172,6 @@ __device__ __forceinline__ P* shifted(P* p, size_t bytes) {
 }
 // Visible splats of a view whose build has not failed.
 __device__ __forceinline__ int visible(const ViewState* vs) { return vs->failed ? 0 : vs->n; }
-
-// ------------------------------------------------- decoupled look-back
-// Prefix sums over a kernel's tiles in the kernel itself (D. Merrill and M.
-// Garland, "Single-pass parallel prefix scan with decoupled look-back", NVIDIA
-// NVR-2016-002): a block publishes its tile's sum, adds up those of the tiles
-// before it until it meets one with its prefix, and publishes its own.  Tiles
-// are numbered by a ticket when their block starts, so the ones waited for
-// have all started, and publish before they wait.  A wait still ends after
-// kWait looks: the view is then marked as failed and samples nothing.  A word
-// holds state and sum together, so no other memory is ordered by it.
-constexpr int kWait = 1 << 20;
-constexpr unsigned long long kSumReady = 1ull << 62, kPrefixReady = 2ull << 62, kSumMask = kSumReady - 1ull;
-
-// By a whole warp: the sum of the tiles before `tile`; false if a wait ran out.
-__device__ __forceinline__ bool look_back(unsigned long long* status, int tile, unsigned long long sum,
-                                          unsigned long long& before) {
-    const unsigned full = 0xffffffffu;
-    const int lane = threadIdx.x & 31;
-    volatile unsigned long long* words = status;
-    before = 0;
-    if (lane == 0) words[tile] = (tile ? kSumReady : kPrefixReady) | sum;
-    if (tile == 0) return true;
-    for (int t = tile - 1;; t -= 32) {
-        unsigned long long x = kPrefixReady;  // before the first tile
-        if (t - lane >= 0) {
-            int looks = 0;
-            do x = words[t - lane];
-            while (!(x >> 62) && ++looks < kWait);
-        }
-        __syncwarp();
-        if (__any_sync(full, !(x >> 62))) return false;
-        const unsigned known = __ballot_sync(full, (x >> 62) == 2);
-        unsigned long long part = lane <= (known ? __ffs(known) - 1 : 31) ? x & kSumMask : 0ull;
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) part += __shfl_xor_sync(full, part, o);
-        before += part;
-        if (known) break;
-    }
-    if (lane == 0) words[tile] = kPrefixReady | (before + sum);
-    return true;
-}
 
 // --------------------------------------------------------- 1 bandwidth
 // IsotropicEigenFunctor (samplingCuda.cu:133-162) with the same float /
@@ -392,19 +352,9 @@ __global__ void __launch_bounds__(kTileThreads) k_cull(int N, Batch bt, const fl
     }
     __syncthreads();
     if (warp == 0) {
-        static_assert(kTileItems * kWarps == 64, "two counts per lane");
-        const unsigned a = before[2 * lane], b = before[2 * lane + 1];
-        unsigned incl = a + b;
-#pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-            const unsigned y = __shfl_up_sync(full, incl, o);
-            if (lane >= o) incl += y;
-        }
-        before[2 * lane] = incl - a - b;
-        before[2 * lane + 1] = incl - b;
-        const unsigned total = __shfl_sync(full, incl, 31);
         unsigned long long first;
-        const bool ok = look_back(status, tile, total, first);
+        unsigned total;
+        const bool ok = tile_places<kTileItems * kWarps>(before, status, tile, first, total);
         if (lane == 0) {
             s_first = ok ? (int)first : -1;
             if (!ok) vs->failed = 1;
@@ -425,147 +375,23 @@ __global__ void __launch_bounds__(kTileThreads) k_cull(int N, Batch bt, const fl
 }
 
 // ---------------------------------------------------------- 3 radix sort
-// One stable pass over (key, id) pairs: warp w of a block owns items [256 w,
-// 256 w + 256) of its tile, lane l holds item 256 w + 32 r + l in round r, so
-// (round, lane) order is item order and per-warp running counts give a stable
-// rank.  A digit's items of a tile go behind those of the smaller digits (from
-// the counts of all keys) and of the tiles before it (look-back, one word per
-// tile and digit, four digits per thread).  Bound by the latency of its few
-// steps: 500k splats 18 us a pass; 4 passes of 8 bits with counts,
-// scans and scatters in launches of their own took 64 us in all; one tile
-// looked at per step instead of four 23 us a pass.
-constexpr uint32_t kDigitSum = 1u << 30, kDigitPrefix = 2u << 30, kDigitMask = kDigitSum - 1u;
-
+// One pass over every view's visible splats (sort_tile); tiles_max: tiles of
+// look-back words per pass.  500k splats: 18 us a pass; 4 passes of 8 bits
+// with counts, scans and scatters in launches of their own took 64 us in all.
 __global__ void __launch_bounds__(kTileThreads) k_sort_pass(Batch bt, int pass, int tiles_max, ViewState* vs,
                                                             const uint32_t* __restrict__ hist, uint32_t* status,
                                                             const uint32_t* __restrict__ kin,
                                                             const uint32_t* __restrict__ vin,
                                                             uint32_t* __restrict__ kout, uint32_t* __restrict__ vout) {
-    constexpr int kWarps = kTileThreads / 32, kPer = kDigits / kTileThreads;
-    static_assert(kPer == 4, "four digits per thread");
-    __shared__ unsigned wcnt[kWarps][kDigits];
-    __shared__ __align__(16) unsigned goff[kDigits];
-    __shared__ unsigned wsum[kWarps];
-    __shared__ int s_tile, s_failed;
-    const unsigned full = 0xffffffffu;
     const size_t off = bt.slot * blockIdx.y;
     vs = shifted(vs, off);
-    const int n = visible(vs), tiles = (n + kTile - 1) / kTile;
-    if ((int)blockIdx.x >= tiles) return;
-    hist = shifted(hist, off) + pass * kDigits;
-    volatile uint32_t* words = shifted(status, off) + (size_t)pass * tiles_max * kDigits;
-    kin = shifted(kin, off);
-    vin = shifted(vin, off);
-    kout = shifted(kout, off);
-    vout = shifted(vout, off);
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, shift = pass * kDigitBits;
-    if (threadIdx.x == 0) {
-        s_tile = (int)atomicAdd(&vs->ticket[pass], 1u);
-        s_failed = 0;
-    }
-    for (int d = lane; d < kDigits; d += 32) wcnt[warp][d] = 0;
-    __syncthreads();
-    const int tile = s_tile;
-    uint32_t key[kTileItems], val[kTileItems];
-    unsigned rank[kTileItems];
-    const unsigned lt = (1u << lane) - 1u;
-    const int base = tile * kTile + warp * 32 * kTileItems;
-#pragma unroll
-    for (int r = 0; r < kTileItems; ++r) {
-        const int i = base + r * 32 + lane;
-        key[r] = i < n ? kin[i] : 0u;
-        val[r] = i < n ? vin[i] : 0u;
-    }
-#pragma unroll
-    for (int r = 0; r < kTileItems; ++r) {
-        const bool ok = base + r * 32 + lane < n;
-        const unsigned dig = ok ? (key[r] >> shift) & (kDigits - 1) : kDigits;
-        const unsigned peers = __match_any_sync(full, dig);
-        const unsigned before = ok ? wcnt[warp][dig] : 0u;
-        rank[r] = before + __popc(peers & lt);
-        __syncwarp();
-        if (ok && (peers & lt) == 0) wcnt[warp][dig] = before + __popc(peers);
-        __syncwarp();
-    }
-    __syncthreads();
-    unsigned count[kPer];
-#pragma unroll
-    for (int q = 0; q < kPer; ++q) {
-        const int d = threadIdx.x + q * kTileThreads;
-        unsigned run = 0;
-#pragma unroll
-        for (int w = 0; w < kWarps; ++w) {
-            const unsigned c = wcnt[w][d];
-            wcnt[w][d] = run;
-            run += c;
-        }
-        count[q] = run;
-        words[(size_t)tile * kDigits + d] = (tile ? kDigitSum : kDigitPrefix) | run;
-    }
-    {  // where each digit's items begin
-        const uint4 h = reinterpret_cast<const uint4*>(hist)[threadIdx.x];
-        const unsigned sum = h.x + h.y + h.z + h.w;
-        unsigned incl = sum;
-#pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-            const unsigned y = __shfl_up_sync(full, incl, o);
-            if (lane >= o) incl += y;
-        }
-        if (lane == 31) wsum[warp] = incl;
-        __syncthreads();
-        unsigned first = incl - sum;
-        for (int w = 0; w < warp; ++w) first += wsum[w];
-        reinterpret_cast<uint4*>(goff)[threadIdx.x] = make_uint4(first, first + h.x, first + h.x + h.y,
-                                                                 first + h.x + h.y + h.z);
-    }
-    unsigned before[kPer] = {0u, 0u, 0u, 0u};
-    if (tile) {
-        int at[kPer] = {tile - 1, tile - 1, tile - 1, tile - 1};  // < 0: done
-        int looks = 0;
-        while ((at[0] >= 0 || at[1] >= 0 || at[2] >= 0 || at[3] >= 0) && looks < kWait) {
-            constexpr int kAhead = 4;  // tiles looked at together
-            uint32_t x[kPer][kAhead];
-#pragma unroll
-            for (int q = 0; q < kPer; ++q)
-#pragma unroll
-                for (int a = 0; a < kAhead; ++a)
-                    x[q][a] = at[q] >= a ? words[(size_t)(at[q] - a) * kDigits + threadIdx.x + q * kTileThreads] : 0u;
-#pragma unroll
-            for (int q = 0; q < kPer; ++q) {
-                bool on = at[q] >= 0;
-#pragma unroll
-                for (int a = 0; a < kAhead; ++a) {
-                    on = on && (x[q][a] >> 30);  // (no state yet: look again)
-                    if (on) {
-                        before[q] += x[q][a] & kDigitMask;
-                        at[q] = (x[q][a] & kDigitPrefix) ? -1 : at[q] - 1;
-                        on = at[q] >= 0;
-                    }
-                }
-            }
-            ++looks;
-        }
-        if (looks >= kWait) s_failed = 1;
-#pragma unroll
-        for (int q = 0; q < kPer; ++q)
-            words[(size_t)tile * kDigits + threadIdx.x + q * kTileThreads] = kDigitPrefix | (before[q] + count[q]);
-    }
-    __syncthreads();
-    if (s_failed) {
-        if (threadIdx.x == 0) vs->failed = 1;
-        return;
-    }
-#pragma unroll
-    for (int q = 0; q < kPer; ++q) goff[threadIdx.x + q * kTileThreads] += before[q];
-    __syncthreads();
-#pragma unroll
-    for (int r = 0; r < kTileItems; ++r)
-        if (base + r * 32 + lane < n) {
-            const unsigned dig = (key[r] >> shift) & (kDigits - 1);
-            const unsigned pos = goff[dig] + wcnt[warp][dig] + rank[r];
-            kout[pos] = key[r];
-            vout[pos] = val[r];
-        }
+    const int n = visible(vs);
+    if ((long long)blockIdx.x * kTile >= n) return;
+    if (!sort_tile<kTileItems, uint32_t>(n, pass * kDigitBits, &vs->ticket[pass], shifted(hist, off) + pass * kDigits,
+                             shifted(status, off) + (size_t)pass * tiles_max * kDigits, shifted(kin, off),
+                             shifted(vin, off), shifted(kout, off), shifted(vout, off)) &&
+        threadIdx.x == 0)
+        vs->failed = 1;
 }
 
 // ---------------------------------------------------- 4 leaves + Karras
