@@ -1047,12 +1047,15 @@ __device__ __noinline__ float node_weight_out_of_line(Tree T, int v, float qx, f
 // (pixels far apart in units of the bandwidth share little of the tree), the
 // caller takes half the lanes at a time.
 constexpr int kOpen = 224, kEvals = 192;  // table entries
-constexpr int kRows = 64;                 // masses in shared memory
+constexpr int kRows = 63;                 // masses in shared memory
 constexpr int kLevels = 64;               // a radix tree over 62-bit keys is at most 63 deep
 // Per-lane records of the descent in shared memory: local memory that is
 // written and read back costs an L2 round trip here (about 700 cycles).
 constexpr int kPathRows = 32;
-constexpr int kSide = 20;                 // Hermite functions and coefficients per side (17, in blocks of four)
+// A staged pair's rows (kPairStride) and the Hermite functions' rows are padded
+// so that the four rows and eight columns a warp reads together lie in
+// different banks.
+constexpr int kPairFloats = 16 * 36, kHermiteStride = 36;
 
 // A child's link: kind, stop bit (the child holds at most M splats), entry
 // of an opened child.
@@ -1072,10 +1075,9 @@ struct WarpTables {
     };
     union {
         struct {                     // until the masses are known
-            uint2 eval[kEvals];      // node, lanes inside
-            float coef[2][kSide * kSide];  // the expansion being evaluated and the next one, in whole blocks of
-                                           // 4 x 4, padded with zeros
-            float hermite[12][kSide];      // Hermite functions of the tile's columns, then of its rows
+            unsigned short eval[kEvals];              // opened parent << 1 | side of each expansion
+            alignas(16) float coef[2][kPairFloats];   // the pair of expansions being evaluated and the next one
+            float hermite[12][kHermiteStride];        // Hermite functions of the tile's columns, then of its rows
         };
         struct {                     // afterwards
             float path[kPathRows][32];         // per-lane records of the levels below the stem
@@ -1088,59 +1090,162 @@ struct WarpTables {
 // Blocks of four coefficients per side of a degree-p expansion.
 __device__ __forceinline__ int coef_blocks(int p) { return (p + 4) >> 2; }
 
-// Row stride of a staged expansion of NB blocks per side.
+// Row stride of a staged pair of expansions of NB <= 4 blocks per side (the
+// coefficients of the two interleaved), and of a single one of five.
 template <int NB>
-constexpr int kCoefStride = NB == 3 ? 16 : 4 * NB;
+constexpr int kPairStride = NB == 4 ? 36 : NB == 3 ? 24 : NB == 2 ? 20 : 8;
+constexpr int kSingleStride = 20;
 
-// Starts the copy of an expansion's P1 x P1 coefficients to dst, rows of 4 NB
-// with zeros past column P1.  Whole rows per warp instruction (two of 16,
-// four of 8), so that a lane's column is fixed.
-template <int NB>
-__device__ __forceinline__ void stage_blocks(float* dst, const float* __restrict__ C, int P1, int lane) {
-    constexpr int S = kCoefStride<NB>, ROWS = NB < 5 ? 32 / S : 1;
+// Two floats in a register pair: one instruction works on both, each rounded
+// as by itself.
+typedef unsigned long long float_pair;
+__device__ __forceinline__ float_pair pair_of(float a, float b) {
+    float_pair r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
+    return r;
+}
+__device__ __forceinline__ void pair_split(float_pair p, float& a, float& b) {
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(p));
+}
+__device__ __forceinline__ float_pair pair_fma(float_pair a, float_pair b, float_pair c) {
+    float_pair r;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+    return r;
+}
+__device__ __forceinline__ float_pair pair_same(float a) { return pair_of(a, a); }
+// Product and difference, rounded by themselves: as multiply-adds, since a
+// product that is subtracted from would be contracted in this form.
+__device__ __forceinline__ float_pair pair_mul(float_pair a, float_pair b) { return pair_fma(a, b, pair_same(-0.0f)); }
+__device__ __forceinline__ float_pair pair_sub(float_pair a, float_pair b) { return pair_fma(b, pair_same(-1.0f), a); }
+
+// Starts the copy of an expansion's P1 x P1 coefficients to dst, rows of
+// STRIDE floats with a coefficient every STEP and zeros past column P1 up to
+// 4 NB.  Whole rows per warp instruction, so that a lane's column is fixed.
+template <int NB, int STRIDE, int STEP>
+__device__ __forceinline__ void stage_rows(float* dst, const float* __restrict__ C, int P1, int lane) {
+    constexpr int S = NB == 3 ? 16 : 4 * NB, ROWS = NB < 5 ? 32 / S : 1;
     const int row = NB < 5 ? lane / S : 0, col = NB < 5 ? lane % S : lane;
     const float* from = C + row * P1 + min(col, P1 - 1);
-    unsigned to = (unsigned)__cvta_generic_to_shared(dst) + 4u * (unsigned)(row * S + col);
+    unsigned to = (unsigned)__cvta_generic_to_shared(dst) + 4u * (unsigned)(row * STRIDE + col * STEP);
     const int size = col < P1 ? 4 : 0;
-    if (NB == 5 && lane >= S) return;
+    if (NB >= 3 && col >= 4 * NB) return;
 #pragma unroll 2
-    for (int r = row; r < P1; r += ROWS, from += ROWS * P1, to += 4u * ROWS * S)
+    for (int r = row; r < P1; r += ROWS, from += ROWS * P1, to += 4u * ROWS * STRIDE)
         asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"(to), "l"(from), "r"(size));
 }
-__device__ __forceinline__ void stage(float* dst, const float* __restrict__ C, int p, int lane) {
-    switch (coef_blocks(p)) {  // uniform over the warp
-        case 0: break;
-        case 1: stage_blocks<1>(dst, C, p + 1, lane); break;
-        case 2: stage_blocks<2>(dst, C, p + 1, lane); break;
-        case 3: stage_blocks<3>(dst, C, p + 1, lane); break;
-        case 4: stage_blocks<4>(dst, C, p + 1, lane); break;
-        default: stage_blocks<5>(dst, C, p + 1, lane); break;
+// A pair of NB <= 4 blocks (P1: coefficients per side of both).
+__device__ __forceinline__ void stage_pair(float* dst, int nb, const float* __restrict__ A, int PA,
+                                           const float* __restrict__ B, int PB, int lane) {
+    switch (nb) {  // uniform over the warp
+        case 1:
+            stage_rows<1, kPairStride<1>, 2>(dst, A, PA, lane);
+            stage_rows<1, kPairStride<1>, 2>(dst + 1, B, PB, lane);
+            break;
+        case 2:
+            stage_rows<2, kPairStride<2>, 2>(dst, A, PA, lane);
+            stage_rows<2, kPairStride<2>, 2>(dst + 1, B, PB, lane);
+            break;
+        case 3:
+            stage_rows<3, kPairStride<3>, 2>(dst, A, PA, lane);
+            stage_rows<3, kPairStride<3>, 2>(dst + 1, B, PB, lane);
+            break;
+        default:
+            stage_rows<4, kPairStride<4>, 2>(dst, A, PA, lane);
+            stage_rows<4, kPairStride<4>, 2>(dst + 1, B, PB, lane);
+            break;
     }
     asm volatile("cp.async.commit_group;");
 }
 
-// The Hermite series of the staged expansion at the 32 pixels of a warp tile
+// The Hermite series of two staged expansions at the 32 pixels of a warp tile
 // of G rows and 32 / G columns (lane % (32 / G) is the column).  Pixels of
 // one column have the same y, hence the same Hermite functions h_b(y) and row
 // sums r_a = sum_b C_ab h_b(y), and pixels of one row the same h_a(x).  So
 // one lane per column and row computes the functions; each of a column's G
-// lanes sums one of G rows at a time, four coefficients per shared-memory
-// read; and the lanes exchange the sums.  Every recursion, every row's chain
-// and the outer sum keep their order; the padding adds zeros at the end of
-// each, so the value is hermite_eval's.  One form per number of blocks: a
-// row's reads are in flight together and the column's functions stay in
-// registers; the loop over rows stays rolled (with the descent around it the
-// kernel is bound by instruction fetch once its code outgrows the instruction
-// cache).  (t2, e): 2 t and exp(-t^2), t this lane's coordinate relative to
-// the expansion's centre.
+// lanes sums one of G rows at a time; and the lanes exchange the sums.  The
+// two expansions go through the same instructions, side by side (float_pair):
+// the descent is bound by the number of instructions a warp issues one after
+// the other.  Every recursion, every row's chain and the outer sum keep their
+// order; the padding adds zeros at the end of each, so the values are
+// hermite_eval's.  One form per number of blocks, the larger one's: a row's
+// reads are in flight together and the column's functions stay in registers;
+// the loop over rows stays rolled (with the descent around it the kernel is
+// bound by instruction fetch once its code outgrows the instruction cache).
+// (t2, e): 2 t and exp(-t^2), t the coordinate of this lane's column or row
+// relative to the expansions' centres.
 template <int NB>
-__device__ __forceinline__ float hermite_blocks(WarpTables& wt, const float* coef, int P1, int cols, float t2, float e,
+__device__ __forceinline__ float_pair hermite_pair(WarpTables& wt, const float* coef, int PA, int PB, int cols,
+                                                   float_pair t2, float_pair e, int lane) {
+    const unsigned full = 0xffffffffu;
+    constexpr int S = kPairStride<NB>;
+    const int G = 32 / cols, P1 = max(PA, PB);
+    {
+        ulonglong2* row = reinterpret_cast<ulonglong2*>(wt.hermite[min(lane, 11)]);  // cols + G = 12
+        const bool writes = lane < 12;
+        float_pair h0 = e, h1 = pair_mul(t2, e);
+        float_pair h2 = pair_sub(pair_mul(t2, h1), pair_mul(pair_same(2.0f), h0));
+        float_pair h3 = pair_sub(pair_mul(t2, h2), pair_mul(pair_same(4.0f), h1));
+        if (writes) {
+            row[0] = make_ulonglong2(h0, h1);
+            row[1] = make_ulonglong2(h2, h3);
+        }
+#pragma unroll
+        for (int b = 1; b < NB; ++b) {  // 2 (k - 1): small whole numbers, exact
+            h0 = pair_sub(pair_mul(t2, h3), pair_mul(pair_same(8.0f * b - 2.0f), h2));
+            h1 = pair_sub(pair_mul(t2, h0), pair_mul(pair_same(8.0f * b), h3));
+            h2 = pair_sub(pair_mul(t2, h1), pair_mul(pair_same(8.0f * b + 2.0f), h0));
+            h3 = pair_sub(pair_mul(t2, h2), pair_mul(pair_same(8.0f * b + 4.0f), h1));
+            if (writes) {
+                row[2 * b] = make_ulonglong2(h0, h1);
+                row[2 * b + 1] = make_ulonglong2(h2, h3);
+            }
+        }
+    }
+    __syncwarp();
+    const int col = lane & (cols - 1), mine = lane / cols;
+    ulonglong2 hy[2 * NB];
+#pragma unroll
+    for (int b = 0; b < 2 * NB; ++b) hy[b] = reinterpret_cast<const ulonglong2*>(wt.hermite[col])[b];
+    float_pair w = pair_same(0.0f);
+#pragma unroll 1
+    for (int a0 = 0; a0 < P1; a0 += G) {
+        const int a = a0 + mine;
+        const ulonglong2* C = reinterpret_cast<const ulonglong2*>(coef + min(a, P1 - 1) * S);
+        float_pair r = pair_same(0.0f);
+#pragma unroll
+        for (int b = 0; b < 2 * NB; ++b) {
+            const ulonglong2 c = C[b];
+            r = pair_fma(c.x, hy[b].x, r);
+            r = pair_fma(c.y, hy[b].y, r);
+        }
+        float ra, rb;
+        pair_split(r, ra, rb);
+        if (a >= PA) ra = 0.0f;  // rows that were not copied
+        if (a >= PB) rb = 0.0f;
+#pragma unroll 1
+        for (int q = 0; q < G && a0 + q < P1; q += 4) {
+            const ulonglong2* hx = reinterpret_cast<const ulonglong2*>(wt.hermite[cols + mine]) + ((a0 + q) >> 1);
+            const ulonglong2 u = hx[0], v = hx[1];
+            const int from = col + cols * q;
+            const float_pair h[4] = {u.x, u.y, v.x, v.y};
+#pragma unroll
+            for (int k = 0; k < 4; ++k) {
+                const float xa = __shfl_sync(full, ra, from + k * cols), xb = __shfl_sync(full, rb, from + k * cols);
+                w = pair_fma(h[k], pair_of(xa, xb), w);
+            }
+        }
+    }
+    return w;
+}
+
+// The same for one expansion of five blocks (degree 16).
+__device__ __forceinline__ float hermite_single(WarpTables& wt, const float* coef, int cols, float t2, float e,
                                                 int lane) {
     const unsigned full = 0xffffffffu;
-    constexpr int S = kCoefStride<NB>;
+    constexpr int NB = 5, S = kSingleStride, P1 = kMaxDegree + 1;
     const int G = 32 / cols;
     {
-        float4* row = reinterpret_cast<float4*>(wt.hermite[min(lane, 11)]);  // cols + G = 12
+        float4* row = reinterpret_cast<float4*>(wt.hermite[min(lane, 11)]);
         const bool writes = lane < 12;
         float4 h;
         h.x = e;
@@ -1148,20 +1253,19 @@ __device__ __forceinline__ float hermite_blocks(WarpTables& wt, const float* coe
         h.z = fsub(fmul(t2, h.y), fmul(2.0f, h.x));
         h.w = fsub(fmul(t2, h.z), fmul(4.0f, h.y));
         if (writes) row[0] = h;
-#pragma unroll
-        for (int b = 1; b < NB; ++b) {  // 2 (k - 1): small whole numbers, exact
-            h.x = fsub(fmul(t2, h.w), fmul(8.0f * b - 2.0f, h.z));
-            h.y = fsub(fmul(t2, h.x), fmul(8.0f * b, h.w));
-            h.z = fsub(fmul(t2, h.y), fmul(8.0f * b + 2.0f, h.x));
-            h.w = fsub(fmul(t2, h.z), fmul(8.0f * b + 4.0f, h.y));
+        float k2 = 6.0f;
+#pragma unroll 1
+        for (int b = 1; b < NB; ++b, k2 += 8.0f) {
+            h.x = fsub(fmul(t2, h.w), fmul(k2, h.z));
+            h.y = fsub(fmul(t2, h.x), fmul(k2 + 2.0f, h.w));
+            h.z = fsub(fmul(t2, h.y), fmul(k2 + 4.0f, h.x));
+            h.w = fsub(fmul(t2, h.z), fmul(k2 + 6.0f, h.y));
             if (writes) row[b] = h;
         }
     }
     __syncwarp();
     const int col = lane & (cols - 1), mine = lane / cols;
-    float4 hy[NB];
-#pragma unroll
-    for (int b = 0; b < NB; ++b) hy[b] = reinterpret_cast<const float4*>(wt.hermite[col])[b];
+    const float4* hy = reinterpret_cast<const float4*>(wt.hermite[col]);
     const float4* hx = reinterpret_cast<const float4*>(wt.hermite[cols + mine]);
     float w = 0.0f;
 #pragma unroll 1
@@ -1170,17 +1274,17 @@ __device__ __forceinline__ float hermite_blocks(WarpTables& wt, const float* coe
         float r = 0.0f;
 #pragma unroll
         for (int b = 0; b < NB; ++b) {
-            const float4 c = C[b];
-            r = __fmaf_rn(c.x, hy[b].x, r);
-            r = __fmaf_rn(c.y, hy[b].y, r);
-            r = __fmaf_rn(c.z, hy[b].z, r);
-            r = __fmaf_rn(c.w, hy[b].w, r);
+            const float4 c = C[b], h = hy[b];
+            r = __fmaf_rn(c.x, h.x, r);
+            r = __fmaf_rn(c.y, h.y, r);
+            r = __fmaf_rn(c.z, h.z, r);
+            r = __fmaf_rn(c.w, h.w, r);
         }
         if (a0 + mine >= P1) r = 0.0f;
 #pragma unroll 1
-        for (int s = 0; s < G && a0 + s < P1; s += 4) {
-            const float4 h = hx[(a0 + s) >> 2];
-            const int from = col + cols * s;
+        for (int q = 0; q < G && a0 + q < P1; q += 4) {
+            const float4 h = hx[(a0 + q) >> 2];
+            const int from = col + cols * q;
             const float r0 = __shfl_sync(full, r, from), r1 = __shfl_sync(full, r, from + cols);
             const float r2 = __shfl_sync(full, r, from + 2 * cols), r3 = __shfl_sync(full, r, from + 3 * cols);
             w = __fmaf_rn(h.x, r0, w);
@@ -1190,20 +1294,6 @@ __device__ __forceinline__ float hermite_blocks(WarpTables& wt, const float* coe
         }
     }
     return w;
-}
-// (q, centre): this lane's coordinate and the expansion's along it, see
-// warp_tables; P1 >= 1 coefficients per side.
-__device__ __forceinline__ float hermite_tile(WarpTables& wt, const float* coef, int P1, int cols, float q,
-                                              float centre, float isq, int lane) {
-    const float t = fmul(fsub(q, centre), isq);
-    const float e = det_expf_neg(-fmul(t, t)), t2 = fmul(2.0f, t);
-    switch ((P1 + 3) >> 2) {  // uniform over the warp
-        case 1: return hermite_blocks<1>(wt, coef, P1, cols, t2, e, lane);
-        case 2: return hermite_blocks<2>(wt, coef, P1, cols, t2, e, lane);
-        case 3: return hermite_blocks<3>(wt, coef, P1, cols, t2, e, lane);
-        case 4: return hermite_blocks<4>(wt, coef, P1, cols, t2, e, lane);
-        default: return hermite_blocks<5>(wt, coef, P1, cols, t2, e, lane);
-    }
 }
 
 // node_weight of one lane's own node, the case of an expansion in few
@@ -1240,7 +1330,7 @@ __device__ __forceinline__ float lane_series(const Tree& T, WarpTables& wt, int 
     for (int a = 0; a < P1; a += 4, C += 4 * P1) {
         const int n1 = a + 1 < P1 ? P1 : 0, n2 = a + 2 < P1 ? 2 * P1 : 0, n3 = a + 3 < P1 ? 3 * P1 : 0;
         float r[4] = {0.0f, 0.0f, 0.0f, 0.0f};
-#pragma unroll 2
+#pragma unroll 4
         for (int b = 0; b < P1; ++b) {
             const float h = wt.series[b][lane];
             r[0] = __fmaf_rn(C[b], h, r[0]);
@@ -1264,6 +1354,21 @@ __device__ __forceinline__ float lane_series(const Tree& T, WarpTables& wt, int 
 __device__ __forceinline__ bool within(float4 b, float r2, float qx, float qy) {
     float dx = fsub(qx, fminf(fmaxf(qx, b.x), b.z)), dy = fsub(qy, fminf(fmaxf(qy, b.y), b.w));
     return fadd(fmul(dx, dx), fmul(dy, dy)) < r2;
+}
+
+// Sum of the listed masses [s, t) of this lane, in order.
+__device__ __forceinline__ float range_sum(const WarpTables& wt, const float* val_hi, int lane, int s, int t) {
+    float acc = 0.0f;
+    int i = s;
+    const int top = min(t, kRows);
+#pragma unroll 1
+    for (; i + 4 <= top; i += 4) {
+        float x0 = wt.val[i][lane], x1 = wt.val[i + 1][lane], x2 = wt.val[i + 2][lane], x3 = wt.val[i + 3][lane];
+        acc = fadd(fadd(fadd(fadd(acc, x0), x1), x2), x3);
+    }
+#pragma unroll 1
+    for (; i < t; ++i) acc = fadd(acc, i < kRows ? wt.val[i][lane] : val_hi[i - kRows]);
+    return acc;
 }
 
 // Fills the tables for the lanes of `lanes` (all 32 lanes call this).
@@ -1378,70 +1483,109 @@ __device__ int warp_tables(const Tree& T, float qx, float qy, unsigned lanes, in
             unsigned la = E.x & 0xffffu, lb = E.x >> 16;
             wt.split[o] = (unsigned short)(s + na);
             if ((la & kLinkKind) == kLinkOpen) wt.first[la & kLinkEntry] = (unsigned short)s;
-            else if (la == kLinkEval) wt.eval[s] = make_uint2(E.y, E.w);
+            else if (la == kLinkEval) wt.eval[s] = (unsigned short)(o << 1);
             if ((lb & kLinkKind) == kLinkOpen) wt.first[lb & kLinkEntry] = (unsigned short)(s + na);
-            else if (lb == kLinkEval) wt.eval[s + na] = make_uint2(E.z, E.w);
+            else if (lb == kLinkEval) wt.eval[s + na] = (unsigned short)(o << 1 | 1);
         }
         __syncwarp();
     }
-    // ---- masses.  Lane l < cols computes the Hermite functions of column l,
-    // lane cols + g those of row g; the next expansion's coefficients are
-    // copied meanwhile.
-    const bool columns = lane < cols;
+    // ---- masses.  32 expansions at a time, in order of their number of
+    // blocks: those of five one by one, the others in pairs, then the leaves.
+    // Lane l < cols computes the Hermite functions of column l, lane cols + g
+    // those of row g (for the second of a pair: their exponentials in lanes
+    // 16 on); the next pair's coefficients are copied meanwhile.
     const float qx0 = __shfl_sync(full, qx, 0);
-    const float q = columns ? qy : qx0 + (float)min(lane - cols, 32 / cols - 1);
+    const int role = lane & 15;
+    const bool columns = role < cols;
+    const float q = columns ? qy : qx0 + (float)min(role - cols, 32 / cols - 1);
 #pragma unroll 1
     for (int v0 = 0; v0 < nV; v0 += 32) {
         const int cnt = min(32, nV - v0);
-        const uint2 ev = wt.eval[v0 + min(lane, cnt - 1)];
-        float4 c = T.cen[ev.x];
-        const bool leaf = (int)ev.x >= T.n - 1;
-        const int p = meta_degree(c.w);
-        if (lane < cnt && !leaf) {  // each lane asks for its expansion's lines
-            const float* C = T.coef + meta_offset(c.w);
+        const unsigned entry = wt.eval[v0 + min(lane, cnt - 1)];
+        const uint4 E = wt.open[entry >> 1];
+        const int node = (int)((entry & 1u) ? E.z : E.y);
+        const float4 c0 = T.cen[node];
+        const int p0 = node >= T.n - 1 ? -1 : meta_degree(c0.w);  // -1: a leaf, no coefficients
+        if (lane < cnt && p0 >= 0) {  // each lane asks for its expansion's lines
+            const float* C = T.coef + meta_offset(c0.w);
 #pragma unroll 1
-            for (int e = 0; e < (p + 1) * (p + 1); e += 32) asm volatile("prefetch.global.L2 [%0];" ::"l"(C + e));
+            for (int e = 0; e < (p0 + 1) * (p0 + 1); e += 32) asm volatile("prefetch.global.L2 [%0];" ::"l"(C + e));
         }
-        if (leaf) c.w = make_meta(0, -1);  // no coefficients
+        const int nb0 = lane < cnt ? coef_blocks(p0) : -1;
+        int rank = 0, fives = 0, sums = 0;  // this lane's place; expansions of five blocks; and of any
 #pragma unroll 1
-        for (int k = -1; k < cnt; ++k) {
-            if (k + 1 < cnt) {
-                const float next = __shfl_sync(full, c.w, k + 1);
-                stage(wt.coef[(k + 1) & 1], T.coef + meta_offset(next), meta_degree(next), lane);
+        for (int k = 5; k >= 0; --k) {
+            const unsigned m = __ballot_sync(full, nb0 == k);
+            if (nb0 == k) rank = sums + __popc(m & lt);
+            if (k > 0) sums += __popc(m);
+            if (k == 5) fives = sums;
+        }
+        if (lane < cnt) wt.owner[rank] = lane;
+        __syncwarp();
+        const int mine = wt.owner[min(lane, cnt - 1)];
+        const float cx = __shfl_sync(full, c0.x, mine), cy = __shfl_sync(full, c0.y, mine);
+        const float meta = __shfl_sync(full, c0.w, mine);
+        const unsigned inside = __shfl_sync(full, E.w, mine);
+        auto put = [&](int at, float w) {  // the mass of the expansion at place `at`
+            const int v = v0 + __shfl_sync(full, mine, at);
+            w = ((__shfl_sync(full, inside, at) >> lane) & 1u) ? w : 0.0f;
+            if (v < kRows) wt.val[v][lane] = w;
+            else val_hi[v - kRows] = w;
+        };
+#pragma unroll 1
+        for (int k = 0; k < fives; ++k) {
+            stage_rows<5, kSingleStride, 1>(wt.coef[0], T.coef + meta_offset(__shfl_sync(full, meta, k)),
+                                            kMaxDegree + 1, lane);
+            asm volatile("cp.async.commit_group;\n\tcp.async.wait_group 0;" ::: "memory");
+            const float x = __shfl_sync(full, cx, k), y = __shfl_sync(full, cy, k);
+            __syncwarp();
+            const float t = fmul(fsub(q, columns ? y : x), T.isq);
+            put(k, hermite_single(wt, wt.coef[0], cols, fmul(2.0f, t), det_expf_neg(-fmul(t, t)), lane));
+            __syncwarp();
+        }
+#pragma unroll 1
+        for (int k = fives - 2; k < sums; k += 2) {
+            if (k + 2 < sums) {
+                const float A = __shfl_sync(full, meta, k + 2), B = __shfl_sync(full, meta, min(k + 3, sums - 1));
+                const int pa = meta_degree(A);
+                stage_pair(wt.coef[((k + 2 - fives) >> 1) & 1], coef_blocks(pa), T.coef + meta_offset(A), pa + 1,
+                           T.coef + meta_offset(B), meta_degree(B) + 1, lane);
             }
-            if (k < 0) continue;
-            const unsigned m = __shfl_sync(full, ev.y, k);
-            const float cx = __shfl_sync(full, c.x, k), cy = __shfl_sync(full, c.y, k);
-            const int P1 = meta_degree(__shfl_sync(full, c.w, k)) + 1;
-            if (k + 1 < cnt) asm volatile("cp.async.wait_group 1;" ::: "memory");
+            if (k < fives) continue;
+            const int k1 = min(k + 1, sums - 1), from = lane < 16 ? k : k1;
+            const int PA = meta_degree(__shfl_sync(full, meta, k)) + 1;
+            const int PB = meta_degree(__shfl_sync(full, meta, k1)) + 1;
+            const float x = __shfl_sync(full, cx, from), y = __shfl_sync(full, cy, from);
+            const float t = fmul(fsub(q, columns ? y : x), T.isq);
+            const float e = det_expf_neg(-fmul(t, t)), t2 = fmul(2.0f, t);
+            const float t2b = __shfl_sync(full, t2, role + 16), eb = __shfl_sync(full, e, role + 16);
+            if (k + 2 < sums) asm volatile("cp.async.wait_group 1;" ::: "memory");
             else asm volatile("cp.async.wait_group 0;" ::: "memory");
             __syncwarp();
-            float w = P1 == 0 ? leaf_mass(T, make_float4(cx, cy, 0.0f, 0.0f), qx, qy)
-                              : hermite_tile(wt, wt.coef[k & 1], P1, cols, q, columns ? cy : cx, T.isq, lane);
-            w = ((m >> lane) & 1u) ? w : 0.0f;
-            if (v0 + k < kRows) wt.val[v0 + k][lane] = w;
-            else val_hi[v0 + k - kRows] = w;
-            total = fadd(total, w);
-            __syncwarp();  // the expansion has been read
+            const float* coef = wt.coef[((k - fives) >> 1) & 1];
+            const float_pair tt = pair_of(t2, t2b), ee = pair_of(e, eb);
+            float_pair w;
+            switch (coef_blocks(PA - 1)) {  // uniform over the warp
+                case 1: w = hermite_pair<1>(wt, coef, PA, PB, cols, tt, ee, lane); break;
+                case 2: w = hermite_pair<2>(wt, coef, PA, PB, cols, tt, ee, lane); break;
+                case 3: w = hermite_pair<3>(wt, coef, PA, PB, cols, tt, ee, lane); break;
+                default: w = hermite_pair<4>(wt, coef, PA, PB, cols, tt, ee, lane); break;
+            }
+            float wa, wb;
+            pair_split(w, wa, wb);
+            put(k, wa);
+            if (k1 > k) put(k1, wb);
+            __syncwarp();  // the pair has been read
         }
+#pragma unroll 1
+        for (int k = sums; k < cnt; ++k)
+            put(k, leaf_mass(T, make_float4(__shfl_sync(full, cx, k), __shfl_sync(full, cy, k), 0.0f, 0.0f), qx, qy));
+        __syncwarp();  // owner is written again
     }
     __syncwarp();
+    total = range_sum(wt, val_hi, lane, 0, nV);
+    __syncwarp();
     return nV;
-}
-
-// Sum of the listed masses [s, t) of this lane, in order.
-__device__ __forceinline__ float range_sum(const WarpTables& wt, const float* val_hi, int lane, int s, int t) {
-    float acc = 0.0f;
-    int i = s;
-    const int top = min(t, kRows);
-#pragma unroll 1
-    for (; i + 4 <= top; i += 4) {
-        float x0 = wt.val[i][lane], x1 = wt.val[i + 1][lane], x2 = wt.val[i + 2][lane], x3 = wt.val[i + 3][lane];
-        acc = fadd(fadd(fadd(fadd(acc, x0), x1), x2), x3);
-    }
-#pragma unroll 1
-    for (; i < t; ++i) acc = fadd(acc, i < kRows ? wt.val[i][lane] : val_hi[i - kRows]);
-    return acc;
 }
 
 // A lane's place in the tables: an opened node, the range of its expansions
@@ -1561,7 +1705,8 @@ constexpr int kKnown = 3;  // nodes outside the tables whose child masses a lane
 // KB of code instead of 54).  500k / 1024^2 / K = 8: 2.7-3.3 ms before these
 // tables, 11 ms where one pixel's cache of 160 nodes overflowed; 1.34 with
 // rolled series, 1.22 with one form of the series per number of blocks, 0.96
-// with the tiles in order of the work they hold (kCells).
+// with the tiles in order of the work they hold (kCells), 0.85 with the series
+// in pairs.
 constexpr int kDescentThreads = 64, kDescentBlocks = 6;
 
 // Views of different sizes in one descent launch: blocks [first[v],
