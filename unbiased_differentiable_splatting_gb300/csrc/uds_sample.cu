@@ -2019,8 +2019,8 @@ __global__ void __launch_bounds__(32 * kDescentWarps<KM>, KM <= 16 ? kDescentBlo
                 }
                 {
                     {
-                        // the K smallest keys in order, the earlier candidate
-                        // first among equals (an infinite or NaN key never enters)
+                        // the K smallest keys in order (an infinite or NaN key
+                        // never enters)
                         if (KM <= 16) {
                             if (key < keys[KR - 1]) {
 #pragma unroll UK
@@ -2035,15 +2035,48 @@ __global__ void __launch_bounds__(32 * kDescentWarps<KM>, KM <= 16 ? kDescentBlo
                                 }
                             }
                         } else if (key < last) {
-                            int q = have < K ? have++ : K - 1;
+                            // behind the keys that are not larger; from the end,
+                            // four entries looked at together: one at a time this
+                            // was two thirds of the descent at K = 40
+                            const bool full_list = have == K;
+                            const uint2 out = list[(K - 1) * 32 + lane];  // leaves a full list
+                            int q = full_list ? K - 1 : have++;
+                            unsigned above = full_list ? out.x : 0xffffffffu;  // (no key: a NaN)
+                            bool equal = false, more = true;
 #pragma unroll 1
-                            while (q > 0) {
-                                uint2 x = list[(q - 1) * 32 + lane];
-                                if (!(__uint_as_float(x.x) > key)) break;
-                                list[q * 32 + lane] = x;
-                                --q;
+                            while (more) {
+                                uint2 x[4];
+#pragma unroll
+                                for (int u = 0; u < 4; ++u) x[u] = list[max(q - 1 - u, 0) * 32 + lane];
+#pragma unroll
+                                for (int u = 0; u < 4; ++u) {
+                                    more = more && q > 0 && __uint_as_float(x[u].x) > key;
+                                    if (more) {
+                                        list[q * 32 + lane] = x[u];
+                                        equal |= x[u].x == above;
+                                        above = x[u].x;
+                                        --q;
+                                    }
+                                }
                             }
                             list[q * 32 + lane] = make_uint2(__float_as_uint(key), (unsigned)index);
+                            // the reference's list moves by swaps that pass equal
+                            // keys by: of a run of them the first comes last (or
+                            // leaves the list, if the run reaches past its end)
+                            if (equal) {
+#pragma unroll 1
+                                for (int a = q + 1; a < have; ++a) {
+                                    uint2 first = list[a * 32 + lane];
+#pragma unroll 1
+                                    for (; a + 1 < have; ++a) {
+                                        const uint2 x = list[(a + 1) * 32 + lane];
+                                        if (x.x != first.x) break;
+                                        list[a * 32 + lane] = x;
+                                    }
+                                    if (full_list && a + 1 == K && out.x == first.x) first = out;
+                                    list[a * 32 + lane] = first;
+                                }
+                            }
                             if (have == K) last = __uint_as_float(list[(K - 1) * 32 + lane].x);
                         }
                     }
