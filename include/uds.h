@@ -314,6 +314,10 @@ int uds_mlp_forward_tiles(int R_max, const int* R_dev, const void* X_tiles, cons
 size_t uds_mlp_grad_workspace_size(int R);
 int uds_mlp_grad(int R, const float* X, const float* target, const float* params, float* grad, float* loss,
                  int* err, void* workspace, size_t workspace_bytes, void* stream);
+/* The same over the R rows of X (n x 16) and target (n) numbered by rows
+ * (device; one outside [0, n) counts as a row without gradient or loss). */
+int uds_mlp_grad_rows(int R, const int64_t* rows, int n, const float* X, const float* target, const float* params,
+                      float* grad, float* loss, int* err, void* workspace, size_t workspace_bytes, void* stream);
 int uds_mlp_adam(float* params, float* grad, float* m1, float* m2, int step, float lr, float beta1, float beta2,
                  float eps, void* stream);
 

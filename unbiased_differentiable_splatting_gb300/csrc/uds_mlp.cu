@@ -379,9 +379,16 @@ __global__ void __launch_bounds__(128) k_mlp_forward_tiles(int R, const int* __r
 // shared memory; the backward pass runs dH = dZ * W (B operand: W
 // transposed, staged once) and the weight gradients dW += dZ^T H (operands
 // written transposed, K = the tile's rows) on the tensor cores, the weight
-// gradients accumulating in TMEM across the CTA's tiles, and the bias
-// gradients on the CUDA cores in shared memory; each CTA writes its partial
-// sums once at the end.
+// gradients accumulating in TMEM across the CTA's tiles, while one thread per
+// column sums dZ for the bias gradients (in row order, eight rows per read of
+// the transposed operand); each CTA writes its partial sums once at the end.
+//
+// One CTA per SM (its operands fill the shared memory), so what bounds it is
+// the latency of a tile's chain of seven products and what lies between them.
+// Two threads share a row, half its columns each, and move 16 bytes at a time;
+// the batch's rows are read where they lie (rows: their numbers).  65536 rows:
+// 51 us; with one thread per row, bias sums by loops over the tile's rows and
+// single elements moved 65 us, after 39 us of gathering the batch.
 struct MlpGradSmem {
     __align__(1024) unsigned char w1[mlp::kHid * mlp::kIn * 2];
     __align__(1024) unsigned char w2[mlp::kHid * mlp::kHid * 2];
@@ -398,9 +405,9 @@ struct MlpGradSmem {
     // zero) and H^T (or X^T), K = the tile's 128 rows
     __align__(1024) unsigned char at[mlp::kTile * mlp::kTile * 2];
     __align__(1024) unsigned char bt[mlp::kHid * mlp::kTile * 2];
-    float dz4f[mlp::kTile][2];
+    __align__(1024) unsigned char xt[mlp::kIn * mlp::kTile * 2];
+    __align__(16) float dz4f[mlp::kTile];
     float bias[3 * mlp::kHid + mlp::kOut];
-    float dbias[3 * mlp::kHid + mlp::kOut];
     float wloss[4];
     uint64_t mbar;
     uint32_t taddr;
@@ -409,6 +416,8 @@ struct MlpGradSmem {
 __device__ __forceinline__ float get_bf16(const unsigned char* base, uint32_t off) {
     return __bfloat162float(*reinterpret_cast<const __nv_bfloat16*>(base + off));
 }
+
+constexpr int kGradThreads = 256;
 
 // 8 consecutive K elements (k0 multiple of 8) of row r of a K-major operand.
 __device__ __forceinline__ void get8(const unsigned char* base, int r, int k0, int K, float (&v)[8]) {
@@ -422,23 +431,29 @@ __device__ __forceinline__ void get8(const unsigned char* base, int r, int k0, i
     }
 }
 
-// Stage W (R x K, fp32 row-major) transposed: operand of K rows x R columns.
-__device__ __forceinline__ void stage_transposed(unsigned char* dst, const float* src, int R, int K) {
-    for (int i = threadIdx.x; i < R * K; i += blockDim.x) {
-        int r = i / K, k = i % K;
-        put_bf16(dst, tc::kmajor_offset(k, r, R), src[i]);
+// Stage W (R x K, fp32 row-major) as bf16 operand and (dst_t) transposed, an
+// operand of K rows x R columns.
+template <int R, int K>
+__device__ __forceinline__ void stage_both(unsigned char* dst, unsigned char* dst_t, const float* __restrict__ src) {
+#pragma unroll 4
+    for (int i = threadIdx.x; i < R * K; i += kGradThreads) {
+        const float v = src[i];
+        put_bf16(dst, tc::kmajor_offset(i / K, i % K, K), v);
+        if (dst_t) put_bf16(dst_t, tc::kmajor_offset(i % K, i / K, R), v);
     }
 }
 
-// Row r of a K-major [128 x K] bf16 tile becomes column r of the K-major
-// [K x 128] tile dst (a transposed operand whose K is the tile's rows).
-__device__ __forceinline__ void transpose_row(unsigned char* dst, const unsigned char* src, int r, int K) {
-    for (int k0 = 0; k0 < K; k0 += 8) {
-        uint4 q = *reinterpret_cast<const uint4*>(src + tc::kmajor_offset(r, k0, K));
+// Elements [k0, k0 + n) of row r of a K-major [128 x K] bf16 tile become
+// column r of the K-major [K x 128] tile dst (a transposed operand whose K is
+// the tile's rows).
+__device__ __forceinline__ void transpose_row(unsigned char* dst, const unsigned char* src, int r, int K, int k0,
+                                              int n) {
+    for (int k = k0; k < k0 + n; k += 8) {
+        uint4 q = *reinterpret_cast<const uint4*>(src + tc::kmajor_offset(r, k, K));
         const unsigned short* e = reinterpret_cast<const unsigned short*>(&q);
 #pragma unroll
         for (int i = 0; i < 8; ++i)
-            *reinterpret_cast<unsigned short*>(dst + tc::kmajor_offset(k0 + i, r, mlp::kTile)) = e[i];
+            *reinterpret_cast<unsigned short*>(dst + tc::kmajor_offset(k + i, r, mlp::kTile)) = e[i];
     }
 }
 
@@ -459,34 +474,37 @@ __device__ __forceinline__ void mma_wgrad(uint32_t taddr, uint32_t col, const un
 constexpr uint32_t kColAct = 0, kColW4 = 64, kColW3 = 128, kColW2 = 192, kColW1 = 256, kGradCols = 512;
 
 // Each block writes its partial gradients (and loss) to its own slice of
-// part (kParams + 1 floats per block, every slot written by one thread);
-// k_mlp_grad_reduce then sums the slices in block order, so the gradient does
-// not depend on the order in which blocks finish.
-constexpr int kGradPart = mlp::kParams + 1;
+// part (the parameters and the loss, padded to 16 bytes; every slot written by
+// one thread); k_mlp_grad_reduce then sums the slices in block order, so the
+// gradient does not depend on the order in which blocks finish.
+constexpr int kGradPart = (mlp::kParams + 1 + 3) / 4 * 4;
 
-__global__ void __launch_bounds__(128) k_mlp_grad(int R, const float* __restrict__ X, const float* __restrict__ target,
-                                                  float scale, const float* __restrict__ P,
-                                                  float* __restrict__ part, int* __restrict__ err) {
+// rows: the numbers of the batch's rows of X and target, of which there are n
+// (null: rows 0 .. R - 1).
+__global__ void __launch_bounds__(kGradThreads, 1)
+    k_mlp_grad(int R, const long long* __restrict__ rows, int n, const float* __restrict__ X,
+               const float* __restrict__ target, float scale, const float* __restrict__ P, float* __restrict__ part,
+               int* __restrict__ err) {
     extern __shared__ __align__(1024) unsigned char s_raw[];
     MlpGradSmem& S = *reinterpret_cast<MlpGradSmem*>(s_raw);
     using namespace mlp;
-    int tid = threadIdx.x, warp = tid >> 5;
-    stage_matrix(S.w1, P + oW1, kHid, kIn);
-    stage_matrix(S.w2, P + oW2, kHid, kHid);
-    stage_matrix(S.w3, P + oW3, kHid, kHid);
-    stage_matrix(S.w4, P + oW4, kOut, kHid);
-    stage_transposed(S.w2t, P + oW2, kHid, kHid);
-    stage_transposed(S.w3t, P + oW3, kHid, kHid);
-    stage_transposed(S.w4t, P + oW4, kOut, kHid);
-    for (int i = tid; i < 3 * kHid + kOut; i += 128) {
+    // thread: row `r` of the tile, columns of half `half`; a warp reads the
+    // TMEM lanes of its place in its warpgroup
+    const int tid = threadIdx.x, warp = tid >> 5, r = tid & (kTile - 1), half = tid / kTile;
+    stage_both<kHid, kIn>(S.w1, nullptr, P + oW1);
+    stage_both<kHid, kHid>(S.w2, S.w2t, P + oW2);
+    stage_both<kHid, kHid>(S.w3, S.w3t, P + oW3);
+    stage_both<kOut, kHid>(S.w4, S.w4t, P + oW4);
+    for (int i = tid; i < 3 * kHid + kOut; i += kGradThreads)
         S.bias[i] = P[oB1 + (i < kHid ? i : i < 2 * kHid ? (oB2 - oB1) + i - kHid
                                               : i < 3 * kHid ? (oB3 - oB1) + i - 2 * kHid : (oB4 - oB1) + i - 3 * kHid)];
-        S.dbias[i] = 0.0f;
-    }
-    // dz4 columns 2..15 stay zero; so do rows 64 .. 127 of the transposed
-    // dZ operand
-    for (int i = tid; i < kTile * kOut * 2 / 16; i += 128) reinterpret_cast<uint4*>(S.dz4)[i] = make_uint4(0, 0, 0, 0);
-    for (int i = tid; i < kTile * kTile * 2 / 16; i += 128) reinterpret_cast<uint4*>(S.at)[i] = make_uint4(0, 0, 0, 0);
+    // dz4 columns 2..15 stay zero; so do rows 64 .. 127 of the transposed dZ
+    // operand
+    auto clear = [&](unsigned char* p, int bytes) {
+        for (int i = tid; i < bytes / 16; i += kGradThreads) reinterpret_cast<uint4*>(p)[i] = make_uint4(0, 0, 0, 0);
+    };
+    clear(S.dz4, kTile * kOut * 2);
+    clear(S.at, kTile * kTile * 2);
     if (tid == 0) tc::mbar_init(&S.mbar, 1);
     if (warp == 0) {
         tc::tmem_alloc(&S.taddr, kGradCols);
@@ -497,26 +515,46 @@ __global__ void __launch_bounds__(128) k_mlp_grad(int R, const float* __restrict
     __syncthreads();
     tc::fence_after_sync();
     uint32_t taddr = S.taddr;
-    uint32_t lane_base = taddr + ((uint32_t)(warp * 32) << 16);
+    uint32_t lane_base = taddr + ((uint32_t)((warp & 3) * 32) << 16);
     uint32_t phase = 0;
     bool ok = true;
     bool first = true;  // the first tile starts the weight-gradient accumulators
     float lsum = 0.0f;
+    float db[4] = {0.0f, 0.0f, 0.0f, 0.0f};  // bias gradients of layers 1 to 3: column tid; of 4: thread 128
+    // the sum of column tid of dZ, from its row of the transposed operand,
+    // while the products run
+    auto column_sum = [&](float& b) {
+        if (tid >= kHid) return;
+        float sum = 0.0f;
+#pragma unroll 4
+        for (int k = 0; k < kTile; k += 8) {
+            float v[8];
+            get8(S.at, tid, k, kTile, v);
+#pragma unroll
+            for (int c = 0; c < 8; ++c) sum += v[c];
+        }
+        b += sum;
+    };
     int tiles = (R + kTile - 1) / kTile;
     for (int t = blockIdx.x; t < tiles && ok; t += gridDim.x) {
-        int row = t * kTile + tid;
+        int row = t * kTile + r;
         bool valid = row < R;
+        if (valid && rows) {
+            const long long at = rows[row];
+            valid = at >= 0 && at < n;
+            row = (int)at;
+        }
         {
-            float xv[kIn];
-            const float4* xr = reinterpret_cast<const float4*>(X + (size_t)row * kIn);
+            float xv[8];
+            const float4* xr = reinterpret_cast<const float4*>(X + (size_t)row * kIn) + 2 * half;
 #pragma unroll
-            for (int q = 0; q < kIn / 4; ++q) {
+            for (int q = 0; q < 2; ++q) {
                 float4 f4 = valid ? xr[q] : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
                 xv[4 * q] = f4.x; xv[4 * q + 1] = f4.y; xv[4 * q + 2] = f4.z; xv[4 * q + 3] = f4.w;
             }
-            put8_bf16(S.x, tid, 0, kIn, xv);
-            put8_bf16(S.x, tid, 8, kIn, xv + 8);
+            put8_bf16(S.x, r, 8 * half, kIn, xv);
         }
+        const float p = valid && half == 0 ? target[row] : 0.0f;
         tc::fence_async_smem();
         __syncthreads();
         // ---- forward
@@ -526,13 +564,14 @@ __global__ void __launch_bounds__(128) k_mlp_grad(int R, const float* __restrict
         for (int l = 0; l < 3 && ok; ++l) {
             ok = mlp_layer(taddr, a, ws[l], K, kHid, &S.mbar, phase);
             if (!ok) break;
-            for (int c0 = 0; c0 < kHid; c0 += 16) {
-                float v[16];
-                tc::tmem_ld16(lane_base + (uint32_t)c0, v);
 #pragma unroll
-                for (int c = 0; c < 16; ++c) v[c] = fmaxf(v[c] + S.bias[l * kHid + c0 + c], 0.0f);
-                put8_bf16(S.h[l], tid, c0, kHid, v);
-                put8_bf16(S.h[l], tid, c0 + 8, kHid, v + 8);
+            for (int c0 = 0; c0 < 32; c0 += 16) {
+                float v[16];
+                tc::tmem_ld16(lane_base + (uint32_t)(32 * half + c0), v);
+#pragma unroll
+                for (int c = 0; c < 16; ++c) v[c] = fmaxf(v[c] + S.bias[l * kHid + 32 * half + c0 + c], 0.0f);
+                put8_bf16(S.h[l], r, 32 * half + c0, kHid, v);
+                put8_bf16(S.h[l], r, 32 * half + c0 + 8, kHid, v + 8);
             }
             tc::fence_before_sync();
             tc::fence_async_smem();
@@ -546,32 +585,32 @@ __global__ void __launch_bounds__(128) k_mlp_grad(int R, const float* __restrict
         {
             float v[16];
             tc::tmem_ld16(lane_base, v);
-            float z0 = v[0] + S.bias[3 * kHid], z1 = v[1] + S.bias[3 * kHid + 1];
-            float m = fmaxf(z0, z1);
-            float e0 = __expf(z0 - m), e1 = __expf(z1 - m);
-            float q0 = e0 / (e0 + e1);
-            float p = valid ? target[row] : 0.0f;
-            float d0 = valid ? (q0 - p) * scale : 0.0f;
-            if (valid) {
-                float lz = m + __logf(e0 + e1);
-                lsum += -(p * (z0 - lz) + (1.0f - p) * (z1 - lz));
+            if (half == 0) {
+                float z0 = v[0] + S.bias[3 * kHid], z1 = v[1] + S.bias[3 * kHid + 1];
+                float m = fmaxf(z0, z1);
+                float e0 = __expf(z0 - m), e1 = __expf(z1 - m);
+                float q0 = e0 / (e0 + e1);
+                float d0 = valid ? (q0 - p) * scale : 0.0f;
+                if (valid) {
+                    float lz = m + __logf(e0 + e1);
+                    lsum += -(p * (z0 - lz) + (1.0f - p) * (z1 - lz));
+                }
+                S.dz4f[r] = d0;
+                put_bf16(S.dz4, tc::kmajor_offset(r, 0, kOut), d0);
+                put_bf16(S.dz4, tc::kmajor_offset(r, 1, kOut), -d0);
             }
-            S.dz4f[tid][0] = d0;
-            S.dz4f[tid][1] = -d0;
-            put_bf16(S.dz4, tc::kmajor_offset(tid, 0, kOut), d0);
-            put_bf16(S.dz4, tc::kmajor_offset(tid, 1, kOut), -d0);
         }
         tc::fence_before_sync();
         __syncthreads();
         // ---- backward.  Each layer stages its weight-gradient operands (dZ^T
         // and the layer input transposed), then one thread issues the input-
         // gradient GEMM dH = dZ W and the weight-gradient GEMM dW += dZ^T H
-        // on the tensor cores, while the CUDA cores sum the bias gradients.
+        // on the tensor cores.
         // layer 4: dZ4^T is 16 rows (2 nonzero); rows 16 .. 63 are cleared
-        transpose_row(S.at, S.dz4, tid, kOut);
-        for (int i = tid; i < 48 * kTile * 2 / 16; i += 128)
-            reinterpret_cast<uint4*>(S.at + 16 * kTile * 2)[i] = make_uint4(0, 0, 0, 0);
-        transpose_row(S.bt, S.h[2], tid, kHid);
+        transpose_row(S.at, S.dz4, r, kOut, 8 * half, 8);
+        clear(S.at + 16 * kTile * 2, 48 * kTile * 2);
+        transpose_row(S.bt, S.h[2], r, kHid, 32 * half, 32);
+        transpose_row(S.xt, S.x, r, kIn, 8 * half, 8);
         tc::fence_async_smem();
         __syncthreads();
         if (tid == 0) {
@@ -583,37 +622,48 @@ __global__ void __launch_bounds__(128) k_mlp_grad(int R, const float* __restrict
             mma_wgrad(taddr, kColW4, S.at, S.bt, kHid, !first);
             tc::mma_commit(&S.mbar);
         }
-        if (tid < 2) {
-            float sb = 0.0f;
-            for (int r = 0; r < kTile; ++r) sb += S.dz4f[r][tid];
-            S.dbias[3 * kHid + tid] += sb;
+        if (tid == kTile) {
+            float sum = 0.0f;
+#pragma unroll 4
+            for (int k = 0; k < kTile; k += 4) {
+                const float4 d = *reinterpret_cast<const float4*>(&S.dz4f[k]);
+                sum = (((sum + d.x) + d.y) + d.z) + d.w;
+            }
+            db[3] += sum;
         }
         ok = tc::mbar_wait(&S.mbar, phase & 1u, kWaitLimit);
         ++phase;
         tc::fence_after_sync();
         ok = __syncthreads_and(ok) != 0;
         if (!ok) break;
-        // dZ3 = dH3 * relu'(Z3) -> dz[0]
-        for (int c0 = 0; c0 < kHid; c0 += 16) {
-            float v[16];
-            tc::tmem_ld16(lane_base + kColAct + (uint32_t)c0, v);
+        // dZ = dH * relu'(Z) into a dz buffer
+        auto input_gradient = [&](unsigned char* dz, const unsigned char* h) {
 #pragma unroll
-            for (int c = 0; c < 16; ++c) {
-                float hv = get_bf16(S.h[2], tc::kmajor_offset(tid, c0 + c, kHid));
-                put_bf16(S.dz[0], tc::kmajor_offset(tid, c0 + c, kHid), hv > 0.0f ? v[c] : 0.0f);
+            for (int c0 = 0; c0 < 32; c0 += 16) {
+                float v[16];
+                tc::tmem_ld16(lane_base + kColAct + (uint32_t)(32 * half + c0), v);
+#pragma unroll
+                for (int q = 0; q < 16; q += 8) {
+                    float hv[8];
+                    get8(h, r, 32 * half + c0 + q, kHid, hv);
+#pragma unroll
+                    for (int c = 0; c < 8; ++c) hv[c] = hv[c] > 0.0f ? v[q + c] : 0.0f;
+                    put8_bf16(dz, r, 32 * half + c0 + q, kHid, hv);
+                }
             }
-        }
-        tc::fence_before_sync();
-        tc::fence_async_smem();
-        __syncthreads();
+            tc::fence_before_sync();
+            tc::fence_async_smem();
+            __syncthreads();
+        };
+        input_gradient(S.dz[0], S.h[2]);
         // layers 3 and 2
         const unsigned char* wt[2] = {S.w3t, S.w2t};
         const uint32_t wcol[2] = {kColW3, kColW2};
         for (int l = 0; l < 2 && ok; ++l) {
             const unsigned char* dzl = S.dz[l];
             const unsigned char* hprev = S.h[1 - l];  // H2 for layer 3, H1 for layer 2
-            transpose_row(S.at, dzl, tid, kHid);
-            transpose_row(S.bt, hprev, tid, kHid);
+            transpose_row(S.at, dzl, r, kHid, 32 * half, 32);
+            transpose_row(S.bt, hprev, r, kHid, 32 * half, 32);
             tc::fence_async_smem();
             __syncthreads();
             if (tid == 0) {
@@ -625,93 +675,70 @@ __global__ void __launch_bounds__(128) k_mlp_grad(int R, const float* __restrict
                 mma_wgrad(taddr, wcol[l], S.at, S.bt, kHid, !first);
                 tc::mma_commit(&S.mbar);
             }
-            if (tid < kHid) {
-                float sb = 0.0f;
-                for (int r = 0; r < kTile; ++r) sb += get_bf16(dzl, tc::kmajor_offset(r, tid, kHid));
-                S.dbias[(2 - l) * kHid + tid] += sb;
-            }
+            column_sum(l ? db[1] : db[2]);
             ok = tc::mbar_wait(&S.mbar, phase & 1u, kWaitLimit);
             ++phase;
             tc::fence_after_sync();
             ok = __syncthreads_and(ok) != 0;
             if (!ok) break;
-            // dZ_{l-1} = dH * relu'(Z_{l-1}) -> the other dz buffer
-            unsigned char* dzn = S.dz[1 - l];
-            for (int c0 = 0; c0 < kHid; c0 += 16) {
-                float v[16];
-                tc::tmem_ld16(lane_base + kColAct + (uint32_t)c0, v);
-#pragma unroll
-                for (int c = 0; c < 16; ++c) {
-                    float hv = get_bf16(hprev, tc::kmajor_offset(tid, c0 + c, kHid));
-                    put_bf16(dzn, tc::kmajor_offset(tid, c0 + c, kHid), hv > 0.0f ? v[c] : 0.0f);
-                }
-            }
-            tc::fence_before_sync();
-            tc::fence_async_smem();
-            __syncthreads();
+            input_gradient(S.dz[1 - l], hprev);  // -> the other dz buffer
         }
         if (!ok) break;
         // layer 1: dW1 += dZ1^T X (dZ1 is in dz[0] after two swaps), db1
-        {
-            const unsigned char* dz1 = S.dz[0];
-            transpose_row(S.at, dz1, tid, kHid);
-            transpose_row(S.bt, S.x, tid, kIn);
-            tc::fence_async_smem();
-            __syncthreads();
-            if (tid == 0) {
-                tc::fence_after_sync();
-                mma_wgrad(taddr, kColW1, S.at, S.bt, kIn, !first);
-                tc::mma_commit(&S.mbar);
-            }
-            if (tid < kHid) {
-                float sb = 0.0f;
-                for (int r = 0; r < kTile; ++r) sb += get_bf16(dz1, tc::kmajor_offset(r, tid, kHid));
-                S.dbias[tid] += sb;
-            }
-            ok = tc::mbar_wait(&S.mbar, phase & 1u, kWaitLimit);
-            ++phase;
+        transpose_row(S.at, S.dz[0], r, kHid, 32 * half, 32);
+        tc::fence_async_smem();
+        __syncthreads();
+        if (tid == 0) {
             tc::fence_after_sync();
-            ok = __syncthreads_and(ok) != 0;
+            mma_wgrad(taddr, kColW1, S.at, S.xt, kIn, !first);
+            tc::mma_commit(&S.mbar);
         }
+        column_sum(db[0]);
+        ok = tc::mbar_wait(&S.mbar, phase & 1u, kWaitLimit);
+        ++phase;
+        tc::fence_after_sync();
+        ok = __syncthreads_and(ok) != 0;
         first = false;
     }
     if (!ok && (tid & 31) == 0) atomicExch(err, 1);
-    // this block's partial sums: one writer per slot, no atomics.  Thread t
-    // reads TMEM lane t: row t of each weight-gradient accumulator (rows
-    // 64 .. 127 are the zero padding)
+    // this block's partial sums: one writer per slot, no atomics.  Row r of
+    // each weight-gradient accumulator is TMEM lane r (rows 64 .. 127 are the
+    // zero padding)
     float* G = part + (size_t)blockIdx.x * kGradPart;
     if (ok) {
-        for (int c0 = 0; c0 < kHid; c0 += 16) {
+        auto put16 = [&](float* to, const float* v) {
+#pragma unroll
+            for (int c = 0; c < 16; c += 4)
+                *reinterpret_cast<float4*>(to + c) = make_float4(v[c], v[c + 1], v[c + 2], v[c + 3]);
+        };
+        for (int c0 = 32 * half; c0 < 32 * half + 32; c0 += 16) {
             float v4[16], v3[16], v2[16];
             tc::tmem_ld16(lane_base + kColW4 + (uint32_t)c0, v4);
             tc::tmem_ld16(lane_base + kColW3 + (uint32_t)c0, v3);
             tc::tmem_ld16(lane_base + kColW2 + (uint32_t)c0, v2);
-            if (tid < kHid) {
-#pragma unroll
-                for (int c = 0; c < 16; ++c) {
-                    G[oW3 + tid * kHid + c0 + c] = v3[c];
-                    G[oW2 + tid * kHid + c0 + c] = v2[c];
-                    if (tid < kLogits) G[oW4 + tid * kHid + c0 + c] = v4[c];
-                }
+            if (r < kHid) {
+                put16(G + oW3 + r * kHid + c0, v3);
+                put16(G + oW2 + r * kHid + c0, v2);
+                if (r < kLogits) put16(G + oW4 + r * kHid + c0, v4);
             }
         }
         float v1[16];
         tc::tmem_ld16(lane_base + kColW1, v1);
-        if (tid < kHid) {
-#pragma unroll
-            for (int c = 0; c < 16; ++c) G[oW1 + tid * kIn + c] = v1[c];
-        }
+        if (half == 0 && r < kHid) put16(G + oW1 + r * kIn, v1);
+    }
+    if (tid < kHid) {
+        G[oB1 + tid] = db[0];
+        G[oB2 + tid] = db[1];
+        G[oB3 + tid] = db[2];
+    }
+    if (tid == kTile) {
+        G[oB4] = db[3];
+        G[oB4 + 1] = -db[3];  // the second logit's gradients are the first's negated
     }
     for (int o = 16; o > 0; o >>= 1) lsum += __shfl_xor_sync(0xffffffffu, lsum, o);
-    if ((tid & 31) == 0) S.wloss[warp] = lsum;
+    if ((tid & 31) == 0 && warp < 4) S.wloss[warp] = lsum;
     tc::fence_before_sync();
     __syncthreads();
-    for (int i = tid; i < kHid; i += 128) {
-        G[oB1 + i] = S.dbias[i];
-        G[oB2 + i] = S.dbias[kHid + i];
-        G[oB3 + i] = S.dbias[2 * kHid + i];
-    }
-    if (tid < 2) G[oB4 + tid] = S.dbias[3 * kHid + tid];
     if (tid == 0) G[kParams] = (((S.wloss[0] + S.wloss[1]) + S.wloss[2]) + S.wloss[3]) * scale;
     if (warp == 0) tc::tmem_dealloc(taddr, kGradCols);
 }
@@ -804,11 +831,11 @@ static int mlp_grad_blocks(int R) {
 
 extern "C" size_t uds_mlp_grad_workspace_size(int R) {
     if (R <= 0) return 0;
-    return sizeof(float) * (size_t)uds::kGradPart * (size_t)mlp_grad_blocks(R);
+    return 16 + sizeof(float) * (size_t)uds::kGradPart * (size_t)mlp_grad_blocks(R);  // (slices start on 16 bytes)
 }
 
-extern "C" int uds_mlp_grad(int R, const float* X, const float* target, const float* params, float* grad,
-                            float* loss, int* err, void* workspace, size_t workspace_bytes, void* stream) {
+static int mlp_grad(int R, const long long* rows, int n, const float* X, const float* target, const float* params,
+                    float* grad, float* loss, int* err, void* workspace, size_t workspace_bytes, void* stream) {
     using namespace uds;
     if (R < 0 || (R > 0 && (!X || !target || !params || !grad || !loss)) || !err) return UDS_ERR_ARGUMENT;
     if (R == 0) return UDS_OK;
@@ -820,11 +847,24 @@ extern "C" int uds_mlp_grad(int R, const float* X, const float* target, const fl
         attr = true;
     }
     int grid = mlp_grad_blocks(R);
-    float* part = reinterpret_cast<float*>(workspace);
+    float* part = reinterpret_cast<float*>((reinterpret_cast<uintptr_t>(workspace) + 15) & ~(uintptr_t)15);
     cudaStream_t s = as_stream(stream);
-    k_mlp_grad<<<grid, 128, smem, s>>>(R, X, target, 1.0f / (float)R, params, part, err);
+    k_mlp_grad<<<grid, kGradThreads, smem, s>>>(R, rows, n, X, target, 1.0f / (float)R, params, part, err);
     k_mlp_grad_reduce<<<cdiv(kGradPart, 256), 256, 0, s>>>(grid, part, grad, loss);
     return launch_status(2);
+}
+
+extern "C" int uds_mlp_grad(int R, const float* X, const float* target, const float* params, float* grad,
+                            float* loss, int* err, void* workspace, size_t workspace_bytes, void* stream) {
+    return mlp_grad(R, nullptr, R, X, target, params, grad, loss, err, workspace, workspace_bytes, stream);
+}
+
+extern "C" int uds_mlp_grad_rows(int R, const int64_t* rows, int n, const float* X, const float* target,
+                                 const float* params, float* grad, float* loss, int* err, void* workspace,
+                                 size_t workspace_bytes, void* stream) {
+    if (R > 0 && (!rows || n <= 0)) return UDS_ERR_ARGUMENT;
+    return mlp_grad(R, reinterpret_cast<const long long*>(rows), n, X, target, params, grad, loss, err, workspace,
+                    workspace_bytes, stream);
 }
 
 extern "C" int uds_mlp_adam(float* params, float* grad, float* m1, float* m2, int step, float lr, float beta1,

@@ -77,9 +77,8 @@ class ProposalNet:
         ws = Workspace.get(self.device, L.uds_mlp_grad_workspace_size(nb), "mlp_grad")
         for i in range(steps):
             sel = torch.randint(0, n, (nb,), device=self.device, generator=g)
-            xb, tb = X[sel].contiguous(), target[sel].contiguous()
-            check(L.uds_mlp_grad(xb.shape[0], ptr(xb), ptr(tb), ptr(self.params), ptr(self.grad), ptr(losses[i:]),
-                                 ptr(self._err), ptr(ws), ws.numel(), s), "mlp grad")
+            check(L.uds_mlp_grad_rows(nb, ptr(sel), n, ptr(X), ptr(target), ptr(self.params), ptr(self.grad),
+                                      ptr(losses[i:]), ptr(self._err), ptr(ws), ws.numel(), s), "mlp grad")
             self.steps += 1
             check(L.uds_mlp_adam(ptr(self.params), ptr(self.grad), ptr(self.m1), ptr(self.m2), self.steps, lr, 0.9,
                                  0.999, 1e-8, s), "mlp adam")
