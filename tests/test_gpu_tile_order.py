@@ -44,3 +44,27 @@ def test_views(smp):
     many = smp.sample(w, h, f, rep(p), rep(n), None, rep(s), 8, 0.0, 0.01, seed=1)
     one = smp.sample(w, h, f, p, n, None, s, 8, 0.0, 0.01, seed=1)
     assert torch.equal(many[:1], one) and (many[..., 0] >= 0).all()
+
+
+def test_descent_of_another_size(smp):
+    """A tree built for one image, descended for images of other sizes: every
+    pixel that the descent for the tree's own size takes, and as it does."""
+    W, H = 70, 90
+    f, p, n, s = scene(W, H)
+    prm = smp.params(W, H, f, p, s, 8, 0.0, 0.01, 1)
+    L = smp.load()
+    ws = torch.empty(L.uds_sample_workspace_size(prm), dtype=torch.uint8, device="cuda")
+    stream = torch.cuda.current_stream().cuda_stream
+    assert L.uds_tree_build(prm, 0, p.data_ptr(), n.data_ptr(), s.data_ptr(), None, None, None, None, None, None, None,
+                            None, None, None, None, ws.data_ptr(), ws.numel(), stream) == 0
+
+    def descend(w, h):
+        q = smp.params(w, h, f, p, s, 8, 0.0, 0.01, 1)
+        idx = torch.full((w, h, 8), -1, dtype=torch.int32, device="cuda")
+        assert L.uds_sample_descent(q, 0, None, idx.data_ptr(), ws.data_ptr(), ws.numel(), stream) == 0
+        return idx
+
+    own = descend(W, H)
+    assert torch.equal(own, smp.sample(W, H, f, p, n, None, s, 8, 0.0, 0.01, seed=1)[0])
+    assert torch.equal(descend(33, H), own[:33])  # (the same pixel numbers, hence uniforms)
+    assert (descend(200, 40)[:W, :, 0] >= 0).all()

@@ -51,6 +51,7 @@ struct ViewState {            // per-view device scalars (lives in the workspace
     unsigned coef_used;
     float isq;                // 1 / sq (the series' scaled offsets multiply by it)
     int failed;               // a wait ran out: the view samples nothing (see look_back)
+    int W, H;                 // of the image the tree was built for
     unsigned ticket[kPasses + 3];  // blocks started: k_sort_pass's, k_cull's, k_p2m's; done: k_bandwidth's
 };
 
@@ -78,12 +79,13 @@ static unsigned cell_blocks(int W, int H, dim3 block) {  // blocks that cover ev
     return (unsigned)(cell_columns(W, sh) * cell_columns(H, sh)) * ((1u << sh) / block.x) * ((1u << sh) / block.y);
 }
 // The first pixel (row i along W, column j along H) of a block of a view, its
-// place among the view's blocks given (order null: cells in their own order).
-__device__ __forceinline__ void cell_block(const unsigned short* __restrict__ order, int W, int H, unsigned at, int& i,
-                                           int& j) {
+// place among the view's blocks given (cells in their own order where the
+// tree was built for an image of another size).
+__device__ __forceinline__ void cell_block(const unsigned short* __restrict__ order, const ViewState* vs, int W, int H,
+                                           unsigned at, int& i, int& j) {
     const int sh = cell_shift(W, H);
     const unsigned across = (1u << sh) / blockDim.x, per = across * ((1u << sh) / blockDim.y);
-    const int cell = order ? order[at / per] : (int)(at / per), columns = cell_columns(H, sh);
+    const int cell = vs->W == W && vs->H == H ? order[at / per] : (int)(at / per), columns = cell_columns(H, sh);
     i = ((cell / columns) << sh) + (int)(at % per / across * blockDim.y);
     j = ((cell % columns) << sh) + (int)(at % across * blockDim.x);
 }
@@ -206,8 +208,9 @@ __device__ __forceinline__ float splat_bandwidth(float W, float H, float f, cons
 }
 
 // h (or its override), the cull radius and bounds (samplingCuda.cu:244-258)
-__device__ void view_setup(ViewState* vs, unsigned long long hsum, unsigned long long hcount, float override_h, float W,
-                           float H, float precision, uds_view_stats* st) {
+__device__ void view_setup(ViewState* vs, unsigned long long hsum, unsigned long long hcount, float override_h,
+                           int width, int height, float precision, uds_view_stats* st) {
+    const float W = (float)width, H = (float)height;
     float h;
     if (override_h > 0.0f) h = override_h;
     else if (hcount == 0) h = __int_as_float(0x7fc00000);
@@ -217,6 +220,8 @@ __device__ void view_setup(ViewState* vs, unsigned long long hsum, unsigned long
     double b = (double)det_logf(norm);
     float r = (float)dmul(dmul(1.4142135623730951, (double)h), __dsqrt_rn(dsub(a, b)));
     vs->h = h;
+    vs->W = width;
+    vs->H = height;
     vs->radius = r;
     vs->lo_x = -r;
     vs->hi_x = fadd(W, r);
@@ -285,7 +290,7 @@ __global__ void __launch_bounds__(kTileThreads) k_bandwidth(int N, Batch bt, con
         if (atomicAdd(&vs->ticket[kPasses + 2], 1u) == gridDim.x - 1) {
             __threadfence();
             view_setup(vs, atomicAdd(&vs->hsum, 0ull), atomicAdd(&vs->hcount, 0ull),
-                       h_override ? h_override[view] : 0.0f, W, H, precision, stats + view);
+                       h_override ? h_override[view] : 0.0f, bt.W[k], bt.H[k], precision, stats + view);
         }
     }
 }
@@ -1756,7 +1761,7 @@ __global__ void __launch_bounds__(32 * kDescentWarps<KM>, KM <= 16 ? kDescentBlo
         T.coef = shifted(T.coef, off);
         T.leaf_xy = shifted(T.leaf_xy, off);
         T.leaf_id = shifted(T.leaf_id, off);
-        if (T.order) T.order = shifted(T.order, off);
+        T.order = shifted(T.order, off);
         vs = shifted(vs, off);
         view += vz;
         if (!UNEVEN) {
@@ -1769,7 +1774,7 @@ __global__ void __launch_bounds__(32 * kDescentWarps<KM>, KM <= 16 ? kDescentBlo
     extern __shared__ uint2 list[];  // K > 16: (key, id) in order, one column per lane
     const unsigned full = 0xffffffffu;
     int i, j;
-    cell_block(T.order, W, H, at_block, i, j);
+    cell_block(T.order, vs, W, H, at_block, i, j);
     if (i >= W || j >= H) return;  // (uniform over the block)
     i += threadIdx.y;
     j += threadIdx.x;
@@ -2122,7 +2127,7 @@ __global__ void __launch_bounds__(kDescentThreads, kDescentBlocks)
     __shared__ WarpTables s_tables[kDescentThreads / 32];
     const unsigned full = 0xffffffffu;
     int i, j;
-    cell_block(T.order, W, H, blockIdx.x, i, j);
+    cell_block(T.order, vs, W, H, blockIdx.x, i, j);
     if (i >= W || j >= H) return;  // (uniform over the block)
     i += threadIdx.y;
     j += threadIdx.x;
@@ -3025,7 +3030,6 @@ extern "C" int uds_sample_descent(const uds_sample_params* prm, int view, const 
     if (prm->N == 0) return UDS_OK;
     cudaStream_t s = as_stream(stream);
     Tree T = tree_of(w);
-    T.order = nullptr;  // (the tree may have been built for an image of another size)
     switch (num_rounds(prm->K)) {
         case 1: launch_sample<1>(T, w, prm, uniforms, view, indices, s); break;
         case 2: launch_sample<2>(T, w, prm, uniforms, view, indices, s); break;
