@@ -70,7 +70,7 @@ typedef struct {
                                 `seed`, so a captured CUDA graph draws new
                                 numbers after the caller updates it */
     int32_t tile_x;          /* descent warp tile width in pixels along y:
-                                4, 8, 16 or 32 (0 = 8); results do not depend
+                                4 or 8 (0, 16, 32: 8); results do not depend
                                 on it, only speed (see the autotuner) */
     int32_t fixed_degree;    /* 0: the reference's adaptive-degree expansions
                                 (P2M per node over its leaves).  4, 6 or 8:
@@ -90,7 +90,7 @@ typedef struct {
                                 over all of them with their exact Gaussians.
                                 A uniforms tensor is then (B,W,H,R,max(K,L)) */
     int32_t spread;          /* Poisson descent with K <= 8: how the child
-                                masses below the expansion frontier are shared
+                                masses below a warp's tables are shared
                                 out: 0 every lane evaluates its own, 1 spread
                                 over the warp's lanes.  Results are identical;
                                 only the speed differs (the autotuner picks) */

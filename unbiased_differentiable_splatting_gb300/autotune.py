@@ -3,11 +3,11 @@
 Two choices change the descent's speed but not its result:
 
 * the warp tile: the descent runs one warp per 32-pixel tile, whose width
-  along y (``tile_x`` in ``uds_sample_params``: 4, 8, 16 or 32 pixels, the
-  height is 32 / tile_x) sets how much of the tree the 32 walks of a warp
-  share; every lane walks its own pixel's tree, so the sampled indices are
-  identical for every tile shape;
-* how the child masses below the expansion frontier are shared out among the
+  along y (``tile_x`` in ``uds_sample_params``: 4 or 8 pixels, the height is
+  32 / tile_x; 16 and 32 are accepted and run as 8) sets how much of the tree
+  the 32 pixels of a warp share; every lane's descent is its own, so the
+  sampled indices are identical for every tile shape;
+* how the child masses below a warp's tables are shared out among the
   lanes (``spread``: 0 every lane evaluates its own, 1 spread over the warp);
   the masses are the same calls either way.  Spreading is faster where few
   lanes need masses at a time, evaluating per lane where neighbouring pixels

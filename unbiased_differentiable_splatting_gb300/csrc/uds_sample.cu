@@ -1703,15 +1703,15 @@ constexpr int kKnown = 3;  // nodes outside the tables whose child masses a lane
 // Two warps per block: their tables fit the 48 KB of static shared memory,
 // and a block's slot is free again when two tiles are done.  Six blocks per
 // SM fill its shared memory (168 registers per thread).  What bounds the
-// descent is the length of its instruction stream (620 million warp
-// instructions at 500k splats / 1024^2, 0.43 per cycle and scheduler, mostly
-// waiting for the previous instruction); the same algorithm with unrolled
-// loops ran 516 million but took 2.6 ms instead of 1.34, fetching them (187
-// KB of code instead of 54).  500k / 1024^2 / K = 8: 2.7-3.3 ms before these
-// tables, 11 ms where one pixel's cache of 160 nodes overflowed; 1.34 with
-// rolled series, 1.22 with one form of the series per number of blocks, 0.96
-// with the tiles in order of the work they hold (kCells), 0.85 with the series
-// in pairs.
+// descent is the length of its instruction stream: 445 million warp
+// instructions at 500k splats / 1024^2, 0.41 per cycle and scheduler while
+// warps are there, mostly waiting for the previous instruction.  (An earlier
+// form with unrolled loops ran 516 million against 620 but took 2.6 ms instead
+// of 1.34, fetching them: 187 KB of code instead of 54.)  500k / 1024^2 / K = 8:
+// 2.7-3.3 ms before these tables, 11 ms where one pixel's cache of 160 nodes
+// overflowed; 1.34 with rolled series, 1.22 with one form of the series per
+// number of blocks, 0.96 with the tiles in order of the work they hold (kCells),
+// 0.85 with the series in pairs.
 constexpr int kDescentThreads = 64, kDescentBlocks = 6;
 
 // Views of different sizes in one descent launch: blocks [first[v],
@@ -2118,11 +2118,10 @@ __global__ void __launch_bounds__(kDescentThreads, kDescentBlocks)
                  const uint64_t* __restrict__ seed_ptr, uint32_t view, int* __restrict__ indices,
                  float* __restrict__ probs, uds_view_stats* st, const unsigned char* __restrict__ mask,
                  float* __restrict__ weights) {
-    // same warp layout and per-pixel mass cache as k_sample: one warp walks
-    // its 32 pixels' trees together, then every lane draws its K paths; the
-    // masses come from the cache, the per-depth cache of earlier draws, or a
-    // direct evaluation by each lane that needs them (all bit-identical to
-    // separate getWeight calls)
+    // same tiles and tables as k_sample, then every lane draws its K paths; the
+    // masses come from the tables, from those kept per depth of earlier draws,
+    // or from the lane that needs them (all bit-identical to separate getWeight
+    // calls)
     if (seed_ptr) seed = *seed_ptr;
     __shared__ WarpTables s_tables[kDescentThreads / 32];
     const unsigned full = 0xffffffffu;

@@ -17,7 +17,7 @@ end so existing calls keep working:
 * ``fixed_degree``: 0 (the reference's adaptive expansions) or 4, 6, 8: every
   internal node gets a degree-P expansion built by the M2M shift from its
   children (no reference counterpart; not bit-identical to the oracle).
-* ``tile_x``: width of the descent's 32-pixel warp tiles (4, 8, 16, 32);
+* ``tile_x``: width of the descent's 32-pixel warp tiles (4 or 8; 16 and 32 run as 8);
   default: the autotuner's cached choice for this shape (see ``autotune``),
   else 8.  The indices do not depend on it.
 * ``spread``: 0 or 1, how the descent shares out the child masses below the
