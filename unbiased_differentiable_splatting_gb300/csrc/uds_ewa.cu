@@ -16,13 +16,14 @@
 
 namespace uds {
 
-// The pairs of one view that some pixel samples (used[o] set), gathered by a
-// block from kPairs consecutive ones: only those get Gaussian constants and
+// The pairs of one view that some pixel samples (a bit each, whole words per
+// view: mark_words), gathered by a block from PER x 256 consecutive ones: only those get Gaussian constants and
 // gradients, as in the reference, whose kernels visit sampled pairs only.  A
 // view of a large scene samples a few percent of its splats; one thread per
 // pair left a warp running the whole frame for one lane in twenty (two passes
 // over 16 views of 2M splats 2.27 ms; gathered 0.51 ms).
 constexpr int kPairThreads = 256;
+__host__ __device__ inline int mark_words(int N) { return (int)(((unsigned)N + 31u) >> 5); }
 
 template <int PER>
 struct PairList {
@@ -33,20 +34,19 @@ struct PairList {
 // Fills the list with the block's used pairs (offsets from base); returns
 // their number.
 template <int PER>
-__device__ __forceinline__ int gather_pairs(PairList<PER>& list, const unsigned char* __restrict__ used, size_t view,
-                                            int base, int N) {
+__device__ __forceinline__ int gather_pairs(PairList<PER>& list, const unsigned* __restrict__ used, int base, int N) {
     if (threadIdx.x == 0) list.count = 0;
     __syncthreads();
+    used += (size_t)mark_words(N) * blockIdx.y;
     const unsigned lane = threadIdx.x & 31;
 #pragma unroll
     for (int i = 0; i < PER; ++i) {
         const int at = i * kPairThreads + (int)threadIdx.x;
-        const bool hit = base + at < N && used[view + base + at];
-        const unsigned m = __ballot_sync(0xffffffffu, hit);
+        const unsigned m = base + at - (int)lane < N ? used[(base + at) >> 5] : 0u;  // the warp's 32 pairs
         unsigned first = 0;
         if (lane == 0 && m) first = atomicAdd(&list.count, (unsigned)__popc(m));
         first = __shfl_sync(0xffffffffu, first, 0);
-        if (hit) list.at[first + __popc(m & ((1u << lane) - 1u))] = (unsigned short)at;
+        if ((m >> lane) & 1u) list.at[first + __popc(m & ((1u << lane) - 1u))] = (unsigned short)at;
     }
     __syncthreads();
     return (int)list.count;
@@ -60,12 +60,12 @@ __global__ void __launch_bounds__(kPairThreads) k_ewa_consts(int N, float W, flo
                                                              const float* __restrict__ pts,
                                                              const float* __restrict__ nrm,
                                                              const float* __restrict__ sd, int sdB, float sm,
-                                                             const unsigned char* __restrict__ used,
+                                                             const unsigned* __restrict__ used,
                                                              float4* __restrict__ consts, float4* __restrict__ stats) {
     __shared__ PairList<PER> list;
     const size_t view = (size_t)N * blockIdx.y;
     const int base = blockIdx.x * kPairThreads * PER;
-    const int count = gather_pairs<PER>(list, used, view, base, N);
+    const int count = gather_pairs<PER>(list, used, base, N);
     for (int i = threadIdx.x; i < count; i += kPairThreads) {
         const int x = base + list.at[i];
         const size_t o = view + x;
@@ -87,28 +87,54 @@ __global__ void __launch_bounds__(kPairThreads) k_ewa_consts(int N, float W, flo
     }
 }
 
-// Flag the (view, splat) pairs that some pixel samples.  Four consecutive
-// indices per thread (VEC: one 16-byte load); S samples per view.  Bound by
-// the scattered byte stores (1024^2 pixels, K = 8, 1.8M samples: 20 us;
-// one thread per pixel took 24 us).  Looking first whether the flag is set
-// costs more than the store (8 times at 6.1M samples).
+// Marks the (view, splat) pairs that some pixel samples; S samples per view,
+// blockIdx.y the view.
+//
+// k_ewa_mark: a block collects the marks of `chunk` samples in a bit map in
+// shared memory (of the splats [range z, range (z + 1)), range a multiple of
+// 32) and adds the words that have any to the view's.  Setting a mark in
+// global memory per sample is bound by the 32 scattered stores of a warp, one
+// a cycle per SM: 1001 x 763, K = 8, 6.1M samples 28 us, now 7.5;
+// 1024^2, 1.8M of 8.4M valid 20 us, now 13.
+constexpr int kMarkThreads = 512;
 template <bool VEC>
-__global__ void k_ewa_mark(size_t S, const int* __restrict__ idx, int N, unsigned char* __restrict__ used) {
-    const size_t s = 4 * ((size_t)blockIdx.x * blockDim.x + threadIdx.x);
-    if (s >= S) return;
+__global__ void __launch_bounds__(kMarkThreads) k_ewa_mark(size_t S, size_t chunk, const int* __restrict__ idx, int N,
+                                                           int range, unsigned* __restrict__ used) {
+    extern __shared__ unsigned bits[];
+    const int lo = (int)blockIdx.z * range, count = min(N - lo, range), words = mark_words(count);
+    for (int w = threadIdx.x; w < words; w += kMarkThreads) bits[w] = 0u;
+    __syncthreads();
     idx += S * blockIdx.y;
-    used += (size_t)N * blockIdx.y;
-    int id[4];
+    const size_t first = chunk * blockIdx.x, end = min(first + chunk, S);
+    auto mark = [&](int id) {
+        const unsigned o = (unsigned)id - (unsigned)lo;  // (no sample: -1, far above)
+        if (id >= 0 && o < (unsigned)count) atomicOr(&bits[o >> 5], 1u << (o & 31u));
+    };
     if (VEC) {
-        const int4 v = *reinterpret_cast<const int4*>(idx + s);
-        id[0] = v.x; id[1] = v.y; id[2] = v.z; id[3] = v.w;
+#pragma unroll 4
+        for (size_t s = first + 4 * threadIdx.x; s < end; s += 4 * kMarkThreads) {
+            const int4 v = *reinterpret_cast<const int4*>(idx + s);
+            mark(v.x);
+            mark(v.y);
+            mark(v.z);
+            mark(v.w);
+        }
     } else {
-#pragma unroll
-        for (int k = 0; k < 4; ++k) id[k] = s + k < S ? idx[s + k] : -1;
+#pragma unroll 4
+        for (size_t s = first + threadIdx.x; s < end; s += kMarkThreads) mark(idx[s]);
     }
-#pragma unroll
-    for (int k = 0; k < 4; ++k)
-        if (id[k] >= 0 && id[k] < N) used[id[k]] = 1;
+    __syncthreads();
+    used += (size_t)mark_words(N) * blockIdx.y + (lo >> 5);
+    for (int w = threadIdx.x; w < words; w += kMarkThreads)
+        if (const unsigned m = bits[w]) atomicOr(&used[w], m);
+}
+
+// The same sample by sample, for few samples or a great many splats.
+__global__ void k_ewa_mark_direct(size_t S, const int* __restrict__ idx, int N, unsigned* __restrict__ used) {
+    const size_t s = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (s >= S) return;
+    const int id = idx[S * blockIdx.y + s];
+    if (id >= 0 && id < N) atomicOr(&used[(size_t)mark_words(N) * blockIdx.y + (id >> 5)], 1u << (id & 31));
 }
 
 // One thread per pixel (x = i, y = j), K samples.
@@ -289,7 +315,7 @@ __global__ void __launch_bounds__(kPairThreads) k_ewa_chain(int N, bool sum_sd, 
                                                             const float* __restrict__ pts,
                                                             const float* __restrict__ nrm,
                                                             const float* __restrict__ sd, int sdB, float sm,
-                                                            const unsigned char* __restrict__ used,
+                                                            const unsigned* __restrict__ used,
                                                             const float4* __restrict__ stats,
                                                             float* __restrict__ gp, float* __restrict__ gn,
                                                             float* __restrict__ gs) {
@@ -303,7 +329,7 @@ __global__ void __launch_bounds__(kPairThreads) k_ewa_chain(int N, bool sum_sd, 
     }
     if (!sum_sd)
         for (int i = threadIdx.x; i < 2 * here; i += kPairThreads) gs[2 * ((sdB > 1 ? view : 0) + base) + i] = 0.0f;
-    const int count = gather_pairs<PER>(list, used, view, base, N);  // (synchronises the block)
+    const int count = gather_pairs<PER>(list, used, base, N);  // (synchronises the block)
     for (int i = threadIdx.x; i < count; i += kPairThreads) {
         const int x = base + list.at[i];
         const size_t o = view + x;
@@ -602,9 +628,9 @@ using namespace uds;
 static size_t align256(size_t x) { return (x + 255) & ~(size_t)255; }
 
 // Workspace: Gaussian constants (2 float4 per pair), gradient statistics (2
-// float4 per pair), one flag byte per pair.
+// float4 per pair), one mark per pair.
 extern "C" size_t uds_splat_workspace_size(int B, int N) {
-    return align256(sizeof(float4) * 2 * (size_t)B * N) * 2 + align256((size_t)B * N);
+    return align256(sizeof(float4) * 2 * (size_t)B * N) * 2 + align256(4 * (size_t)mark_words(N) * B);
 }
 
 static int check_splat_args(int B, int W, int H, int K, int std_batch, int N) {
@@ -624,26 +650,47 @@ static bool few_pairs(int B, int N) { return (size_t)cdiv(N, 4 * kPairThreads) *
 // Gaussian constants, gradient statistics and flags of the workspace.
 struct SplatWs {
     float4 *consts, *stats;
-    unsigned char* used;
+    unsigned* used;
 };
 static SplatWs splat_ws(int B, int N, void* workspace) {
     char* p = reinterpret_cast<char*>(workspace);
     size_t half = align256(sizeof(float4) * 2 * (size_t)B * N);
     return {reinterpret_cast<float4*>(p), reinterpret_cast<float4*>(p + half),
-            reinterpret_cast<unsigned char*>(p + 2 * half)};
+            reinterpret_cast<unsigned*>(p + 2 * half)};
 }
 
-// Flags of the sampled pairs and their Gaussian constants; with stats, their
+// Marks of the sampled pairs (zeroed first).
+static int mark_sampled(int B, size_t S, int N, const int32_t* indices, unsigned* used, cudaStream_t s) {
+    cudaError_t e = cudaMemsetAsync(used, 0, 4 * (size_t)mark_words(N) * B, s);
+    // the splats in one bit map of at most 128 KB, or in up to four
+    constexpr int kRange = 1 << 20;
+    const int ranges = (int)(((long long)N + kRange - 1) / kRange), range = ranges > 1 ? kRange : 32 * mark_words(N);
+    if (S >= 32768 && ranges <= 4) {
+        // about two blocks per SM in all, of at least 16384 samples
+        size_t blocks = 304 / ((size_t)B * ranges), most = (S + 16383) / 16384;
+        if (blocks > most) blocks = most;
+        if (blocks < 1) blocks = 1;
+        const bool vec = S % 4 == 0 && aligned16(indices);
+        const size_t chunk = ((S + blocks - 1) / blocks + 3) / 4 * 4, bytes = (size_t)range / 8;
+        const dim3 grid(cdiv(S, chunk), B, ranges);
+        auto kernel = vec ? k_ewa_mark<true> : k_ewa_mark<false>;
+        if (e == cudaSuccess && bytes > 48 * 1024)
+            e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+        if (e == cudaSuccess) kernel<<<grid, kMarkThreads, bytes, s>>>(S, chunk, indices, N, range, used);
+    } else if (e == cudaSuccess) {
+        k_ewa_mark_direct<<<dim3(cdiv(S, 256), B), 256, 0, s>>>(S, indices, N, used);
+    }
+    if (e != cudaSuccess) { set_last_error(e); return UDS_ERR_CUDA; }
+    return launch_status();
+}
+
+// Marks of the sampled pairs and their Gaussian constants; with stats, their
 // gradient statistics zeroed.
 static int sampled_consts(int B, int W, int H, int K, float focal, const int32_t* indices, const float* points,
                           const float* normals, int std_batch, int N, const float* std_devs, float smoothing,
                           const SplatWs& ws, bool stats, cudaStream_t s) {
-    cudaError_t e = cudaMemsetAsync(ws.used, 0, (size_t)B * N, s);
-    if (e != cudaSuccess) { set_last_error(e); return UDS_ERR_CUDA; }
-    const size_t S = (size_t)W * H * K;
-    const dim3 grid(cdiv((S + 3) / 4, 256), B);
-    if (S % 4 == 0 && aligned16(indices)) k_ewa_mark<true><<<grid, 256, 0, s>>>(S, indices, N, ws.used);
-    else k_ewa_mark<false><<<grid, 256, 0, s>>>(S, indices, N, ws.used);
+    int st = mark_sampled(B, (size_t)W * H * K, N, indices, ws.used, s);
+    if (st) return st;
     float4* z = stats ? ws.stats : nullptr;
     if (few_pairs(B, N))
         k_ewa_consts<1><<<dim3(cdiv(N, kPairThreads), B), kPairThreads, 0, s>>>(
@@ -651,7 +698,7 @@ static int sampled_consts(int B, int W, int H, int K, float focal, const int32_t
     else
         k_ewa_consts<4><<<dim3(cdiv(N, 4 * kPairThreads), B), kPairThreads, 0, s>>>(
             N, (float)W, (float)H, focal, points, normals, std_devs, std_batch, smoothing, ws.used, ws.consts, z);
-    return launch_status(2);
+    return launch_status();
 }
 
 // The splat gradients from the statistics.  clamp: with the reference's
