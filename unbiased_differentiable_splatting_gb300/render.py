@@ -275,20 +275,28 @@ class MultiViewSplatting(th.nn.Module):
             perSplat = self.forwardHarmonics(flipped, pointDiffuse)
         else:
             perSplat = pointDiffuse
-        B = camPoints.shape[0]
+        # Split once rather than sliced per group and image: each slice's
+        # gradient is a whole tensor of zeros with the slice's in it, and all of
+        # them are added up; a split's is one concatenation.  (The unsafe form's
+        # parts may be written in place, as slices may.)
+        sizes = [g[1] for g in self.groups]
+
+        def by_group(t):
+            if t.shape[0] == 1:
+                return [t] * len(sizes)
+            if t.shape[0] != sum(sizes):
+                return [t[g[0]:g[0] + g[1]] for g in self.groups]
+            return th.unsafe_split_with_sizes(t, sizes) if len(sizes) > 1 else [t]
+
         images, indices, depth = [], [], []
-        for (b0, nb, W, H, f) in self.groups:
-            sl = slice(b0, b0 + nb)
+        parts = zip(self.groups, *(by_group(t) for t in (camPoints, camNormals, pointStdDevs, perSplat)))
+        for (b0, nb, W, H, f), pts, nrm, sd, attr in parts:
             # consecutive views of one size are consecutive in the packed buffer
             K = self.numSamples
             idx = packed[b0].as_strided((nb, W, H, K), (W * H * K, H * K, K, 1))
-            sd = pointStdDevs if pointStdDevs.shape[0] == 1 else pointStdDevs[sl]
-            attr = perSplat if perSplat.shape[0] == 1 and B > 1 else perSplat[sl]
-            img, dw, _ = th.ops.uds.render_splats(W, H, f, idx, camPoints[sl].contiguous(),
-                                                  camNormals[sl].contiguous(), sd.contiguous(), self.smoothing,
-                                                  attr.contiguous())
-            for k in range(nb):
-                images.append(img[k:k + 1])
-                indices.append(idx[k:k + 1])
-                depth.append(dw[k:k + 1])
+            img, dw, _ = th.ops.uds.render_splats(W, H, f, idx, pts.contiguous(), nrm.contiguous(), sd.contiguous(),
+                                                  self.smoothing, attr.contiguous())
+            images.extend(th.unsafe_split(img, 1) if nb > 1 else [img])
+            indices.extend(idx[k:k + 1] for k in range(nb))
+            depth.extend(th.unsafe_split(dw, 1) if nb > 1 else [dw])
         return images, indices, depth
