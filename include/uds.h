@@ -131,7 +131,9 @@ int uds_backface_backward(int B, int N, const float* cam_normals, const float* g
  *      R = ceil(sqrt(K)), M = max(K, leaf_size); NULL draws Philox4x32-10
  *      uniforms from seed.
  *      h_override: optional device float[B]; entries > 0 replace the
- *      computed bandwidth.  stats: device uds_view_stats[B] (may be NULL). ---- */
+ *      computed bandwidth.  stats: device uds_view_stats[B] (may be NULL).
+ *      Workspace: B trees, and up to 108 MB (once per call) for tiles with
+ *      pixels that meet thousands of tree nodes. ---- */
 size_t uds_sample_workspace_size(const uds_sample_params* prm);
 int uds_sample(const uds_sample_params* prm, const float* points, const float* normals,
                const float* std_devs, const float* uniforms, const float* h_override,

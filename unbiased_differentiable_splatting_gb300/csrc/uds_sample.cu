@@ -53,6 +53,7 @@ struct ViewState {            // per-view device scalars (lives in the workspace
     int failed;               // a wait ran out: the view samples nothing (see look_back)
     int W, H;                 // of the image the tree was built for
     unsigned ticket[kPasses + 3];  // blocks started: k_sort_pass's, k_cull's, k_p2m's; done: k_bandwidth's
+    unsigned deferred[3];     // tiles left for the long tables (LongTables), those taken, blocks done with them
 };
 
 // ----------------------------------------------------- order of the tiles
@@ -1050,9 +1051,8 @@ __device__ __noinline__ float node_weight_out_of_line(Tree T, int v, float qx, f
 // per expansion (a lane reads its own column: no bank conflicts whatever row
 // it is at); rows past kRows go to local memory.  Where the tables are full
 // (pixels far apart in units of the bandwidth share little of the tree), the
-// caller takes half the lanes at a time.
-constexpr int kOpen = 224, kEvals = 192;  // table entries
-constexpr int kRows = 63;                 // masses in shared memory
+// caller takes half the lanes at a time, and where those of a single pixel are
+// (LongTables), it leaves the rest of the tile to a second kernel.
 constexpr int kLevels = 64;               // a radix tree over 62-bit keys is at most 63 deep
 // Per-lane records of the descent in shared memory: local memory that is
 // written and read back costs an L2 round trip here (about 700 cycles).
@@ -1068,6 +1068,9 @@ constexpr unsigned kLinkOpen = 0u, kLinkEval = 0x4000u, kLinkNone = 0x8000u;
 constexpr unsigned kLinkKind = 0xC000u, kLinkStop = 0x2000u, kLinkEntry = 0x1FFFu;
 
 struct WarpTables {
+    static constexpr int kOpen = 224, kEvals = 192;  // entries
+    static constexpr int kRows = 63;                 // masses in shared memory
+    static constexpr bool kLong = false;
     uint4 open[kOpen];               // links (left | right << 16), left child, right child, lanes that opened it
     unsigned short split[kOpen];     // first expansion of the right subtree
     union {
@@ -1090,7 +1093,103 @@ struct WarpTables {
         };
     };
     int owner[32];                   // warp_child_masses
+    __device__ __forceinline__ float& mass(int v, int lane) { return val[v][lane]; }
+    __device__ __forceinline__ float mass(int v, int lane) const { return val[v][lane]; }
 };
+
+// The tables of tiles with a pixel that opens more nodes, or meets more
+// expansions, than WarpTables holds: lists and masses in a slab of global
+// memory, the rest as there.  Images several times taller than wide have such
+// pixels at silhouettes: Morton keys are normalised per axis, so nodes are as
+// elongated as the image, and the error bound (half their longer side against
+// the bandwidth) holds for few splats only.  500k splats at 128 x 1024: up to
+// 1312 nodes and 1188 expansions for one pixel.  The descent's first kernel
+// only lists these tiles; a second one (k_sample_long and its like), a warp and
+// a slab per block, takes them one after the other.  What bounds it is the
+// latency of one tile; a step of those 500k splats takes 8.4 ms so (2388 with
+// one lane at a time walking the tree, 240 with 32 side by side), two views of
+// a room of 2M splats at 128 x 480 6.4 ms (716 and 76).  Pixels past these
+// tables too, millions of splats in such an image, walk side by side.
+constexpr int kLongEntries = 8192;       // nodes and expansions (what kLinkEntry can number)
+constexpr int kLongMasses = 4096 * 32;   // expansions times lanes of a group
+struct LongTables {
+    static constexpr int kOpen = kLongEntries, kEvals = kLongEntries, kRows = kLongEntries;
+    static constexpr bool kLong = true;
+    uint4* open;
+    unsigned short *split, *count, *first, *eval;
+    float* val;  // rows of `columns` masses: as many as the group has lanes
+    int columns;
+    __device__ __forceinline__ float& mass(int v, int lane) { return val[v * columns + (lane & (columns - 1))]; }
+    __device__ __forceinline__ float mass(int v, int lane) const { return val[v * columns + (lane & (columns - 1))]; }
+    unsigned short level[kLevels + 8];
+    float4 box[2][32];
+    float r2[2][32];
+    union {
+        struct {
+            alignas(16) float coef[2][kPairFloats];
+            float hermite[12][kHermiteStride];
+        };
+        struct {
+            float path[kPathRows][32];
+            float series[kMaxDegree + 1][32];
+        };
+    };
+    int owner[32];
+};
+struct LongSlab {
+    float val[kLongMasses];
+    uint4 open[kLongEntries];
+    unsigned short split[kLongEntries], count[kLongEntries], first[kLongEntries], eval[kLongEntries];
+};
+__device__ __forceinline__ void use_slab(LongTables& wt, LongSlab& s) {  // (the whole warp writes the same)
+    wt.open = s.open;
+    wt.split = s.split;
+    wt.count = s.count;
+    wt.first = s.first;
+    wt.eval = s.eval;
+    wt.val = s.val;
+    __syncwarp();
+}
+
+// The tiles left for the long tables: a tile is left as soon as kDeferWidth or
+// fewer of its lanes fill the short ones (4: as fast as any; at 8 and 16 dense
+// small images, whose tiles narrow to 8 lanes all over, lose up to a fifth to
+// the few warps that the slabs allow).  counters: ViewState::deferred of the
+// first view of the launch; tiles: first pixel, view, lanes.
+struct Deferred {
+    unsigned* counters;
+    uint4* tiles;
+    LongSlab* slabs;
+};
+constexpr int kDeferWidth = 4;
+constexpr unsigned kDeferredTiles = 1u << 16;  // more than that are sampled without tables
+// By a whole warp: leaves lanes of a tile to the second kernel ((i, j): the
+// lane's pixel); false if the list is full.
+__device__ __forceinline__ bool defer_tile(const Deferred& df, int i, int j, unsigned view, unsigned lanes) {
+    unsigned at = 0;
+    if (((threadIdx.x + blockDim.x * threadIdx.y) & 31) == 0) {
+        at = atomicAdd(&df.counters[0], 1u);
+        if (at < kDeferredTiles) df.tiles[at] = make_uint4((unsigned)i, (unsigned)j, view, lanes);
+    }
+    return __shfl_sync(0xffffffffu, at, 0) < kDeferredTiles;
+}
+// The next listed tile; false when there is none left.  The block that finds
+// the list empty last clears the counters for the next launch.
+__device__ __forceinline__ bool next_deferred(const Deferred& df, unsigned count, uint4& tile) {
+    unsigned at = 0;
+    if (threadIdx.x == 0 && threadIdx.y == 0) {
+        at = atomicAdd(&df.counters[1], 1u);
+        if (at >= count && atomicAdd(&df.counters[2], 1u) == gridDim.x - 1) {
+            df.counters[0] = 0u;
+            df.counters[1] = 0u;
+            df.counters[2] = 0u;
+        }
+    }
+    at = __shfl_sync(0xffffffffu, at, 0);
+    if (at >= count) return false;
+    tile = df.tiles[at];
+    return true;
+}
 
 // Blocks of four coefficients per side of a degree-p expansion.
 __device__ __forceinline__ int coef_blocks(int p) { return (p + 4) >> 2; }
@@ -1178,8 +1277,8 @@ __device__ __forceinline__ void stage_pair(float* dst, int nb, const float* __re
 // bound by instruction fetch once its code outgrows the instruction cache).
 // (t2, e): 2 t and exp(-t^2), t the coordinate of this lane's column or row
 // relative to the expansions' centres.
-template <int NB>
-__device__ __forceinline__ float_pair hermite_pair(WarpTables& wt, const float* coef, int PA, int PB, int cols,
+template <int NB, class Tables>
+__device__ __forceinline__ float_pair hermite_pair(Tables& wt, const float* coef, int PA, int PB, int cols,
                                                    float_pair t2, float_pair e, int lane) {
     const unsigned full = 0xffffffffu;
     constexpr int S = kPairStride<NB>;
@@ -1244,7 +1343,8 @@ __device__ __forceinline__ float_pair hermite_pair(WarpTables& wt, const float* 
 }
 
 // The same for one expansion of five blocks (degree 16).
-__device__ __forceinline__ float hermite_single(WarpTables& wt, const float* coef, int cols, float t2, float e,
+template <class Tables>
+__device__ __forceinline__ float hermite_single(Tables& wt, const float* coef, int cols, float t2, float e,
                                                 int lane) {
     const unsigned full = 0xffffffffu;
     constexpr int NB = 5, S = kSingleStride, P1 = kMaxDegree + 1;
@@ -1305,7 +1405,8 @@ __device__ __forceinline__ float hermite_single(WarpTables& wt, const float* coe
 // instructions: Hermite functions of y in the lane's column of wt.series,
 // rows four at a time (independent chains); hermite_eval's operations in its
 // order.  Nodes without one (rare here) go out of line.
-__device__ __forceinline__ float lane_series(const Tree& T, WarpTables& wt, int lane, int v, float qx, float qy) {
+template <class Tables>
+__device__ __forceinline__ float lane_series(const Tree& T, Tables& wt, int lane, int v, float qx, float qy) {
     const float4 c = T.cen[v];
     const int p = meta_degree(c.w);
     if (p < 0) return node_weight_out_of_line(T, v, qx, qy);
@@ -1362,26 +1463,30 @@ __device__ __forceinline__ bool within(float4 b, float r2, float qx, float qy) {
 }
 
 // Sum of the listed masses [s, t) of this lane, in order.
-__device__ __forceinline__ float range_sum(const WarpTables& wt, const float* val_hi, int lane, int s, int t) {
+template <class Tables>
+__device__ __forceinline__ float range_sum(const Tables& wt, const float* val_hi, int lane, int s, int t) {
     float acc = 0.0f;
     int i = s;
+    constexpr int kRows = Tables::kRows;
     const int top = min(t, kRows);
 #pragma unroll 1
     for (; i + 4 <= top; i += 4) {
-        float x0 = wt.val[i][lane], x1 = wt.val[i + 1][lane], x2 = wt.val[i + 2][lane], x3 = wt.val[i + 3][lane];
+        float x0 = wt.mass(i, lane), x1 = wt.mass(i + 1, lane), x2 = wt.mass(i + 2, lane), x3 = wt.mass(i + 3, lane);
         acc = fadd(fadd(fadd(fadd(acc, x0), x1), x2), x3);
     }
 #pragma unroll 1
-    for (; i < t; ++i) acc = fadd(acc, i < kRows ? wt.val[i][lane] : val_hi[i - kRows]);
+    for (; i < t; ++i) acc = fadd(acc, i < kRows ? wt.mass(i, lane) : val_hi[i - kRows]);
     return acc;
 }
 
-// Fills the tables for the lanes of `lanes` (all 32 lanes call this).
+// Fills the tables for the lanes of `lanes`, a group of `width` (all 32 lanes
+// call this).
 // Returns the number of expansions listed (opened node 0 is the root), 0
 // when there are no tables (the root carries an expansion, or no lane
 // reaches it), -1 when they are full (nothing computed).  total is getWeight
 // of the root for the lanes inside.
-__device__ int warp_tables(const Tree& T, float qx, float qy, unsigned lanes, int M, int cols, WarpTables& wt,
+template <class Tables>
+__device__ int warp_tables(const Tree& T, float qx, float qy, unsigned lanes, int width, int M, int cols, Tables& wt,
                            float* val_hi, float& total) {
     const unsigned full = 0xffffffffu;
     const int lane = (threadIdx.x + blockDim.x * threadIdx.y) & 31;
@@ -1437,7 +1542,7 @@ __device__ int warp_tables(const Tree& T, float qx, float qy, unsigned lanes, in
             const unsigned Ba = __ballot_sync(full, oa), Bb = __ballot_sync(full, ob);
             const int pa = next + __popc(Ba & lt) + __popc(Bb & lt), pb = pa + (oa ? 1 : 0);
             next += __popc(Ba) + __popc(Bb);
-            if (next > kOpen) return -1;
+            if (next > Tables::kOpen) return -1;
             if (lane < cnt) {
                 unsigned la = ea ? kLinkEval : kLinkNone, lb = eb ? kLinkEval : kLinkNone;
                 if (oa) {
@@ -1474,7 +1579,11 @@ __device__ int warp_tables(const Tree& T, float qx, float qy, unsigned lanes, in
         __syncwarp();
     }
     const int nV = wt.count[0];
-    if (nV > kEvals) return -1;
+    if (nV > Tables::kEvals) return -1;
+    if constexpr (Tables::kLong) {
+        if (nV > kLongMasses / width) return -1;
+        wt.columns = width;
+    }
     // ---- and their places in depth-first order, down the levels
     if (lane == 0) wt.first[0] = 0;
     __syncwarp();
@@ -1534,8 +1643,9 @@ __device__ int warp_tables(const Tree& T, float qx, float qy, unsigned lanes, in
         auto put = [&](int at, float w) {  // the mass of the expansion at place `at`
             const int v = v0 + __shfl_sync(full, mine, at);
             w = ((__shfl_sync(full, inside, at) >> lane) & 1u) ? w : 0.0f;
-            if (v < kRows) wt.val[v][lane] = w;
-            else val_hi[v - kRows] = w;
+            if (Tables::kLong && !live) return;  // (another lane's column)
+            if (v < Tables::kRows) wt.mass(v, lane) = w;
+            else val_hi[v - Tables::kRows] = w;
         };
 #pragma unroll 1
         for (int k = 0; k < fives; ++k) {
@@ -1608,7 +1718,8 @@ struct Stem {
     unsigned long long path;
 };
 
-__device__ __forceinline__ Stem find_stem(const WarpTables& wt) {
+template <class Tables>
+__device__ __forceinline__ Stem find_stem(const Tables& wt) {
     Stem s{0, 0, 0ull};
 #pragma unroll 1
     while (s.depth < kTrace - 2) {  // uniform over the warp
@@ -1626,7 +1737,8 @@ __device__ __forceinline__ Stem find_stem(const WarpTables& wt) {
 // The sums of the children's ranges (getWeight of both children); E: the
 // node's entry, m: its split.  A child that holds the whole range has the
 // node's own sum.
-__device__ __forceinline__ void child_sums(const WarpTables& wt, const float* val_hi, int lane, const Place& at, int m,
+template <class Tables>
+__device__ __forceinline__ void child_sums(const Tables& wt, const float* val_hi, int lane, const Place& at, int m,
                                            float& w0, float& w1) {
     if (m == at.t) { w0 = at.sum; w1 = 0.0f; }
     else if (m == at.s) { w0 = 0.0f; w1 = at.sum; }
@@ -1659,8 +1771,8 @@ __device__ __forceinline__ unsigned lane_group(unsigned todo, int width) {
 //   order), then their right children, so a lane waits for one series
 //   instead of two while c <= 16.  `owner`: 32 ints of the warp's shared
 //   memory.
-template <bool SPREAD>
-__device__ __forceinline__ void warp_child_masses(const Tree& T, WarpTables& wt, bool need, int a, int b, float qx,
+template <bool SPREAD, class Tables>
+__device__ __forceinline__ void warp_child_masses(const Tree& T, Tables& wt, bool need, int a, int b, float qx,
                                                   float qy, float& w0, float& w1) {
     int* owner = wt.owner;
     const int lane = (threadIdx.x + blockDim.x * threadIdx.y) & 31;
@@ -1730,76 +1842,44 @@ struct UnevenViews {
 template <int KM>
 constexpr int kDescentWarps = KM <= 16 ? kDescentThreads / 32 : 1;
 
-template <int R, int KM, bool UNEVEN, bool SPREAD>
-__global__ void __launch_bounds__(32 * kDescentWarps<KM>, KM <= 16 ? kDescentBlocks : 8)
-    k_sample(Tree T, const ViewState* vs, int W, int H, int K, int M, float precision,
-             const float* __restrict__ uniforms, uint64_t seed, const uint64_t* __restrict__ seed_ptr, uint32_t view,
-             int* __restrict__ indices, uds_view_stats* st, size_t vstride, size_t ustride, size_t istride,
-             UnevenViews uv) {
-    // block tile_x (y) x threads / tile_x (x), blockIdx.x its place among
-    // the view's (cell_block).  blockIdx.y selects the view: its tree lives
-    // vstride bytes after the previous view's, its uniforms ustride floats and
-    // its indices istride entries further on.  With UNEVEN the view and the
-    // block's place in it come from uv (blockIdx.x only; no uniforms tensor).
-    if (seed_ptr) seed = *seed_ptr;
-    unsigned at_block = blockIdx.x, vz = blockIdx.y;
-    if (UNEVEN) {
-        int b = 0;
-        while (b + 1 < uv.nv && uv.first[b + 1] <= (int)blockIdx.x) ++b;
-        at_block = blockIdx.x - (unsigned)uv.first[b];
-        vz = (unsigned)b;
-        W = uv.W[b];
-        H = uv.H[b];
-        indices += uv.ioff[b];
-    }
-    if (vz) {
-        size_t off = (size_t)vz * vstride;
-        T.lnk = shifted(T.lnk, off);
-        T.par = shifted(T.par, off);
-        T.box = shifted(T.box, off);
-        T.cen = shifted(T.cen, off);
-        T.coef = shifted(T.coef, off);
-        T.leaf_xy = shifted(T.leaf_xy, off);
-        T.leaf_id = shifted(T.leaf_id, off);
-        T.order = shifted(T.order, off);
-        vs = shifted(vs, off);
-        view += vz;
-        if (!UNEVEN) {
-            indices += (size_t)vz * istride;
-            if (uniforms) uniforms += (size_t)vz * ustride;
-        }
-        st += vz;
-    }
-    __shared__ WarpTables s_tables[kDescentWarps<KM>];
-    extern __shared__ uint2 list[];  // K > 16: (key, id) in order, one column per lane
+// The tree of the view vz places after the first one of a launch.
+__device__ __forceinline__ void shift_tree(Tree& T, size_t off) {
+    T.lnk = shifted(T.lnk, off);
+    T.par = shifted(T.par, off);
+    T.box = shifted(T.box, off);
+    T.cen = shifted(T.cen, off);
+    T.coef = shifted(T.coef, off);
+    T.leaf_xy = shifted(T.leaf_xy, off);
+    T.leaf_id = shifted(T.leaf_id, off);
+    T.order = shifted(T.order, off);
+}
+
+// The descents of the lanes of `todo` of a tile; (i, j): the lane's pixel, vz:
+// the view's place in the launch.
+template <int R, int KM, bool SPREAD, class Tables>
+__device__ __forceinline__ void sample_tile(const Tree& T, Tables& wt, uint2* list, unsigned todo, int i, int j, int H,
+                                            int K, int M, float precision, const float* __restrict__ uniforms,
+                                            uint64_t seed, uint32_t view, int* __restrict__ indices,
+                                            uds_view_stats* st, const Deferred& df, unsigned vz) {
     const unsigned full = 0xffffffffu;
-    int i, j;
-    cell_block(T.order, vs, W, H, at_block, i, j);
-    if (i >= W || j >= H) return;  // (uniform over the block)
-    i += threadIdx.y;
-    j += threadIdx.x;
-    int tid = threadIdx.x + blockDim.x * threadIdx.y;
-    int warp = tid >> 5, lane = tid & 31;
-    bool live = (i < W && j < H);
-    T.n = vs->n;
-    T.sq = vs->sq;
-    T.isq = vs->isq;
-    if (T.n == 0) return;  // indices were preset to -1 (uniform over the grid)
     size_t pixel = (size_t)j + (size_t)H * i;
     float qx = (float)i, qy = (float)j;
-    WarpTables& wt = s_tables[warp];
-    float val_hi[kEvals - kRows];
+    const int lane = (threadIdx.x + blockDim.x * threadIdx.y) & 31;
+    float val_hi[Tables::kLong ? 1 : Tables::kEvals - Tables::kRows];
     // K-sized arrays stay in registers for K <= 16 (loops fully unrolled)
     constexpr int UK = KM <= 16 ? KM : 1;
-    unsigned todo = __ballot_sync(full, live);
     int width = 32;
     while (todo) {
-        const unsigned group = lane_group(todo, width);
+        unsigned group = lane_group(todo, width);
         float total;
-        const int state = warp_tables(T, qx, qy, group, M, blockDim.x, wt, val_hi, total);
-        if (state < 0 && width > 1) {
-            width >>= 1;
-            continue;
+        const int state = warp_tables(T, qx, qy, group, width, M, blockDim.x, wt, val_hi, total);
+        if (state < 0) {
+            if (!Tables::kLong && width <= kDeferWidth && defer_tile(df, i, j, vz, todo)) break;
+            if (width > 1) {
+                width >>= 1;
+                continue;
+            }
+            group = todo;  // without tables: the lanes left walk side by side
         }
         todo &= ~group;
         const bool mine = (group >> lane) & 1u;
@@ -1830,11 +1910,18 @@ __global__ void __launch_bounds__(32 * kDescentWarps<KM>, KM <= 16 ? kDescentBlo
         float* far = far_rows;
         asm volatile("" : "+l"(far));  // stays an array in memory
         constexpr int kNear = kPathRows / R;  // levels in wt.path, R rows each: the share, R - 1 capacities
-        // child masses of the last nodes met outside the tables
-        int kv[kKnown];
-        float kw0[kKnown], kw1[kKnown];
+        // child masses of the last nodes met outside the tables (of the last one
+        // at each depth with the long ones: without any at all, a walk of its
+        // subtree is what they save)
+        constexpr int kKept = Tables::kLong ? kTrace : kKnown;
+        int kv[kKept];
+        float kw0[kKept], kw1[kKept];
+        if (Tables::kLong) {
+            for (int q = 0; q < kKept; ++q) kv[q] = -1;
+        } else {
 #pragma unroll
-        for (int q = 0; q < kKnown; ++q) { kv[q] = -1; kw0[q] = 0.0f; kw1[q] = 0.0f; }
+            for (int q = 0; q < kKnown; ++q) { kv[q] = -1; kw0[q] = 0.0f; kw1[q] = 0.0f; }
+        }
         bool overflow = false;
         // A node of the stem gives its one child its whole mass, so the child's
         // capacity is always the node's: one number, cap, for the whole stem, and
@@ -1888,9 +1975,13 @@ __global__ void __launch_bounds__(32 * kDescentWarps<KM>, KM <= 16 ? kDescentBlo
                         w1 = fmaxf(0.0f, sum1);
                     } else {
                         pend = true;
+                        if (Tables::kLong) {
+                            if (kv[d] == v) { w0 = kw0[d]; w1 = kw1[d]; pend = false; }
+                        } else {
 #pragma unroll
-                        for (int q = 0; q < kKnown; ++q)
-                            if (kv[q] == v) { w0 = kw0[q]; w1 = kw1[q]; pend = false; }
+                            for (int q = 0; q < kKnown; ++q)
+                                if (kv[q] == v) { w0 = kw0[q]; w1 = kw1[q]; pend = false; }
+                        }
                     }
                 }
                 bool can = going && !pend;
@@ -1900,15 +1991,18 @@ __global__ void __launch_bounds__(32 * kDescentWarps<KM>, KM <= 16 ? kDescentBlo
                     can = pend;
                     pend = false;
                     if (can) {
+                        if (!Tables::kLong) {
 #pragma unroll
-                        for (int q = kKnown - 1; q > 0; --q) {
-                            kv[q] = kv[q - 1];
-                            kw0[q] = kw0[q - 1];
-                            kw1[q] = kw1[q - 1];
+                            for (int q = kKnown - 1; q > 0; --q) {
+                                kv[q] = kv[q - 1];
+                                kw0[q] = kw0[q - 1];
+                                kw1[q] = kw1[q - 1];
+                            }
                         }
-                        kv[0] = v;
-                        kw0[0] = w0;
-                        kw1[0] = w1;
+                        const int q = Tables::kLong ? d : 0;
+                        kv[q] = v;
+                        kw0[q] = w0;
+                        kw1[q] = w1;
                     }
                 }
                 if (can) {
@@ -2103,6 +2197,85 @@ __global__ void __launch_bounds__(32 * kDescentWarps<KM>, KM <= 16 ? kDescentBlo
     }
 }
 
+template <int R, int KM, bool UNEVEN, bool SPREAD>
+__global__ void __launch_bounds__(32 * kDescentWarps<KM>, KM <= 16 ? kDescentBlocks : 8)
+    k_sample(Tree T, const ViewState* vs, int W, int H, int K, int M, float precision,
+             const float* __restrict__ uniforms, uint64_t seed, const uint64_t* __restrict__ seed_ptr, uint32_t view,
+             int* __restrict__ indices, uds_view_stats* st, size_t vstride, size_t ustride, size_t istride,
+             UnevenViews uv, Deferred df) {
+    // block tile_x (y) x threads / tile_x (x), blockIdx.x its place among
+    // the view's (cell_block).  blockIdx.y selects the view: its tree lives
+    // vstride bytes after the previous view's, its uniforms ustride floats and
+    // its indices istride entries further on.  With UNEVEN the view and the
+    // block's place in it come from uv (blockIdx.x only; no uniforms tensor).
+    if (seed_ptr) seed = *seed_ptr;
+    unsigned at_block = blockIdx.x, vz = blockIdx.y;
+    if (UNEVEN) {
+        int b = 0;
+        while (b + 1 < uv.nv && uv.first[b + 1] <= (int)blockIdx.x) ++b;
+        at_block = blockIdx.x - (unsigned)uv.first[b];
+        vz = (unsigned)b;
+        W = uv.W[b];
+        H = uv.H[b];
+        indices += uv.ioff[b];
+    }
+    if (vz) {
+        const size_t off = (size_t)vz * vstride;
+        shift_tree(T, off);
+        vs = shifted(vs, off);
+        view += vz;
+        if (!UNEVEN) {
+            indices += (size_t)vz * istride;
+            if (uniforms) uniforms += (size_t)vz * ustride;
+        }
+        st += vz;
+    }
+    __shared__ WarpTables s_tables[kDescentWarps<KM>];
+    extern __shared__ uint2 list[];  // K > 16: (key, id) in order, one column per lane
+    int i, j;
+    cell_block(T.order, vs, W, H, at_block, i, j);
+    if (i >= W || j >= H) return;  // (uniform over the block)
+    i += threadIdx.y;
+    j += threadIdx.x;
+    int tid = threadIdx.x + blockDim.x * threadIdx.y;
+    bool live = (i < W && j < H);
+    T.n = vs->n;
+    T.sq = vs->sq;
+    T.isq = vs->isq;
+    if (T.n == 0) return;  // indices were preset to -1 (uniform over the grid)
+    sample_tile<R, KM, SPREAD>(T, s_tables[tid >> 5], list, __ballot_sync(0xffffffffu, live), i, j, H, K, M, precision,
+                               uniforms, seed, view, indices, st, df, vz);
+}
+
+// The tiles that k_sample left for the long tables, a warp per block; uv.nv: 0
+// or the number of views of different sizes.
+template <int R, int KM>
+__global__ void __launch_bounds__(32)
+    k_sample_long(Tree first, const ViewState* first_vs, int H, int K, int M, float precision,
+                  const float* __restrict__ uniforms, uint64_t seed, const uint64_t* __restrict__ seed_ptr,
+                  uint32_t view, int* __restrict__ indices, uds_view_stats* st, size_t vstride, size_t ustride,
+                  size_t istride, UnevenViews uv, Deferred df) {
+    __shared__ LongTables wt;
+    extern __shared__ uint2 list[];
+    const unsigned count = min(df.counters[0], kDeferredTiles);
+    if (count == 0) return;  // (the counters are still clear)
+    if (seed_ptr) seed = *seed_ptr;
+    use_slab(wt, df.slabs[blockIdx.x]);
+    for (uint4 tile; next_deferred(df, count, tile);) {
+        const unsigned vz = tile.z;
+        Tree T = first;
+        shift_tree(T, (size_t)vz * vstride);
+        const ViewState* vs = shifted(first_vs, (size_t)vz * vstride);
+        T.n = vs->n;
+        T.sq = vs->sq;
+        T.isq = vs->isq;
+        sample_tile<R, KM, true>(T, wt, list, tile.w, (int)(tile.x + threadIdx.y), (int)(tile.y + threadIdx.x),
+                                 uv.nv ? uv.H[vz] : H, K, M, precision, uniforms ? uniforms + vz * ustride : nullptr,
+                                 seed, view + vz, indices + (uv.nv ? (size_t)uv.ioff[vz] : vz * istride), st + vz, df,
+                                 vz);
+    }
+}
+
 // Stochastic mode (no reference counterpart).  Each of the K draws of a
 // pixel descends from the root into a child with probability
 // m_child / (m_left + m_right), masses by getWeight, and records the product
@@ -2113,45 +2286,29 @@ __global__ void __launch_bounds__(32 * kDescentWarps<KM>, KM <= 16 ? kDescentBlo
 // their upper paths, so the child masses of the last path are kept per depth
 // (node ids are unique, so a hit is exact).  A draw that meets two zero
 // masses, or is still above the leaves after kTrace levels, stays -1 / 0.
-__global__ void __launch_bounds__(kDescentThreads, kDescentBlocks)
-    k_stochastic(Tree T, const ViewState* vs, int W, int H, int K, float precision, uint64_t seed,
-                 const uint64_t* __restrict__ seed_ptr, uint32_t view, int* __restrict__ indices,
-                 float* __restrict__ probs, uds_view_stats* st, const unsigned char* __restrict__ mask,
-                 float* __restrict__ weights) {
-    // same tiles and tables as k_sample, then every lane draws its K paths; the
-    // masses come from the tables, from those kept per depth of earlier draws,
-    // or from the lane that needs them (all bit-identical to separate getWeight
-    // calls)
-    if (seed_ptr) seed = *seed_ptr;
-    __shared__ WarpTables s_tables[kDescentThreads / 32];
-    const unsigned full = 0xffffffffu;
-    int i, j;
-    cell_block(T.order, vs, W, H, blockIdx.x, i, j);
-    if (i >= W || j >= H) return;  // (uniform over the block)
-    i += threadIdx.y;
-    j += threadIdx.x;
-    int tid = threadIdx.x + blockDim.x * threadIdx.y;
-    int warp = tid >> 5, lane = tid & 31;
-    size_t pixel = (size_t)j + (size_t)H * i;
-    bool live = (i < W && j < H) && (!mask || mask[pixel]);
-    T.n = vs->n;
-    T.sq = vs->sq;
-    T.isq = vs->isq;
-    int n = T.n;
-    if (n == 0) return;
+template <class Tables>
+__device__ __forceinline__ void stochastic_tile(const Tree& T, Tables& wt, unsigned todo, int i, int j, int H, int K,
+                                                float precision, uint64_t seed, uint32_t view,
+                                                int* __restrict__ indices, float* __restrict__ probs,
+                                                uds_view_stats* st, float* __restrict__ weights, const Deferred& df) {
     float qx = (float)i, qy = (float)j;
-    WarpTables& wt = s_tables[warp];
-    float val_hi[kEvals - kRows];
+    const unsigned full = 0xffffffffu;
+    const int lane = (threadIdx.x + blockDim.x * threadIdx.y) & 31, n = T.n;
+    const size_t pixel = (size_t)j + (size_t)H * i;
+    float val_hi[Tables::kLong ? 1 : Tables::kEvals - Tables::kRows];
     bool overflow = false;
-    unsigned todo = __ballot_sync(full, live);
     int width = 32;
     while (todo) {
-        const unsigned group = lane_group(todo, width);
+        unsigned group = lane_group(todo, width);
         float m0;
-        const int state = warp_tables(T, qx, qy, group, 1, blockDim.x, wt, val_hi, m0);
-        if (state < 0 && width > 1) {
-            width >>= 1;
-            continue;
+        const int state = warp_tables(T, qx, qy, group, width, 1, blockDim.x, wt, val_hi, m0);
+        if (state < 0) {
+            if (!Tables::kLong && width <= kDeferWidth && defer_tile(df, i, j, 0u, todo)) break;
+            if (width > 1) {
+                width >>= 1;
+                continue;
+            }
+            group = todo;  // without tables: the lanes left walk side by side
         }
         todo &= ~group;
         const bool mine = (group >> lane) & 1u;
@@ -2286,6 +2443,51 @@ __global__ void __launch_bounds__(kDescentThreads, kDescentBlocks)
     if (overflow) atomicAdd(&st->overflow, 1);
 }
 
+__global__ void __launch_bounds__(kDescentThreads, kDescentBlocks)
+    k_stochastic(Tree T, const ViewState* vs, int W, int H, int K, float precision, uint64_t seed,
+                 const uint64_t* __restrict__ seed_ptr, uint32_t view, int* __restrict__ indices,
+                 float* __restrict__ probs, uds_view_stats* st, const unsigned char* __restrict__ mask,
+                 float* __restrict__ weights, Deferred df) {
+    // same tiles and tables as k_sample, then every lane draws its K paths; the
+    // masses come from the tables, from those kept per depth of earlier draws,
+    // or from the lane that needs them (all bit-identical to separate getWeight
+    // calls)
+    if (seed_ptr) seed = *seed_ptr;
+    __shared__ WarpTables s_tables[kDescentThreads / 32];
+    int i, j;
+    cell_block(T.order, vs, W, H, blockIdx.x, i, j);
+    if (i >= W || j >= H) return;  // (uniform over the block)
+    i += threadIdx.y;
+    j += threadIdx.x;
+    int tid = threadIdx.x + blockDim.x * threadIdx.y;
+    size_t pixel = (size_t)j + (size_t)H * i;
+    bool live = (i < W && j < H) && (!mask || mask[pixel]);
+    T.n = vs->n;
+    T.sq = vs->sq;
+    T.isq = vs->isq;
+    if (T.n == 0) return;
+    stochastic_tile(T, s_tables[tid >> 5], __ballot_sync(0xffffffffu, live), i, j, H, K, precision, seed, view, indices,
+                    probs, st, weights, df);
+}
+
+// The tiles that k_stochastic left for the long tables.
+__global__ void __launch_bounds__(32)
+    k_stochastic_long(Tree T, const ViewState* vs, int H, int K, float precision, uint64_t seed,
+                      const uint64_t* __restrict__ seed_ptr, uint32_t view, int* __restrict__ indices,
+                      float* __restrict__ probs, uds_view_stats* st, float* __restrict__ weights, Deferred df) {
+    __shared__ LongTables wt;
+    const unsigned count = min(df.counters[0], kDeferredTiles);
+    if (count == 0) return;  // (the counters are still clear)
+    if (seed_ptr) seed = *seed_ptr;
+    T.n = vs->n;
+    T.sq = vs->sq;
+    T.isq = vs->isq;
+    use_slab(wt, df.slabs[blockIdx.x]);
+    for (uint4 tile; next_deferred(df, count, tile);)
+        stochastic_tile(T, wt, tile.w, (int)(tile.x + threadIdx.y), (int)(tile.y + threadIdx.x), H, K, precision, seed,
+                        view, indices, probs, st, weights, df);
+}
+
 // ============================================================ proposal
 // Learned proposal for the stochastic mode (no reference counterpart).  A
 // draw descends from the root; at each internal node a small network maps
@@ -2392,35 +2594,40 @@ __global__ void __launch_bounds__(128) k_prop_dataset(Tree T, const ViewState* v
 }
 
 // Per pixel: root mass; active pixels put their K draws on the list.
-__global__ void __launch_bounds__(kDescentThreads, kDescentBlocks) k_prop_init(Tree T, const ViewState* vs, int W, int H, int K, float precision,
-                            float* __restrict__ root_mass, int* __restrict__ node_out, int* __restrict__ draw_out,
-                            float* __restrict__ logq_out, int* __restrict__ count_out, int* __restrict__ indices,
-                            float* __restrict__ weights) {
-    // root masses from the tables of k_sample (warps of consecutive
-    // threads)
-    __shared__ WarpTables s_tables[kDescentThreads / 32];
-    int j = blockIdx.x * blockDim.x + threadIdx.x;
-    int i = blockIdx.y * blockDim.y + threadIdx.y;
-    int tid = threadIdx.x + blockDim.x * threadIdx.y;
-    int warp = tid >> 5, lane = tid & 31;
-    bool live = i < W && j < H;
-    T.n = vs->n;
-    T.sq = vs->sq;
-    T.isq = vs->isq;
-    size_t pixel = (size_t)j + (size_t)H * i;
-    float qx = (float)i, qy = (float)j;
+struct PropInit {
+    int K;
+    float precision;
+    float* root_mass;
+    int *node, *draw;
+    float* logq;
+    int *count, *indices;
+    float* weights;
+};
+template <class Tables>
+__device__ __forceinline__ void prop_init_tile(const Tree& T, Tables& wt, unsigned todo, int i, int j, int H,
+                                               const PropInit& out, const Deferred& df) {
+    const int lane = (threadIdx.x + blockDim.x * threadIdx.y) & 31;
+    const size_t pixel = (size_t)j + (size_t)H * i;
+    const float qx = (float)i, qy = (float)j;
+    bool live = (todo >> lane) & 1u;
     float m0 = 0.0f;
     if (T.n > 0) {
-        float val_hi[kEvals - kRows];
-        unsigned todo = __ballot_sync(0xffffffffu, live);
+        float val_hi[Tables::kLong ? 1 : Tables::kEvals - Tables::kRows];
         int width = 32;
         while (todo) {
-            const unsigned group = lane_group(todo, width);
+            unsigned group = lane_group(todo, width);
             float total;
-            const int state = warp_tables(T, qx, qy, group, 1, blockDim.x, s_tables[warp], val_hi, total);
-            if (state < 0 && width > 1) {
-                width >>= 1;
-                continue;
+            const int state = warp_tables(T, qx, qy, group, width, 1, blockDim.x, wt, val_hi, total);
+            if (state < 0) {
+                if (!Tables::kLong && width <= kDeferWidth && defer_tile(df, i, j, 0u, todo)) {
+                    live = live && !((todo >> lane) & 1u);
+                    break;
+                }
+                if (width > 1) {
+                    width >>= 1;
+                    continue;
+                }
+                group = todo;  // without tables: the lanes left walk side by side
             }
             todo &= ~group;
             if ((group >> lane) & 1u) m0 = state < 0 ? node_weight_out_of_line(T, 0, qx, qy) : total;
@@ -2428,21 +2635,50 @@ __global__ void __launch_bounds__(kDescentThreads, kDescentBlocks) k_prop_init(T
         m0 = fmaxf(0.0f, m0);
     }
     if (!live) return;
-    root_mass[pixel] = m0;
-    if (T.n == 0 || m0 < precision) return;
+    out.root_mass[pixel] = m0;
+    if (T.n == 0 || m0 < out.precision) return;
+    const int K = out.K;
     if (T.n == 1) {  // the root is the only leaf
         for (int k = 0; k < K; ++k) {
-            indices[(size_t)K * pixel + k] = T.leaf_id[0];
-            weights[(size_t)K * pixel + k] = leaf_mass(T, T.cen[0], qx, qy) / m0;
+            out.indices[(size_t)K * pixel + k] = T.leaf_id[0];
+            out.weights[(size_t)K * pixel + k] = leaf_mass(T, T.cen[0], qx, qy) / m0;
         }
         return;
     }
-    int base = atomicAdd(count_out, K);
+    int base = atomicAdd(out.count, K);
     for (int k = 0; k < K; ++k) {
-        node_out[base + k] = 0;
-        draw_out[base + k] = (int)(pixel * K + k);
-        logq_out[base + k] = 0.0f;
+        out.node[base + k] = 0;
+        out.draw[base + k] = (int)(pixel * K + k);
+        out.logq[base + k] = 0.0f;
     }
+}
+
+__global__ void __launch_bounds__(kDescentThreads, kDescentBlocks)
+    k_prop_init(Tree T, const ViewState* vs, int W, int H, PropInit out, Deferred df) {
+    // root masses from the tables of k_sample (warps of consecutive
+    // threads)
+    __shared__ WarpTables s_tables[kDescentThreads / 32];
+    int j = blockIdx.x * blockDim.x + threadIdx.x;
+    int i = blockIdx.y * blockDim.y + threadIdx.y;
+    int tid = threadIdx.x + blockDim.x * threadIdx.y;
+    T.n = vs->n;
+    T.sq = vs->sq;
+    T.isq = vs->isq;
+    prop_init_tile(T, s_tables[tid >> 5], __ballot_sync(0xffffffffu, i < W && j < H), i, j, H, out, df);
+}
+
+// The tiles that k_prop_init left for the long tables.
+__global__ void __launch_bounds__(32)
+    k_prop_init_long(Tree T, const ViewState* vs, int H, PropInit out, Deferred df) {
+    __shared__ LongTables wt;
+    const unsigned count = min(df.counters[0], kDeferredTiles);
+    if (count == 0) return;  // (the counters are still clear)
+    T.n = vs->n;
+    T.sq = vs->sq;
+    T.isq = vs->isq;
+    use_slab(wt, df.slabs[blockIdx.x]);
+    for (uint4 tile; next_deferred(df, count, tile);)
+        prop_init_tile(T, wt, tile.w, (int)(tile.x + threadIdx.y), (int)(tile.y + threadIdx.x), H, out, df);
 }
 
 // Rows go straight into the network's operand layout: bf16, 128-row tiles of
@@ -2713,6 +2949,25 @@ static int build_views(const uds_sample_params* p, char* base, size_t slot, cons
     return UDS_OK;
 }
 
+// What the tiles left for the long tables take: their list and the slabs,
+// one per block of the second kernel (fewer for few splats, where such tiles
+// are fewer), at the end of the workspace.  None where every pixel fits the
+// short ones.
+static unsigned long_blocks(const uds_sample_params* p) {
+    if (p->N <= WarpTables::kEvals) return 0;  // (fewer nodes than splats)
+    const int n = p->N / 1024;
+    return (unsigned)(n < 8 ? 8 : n > 152 ? 152 : n);
+}
+static size_t deferred_bytes(const uds_sample_params* p) {
+    const unsigned blocks = long_blocks(p);
+    return blocks ? a256(sizeof(uint4) * kDeferredTiles) + blocks * a256(sizeof(LongSlab)) : 0;
+}
+static Deferred deferred_of(const uds_sample_params* p, const Ws& w, char* workspace, size_t workspace_bytes) {
+    char* at = workspace + ((workspace_bytes - deferred_bytes(p)) & ~(size_t)255);
+    return {w.vs->deferred, reinterpret_cast<uint4*>(at),
+            reinterpret_cast<LongSlab*>(at + a256(sizeof(uint4) * kDeferredTiles))};
+}
+
 // Leaves one order-sampling round considers: the descent stops at the first
 // node holding at most max(K, leaf_size) splats.
 static int candidates(const uds_sample_params* p) { return p->leaf_size > p->K ? p->leaf_size : p->K; }
@@ -2728,57 +2983,70 @@ static Tree tree_of(const Ws& w) {
     return T;
 }
 
-template <int R>
 // Descent for views view .. view + nviews - 1 in one launch (grid.y = view),
-// their trees vstride bytes apart in the workspace.
-// Block: tile_x (y) by kDescentThreads / tile_x (x) pixels; each warp is a
-// tile_x by 32 / tile_x pixel tile.  Every lane's walk is its own, so the
-// indices do not depend on the tile shape, only the speed does.
-static void launch_sample(const Tree& T, const Ws& w, const uds_sample_params* p, const float* u, int view,
-                          int* idx, cudaStream_t s, int nviews = 1, size_t vstride = 0) {
-    int tx = tile_of(p);
-    dim3 block(tx, kDescentThreads / tx);
-    dim3 grid(cell_blocks(p->W, p->H, block), nviews);
-    size_t istride = (size_t)p->W * p->H * p->K;
-    const int M = candidates(p);
-    size_t ustride = (size_t)p->W * p->H * R * M;
+// their trees vstride bytes apart in the workspace, and that of the tiles it
+// leaves for the long tables.  Block: tile_x (y) by kDescentThreads / tile_x
+// (x) pixels; each warp is a tile_x by 32 / tile_x pixel tile.  Every lane's
+// walk is its own, so the indices do not depend on the tile shape, only the
+// speed does.
+template <int R>
+static int launch_sample(const Tree& T, const Ws& w, const uds_sample_params* p, const Deferred& df, const float* u,
+                         int view, int* idx, cudaStream_t s, int nviews = 1, size_t vstride = 0) {
+    // the K smallest keys in registers up to 16, in shared memory above
+    constexpr bool kEight = R <= 3;
+    constexpr int RR = R >= 3 ? R : 3, KM = RR <= 4 ? 16 : kMaxK;
+    const int tx = tile_of(p), M = candidates(p);
+    const size_t istride = (size_t)p->W * p->H * p->K, ustride = (size_t)p->W * p->H * R * M;
+    const unsigned more = long_blocks(p);
+    const dim3 tile(tx, 32 / tx);
     UnevenViews none{};
-    if (R <= 3 && p->K <= 8) {
-        constexpr int RR = R <= 3 ? R : 3;
-        if (p->spread)
-            k_sample<RR, 8, false, true><<<grid, block, 0, s>>>(T, w.vs, p->W, p->H, p->K, M, p->precision, u, p->seed,
-                                                                p->seed_dev, (uint32_t)view, idx, w.stats + view,
-                                                                vstride, ustride, istride, none);
-        else
-            k_sample<RR, 8, false, false><<<grid, block, 0, s>>>(T, w.vs, p->W, p->H, p->K, M, p->precision, u,
-                                                                 p->seed, p->seed_dev, (uint32_t)view, idx,
-                                                                 w.stats + view, vstride, ustride, istride, none);
+    auto launch = [&](auto kernel, auto rest, int warps, size_t list) {
+        const dim3 block(tx, 32 * warps / tx), grid(cell_blocks(p->W, p->H, block), nviews);
+        kernel<<<grid, block, list, s>>>(T, w.vs, p->W, p->H, p->K, M, p->precision, u, p->seed, p->seed_dev,
+                                         (uint32_t)view, idx, w.stats + view, vstride, ustride, istride, none, df);
+        if (more)
+            rest<<<more, tile, list, s>>>(T, w.vs, p->H, p->K, M, p->precision, u, p->seed, p->seed_dev,
+                                          (uint32_t)view, idx, w.stats + view, vstride, ustride, istride, none, df);
+    };
+    if (kEight && p->K <= 8) {
+        constexpr int R8 = kEight ? R : 3;
+        launch(p->spread ? k_sample<R8, 8, false, true> : k_sample<R8, 8, false, false>, k_sample_long<R8, 8>,
+               kDescentWarps<8>, 0);
     } else {
-        // the K smallest keys in registers up to 16, in shared memory above
-        constexpr int RR = R >= 3 ? R : 3, KM = RR <= 4 ? 16 : kMaxK;
-        dim3 block(tx, 32 * kDescentWarps<KM> / tx);
-        dim3 grid(cell_blocks(p->W, p->H, block), nviews);
-        k_sample<RR, KM, false, true><<<grid, block, KM <= 16 ? 0 : 256 * (size_t)p->K, s>>>(
-            T, w.vs, p->W, p->H, p->K, M, p->precision, u, p->seed, p->seed_dev, (uint32_t)view, idx,
-            w.stats + view, vstride, ustride, istride, none);
+        launch(k_sample<RR, KM, false, true>, k_sample_long<RR, KM>, kDescentWarps<KM>,
+               KM <= 16 ? 0 : 256 * (size_t)p->K);
+    }
+    return launch_status(more ? 2 : 1);
+}
+static int launch_descent(const Tree& T, const Ws& w, const uds_sample_params* p, const Deferred& df, const float* u,
+                          int view, int* idx, cudaStream_t s, int nviews = 1, size_t vstride = 0) {
+    switch (num_rounds(p->K)) {
+        case 1: return launch_sample<1>(T, w, p, df, u, view, idx, s, nviews, vstride);
+        case 2: return launch_sample<2>(T, w, p, df, u, view, idx, s, nviews, vstride);
+        case 3: return launch_sample<3>(T, w, p, df, u, view, idx, s, nviews, vstride);
+        case 4: return launch_sample<4>(T, w, p, df, u, view, idx, s, nviews, vstride);
+        case 5: return launch_sample<5>(T, w, p, df, u, view, idx, s, nviews, vstride);
+        case 6: return launch_sample<6>(T, w, p, df, u, view, idx, s, nviews, vstride);
+        case 7: return launch_sample<7>(T, w, p, df, u, view, idx, s, nviews, vstride);
+        default: return launch_sample<8>(T, w, p, df, u, view, idx, s, nviews, vstride);
     }
 }
 
 // Views of different sizes (K <= 8) in one launch: a one-dimensional grid of
 // every view's blocks; uv built by the caller.
 template <int R>
-static void launch_sample_uneven(const Tree& T, const Ws& w, const uds_sample_params* p, const UnevenViews& uv,
-                                 int* idx, cudaStream_t s, size_t vstride) {
-    int tx = tile_of(p);
-    dim3 block(tx, kDescentThreads / tx);
-    if (p->spread)
-        k_sample<R, 8, true, true><<<uv.first[uv.nv], block, 0, s>>>(T, w.vs, 0, 0, p->K, candidates(p), p->precision,
-                                                                     nullptr, p->seed, p->seed_dev, 0u, idx, w.stats,
-                                                                     vstride, 0, 0, uv);
-    else
-        k_sample<R, 8, true, false><<<uv.first[uv.nv], block, 0, s>>>(T, w.vs, 0, 0, p->K, candidates(p),
-                                                                      p->precision, nullptr, p->seed, p->seed_dev,
-                                                                      0u, idx, w.stats, vstride, 0, 0, uv);
+static int launch_sample_uneven(const Tree& T, const Ws& w, const uds_sample_params* p, const Deferred& df,
+                                const UnevenViews& uv, int* idx, cudaStream_t s, size_t vstride) {
+    const int tx = tile_of(p), M = candidates(p);
+    const unsigned more = long_blocks(p);
+    auto kernel = p->spread ? k_sample<R, 8, true, true> : k_sample<R, 8, true, false>;
+    kernel<<<uv.first[uv.nv], dim3(tx, kDescentThreads / tx), 0, s>>>(T, w.vs, 0, 0, p->K, M, p->precision, nullptr,
+                                                                     p->seed, p->seed_dev, 0u, idx, w.stats, vstride,
+                                                                     0, 0, uv, df);
+    if (more)
+        k_sample_long<R, 8><<<more, dim3(tx, 32 / tx), 0, s>>>(T, w.vs, 0, p->K, M, p->precision, nullptr, p->seed,
+                                                              p->seed_dev, 0u, idx, w.stats, vstride, 0, 0, uv, df);
+    return launch_status(more ? 2 : 1);
 }
 
 static int check_params(const uds_sample_params* p) {
@@ -2811,7 +3079,7 @@ using namespace uds;
 // descent launch covers all views; the other entry points use slot 0.
 extern "C" size_t uds_sample_workspace_size(const uds_sample_params* prm) {
     if (check_params(prm)) return 0;
-    return layout(prm, nullptr).bytes * (size_t)prm->B;
+    return layout(prm, nullptr).bytes * (size_t)prm->B + deferred_bytes(prm);
 }
 
 extern "C" int uds_sample(const uds_sample_params* prm, const float* points, const float* normals,
@@ -2824,7 +3092,7 @@ extern "C" int uds_sample(const uds_sample_params* prm, const float* points, con
     char* base = reinterpret_cast<char*>(workspace);
     Ws w = layout(prm, base);
     size_t slot = w.bytes;
-    if (!workspace || workspace_bytes < slot * (size_t)prm->B) return UDS_ERR_WORKSPACE;
+    if (!workspace || workspace_bytes < slot * (size_t)prm->B + deferred_bytes(prm)) return UDS_ERR_WORKSPACE;
     cudaStream_t s = as_stream(stream);
     size_t per_view = (size_t)prm->W * prm->H * prm->K;
     cudaError_t e = cudaMemsetAsync(indices, 0xFF, sizeof(int32_t) * per_view * prm->B, s);
@@ -2832,19 +3100,8 @@ extern "C" int uds_sample(const uds_sample_params* prm, const float* points, con
     if ((st = build_views(prm, base, slot, nullptr, points, normals, std_devs, h_override, s))) return st;
     if (prm->N > 0) {
         // one descent launch over all views
-        Tree T = tree_of(w);
-        int B = prm->B;
-        switch (num_rounds(prm->K)) {
-            case 1: launch_sample<1>(T, w, prm, uniforms, 0, indices, s, B, slot); break;
-            case 2: launch_sample<2>(T, w, prm, uniforms, 0, indices, s, B, slot); break;
-            case 3: launch_sample<3>(T, w, prm, uniforms, 0, indices, s, B, slot); break;
-            case 4: launch_sample<4>(T, w, prm, uniforms, 0, indices, s, B, slot); break;
-            case 5: launch_sample<5>(T, w, prm, uniforms, 0, indices, s, B, slot); break;
-            case 6: launch_sample<6>(T, w, prm, uniforms, 0, indices, s, B, slot); break;
-            case 7: launch_sample<7>(T, w, prm, uniforms, 0, indices, s, B, slot); break;
-            default: launch_sample<8>(T, w, prm, uniforms, 0, indices, s, B, slot); break;
-        }
-        if ((st = launch_status())) return st;
+        const Deferred df = deferred_of(prm, w, base, workspace_bytes);
+        if ((st = launch_descent(tree_of(w), w, prm, df, uniforms, 0, indices, s, prm->B, slot))) return st;
     }
     if (stats) {
         e = cudaMemcpyAsync(stats, w.stats, sizeof(uds_view_stats) * prm->B, cudaMemcpyDeviceToDevice, s);
@@ -2872,7 +3129,7 @@ extern "C" int uds_sample_views(const uds_sample_params* prm, const uds_view_des
     char* base = reinterpret_cast<char*>(workspace);
     Ws w = layout(prm, base);
     size_t slot = w.bytes;  // does not depend on the image size
-    if (!workspace || workspace_bytes < slot * (size_t)prm->B) return UDS_ERR_WORKSPACE;
+    if (!workspace || workspace_bytes < slot * (size_t)prm->B + deferred_bytes(prm)) return UDS_ERR_WORKSPACE;
     cudaStream_t s = as_stream(stream);
     cudaError_t e = cudaMemsetAsync(indices, 0xFF, sizeof(int32_t) * total, s);
     if (e != cudaSuccess) { set_last_error(e); return UDS_ERR_CUDA; }
@@ -2895,12 +3152,13 @@ extern "C" int uds_sample_views(const uds_sample_params* prm, const uds_view_des
                 off += (long long)views[b].W * views[b].H * prm->K;
             }
             uv.first[prm->B] = blocks;
+            const Deferred df = deferred_of(prm, w, base, workspace_bytes);
             switch (R) {
-                case 1: launch_sample_uneven<1>(T, w, prm, uv, indices, s, slot); break;
-                case 2: launch_sample_uneven<2>(T, w, prm, uv, indices, s, slot); break;
-                default: launch_sample_uneven<3>(T, w, prm, uv, indices, s, slot); break;
+                case 1: st = launch_sample_uneven<1>(T, w, prm, df, uv, indices, s, slot); break;
+                case 2: st = launch_sample_uneven<2>(T, w, prm, df, uv, indices, s, slot); break;
+                default: st = launch_sample_uneven<3>(T, w, prm, df, uv, indices, s, slot); break;
             }
-            if ((st = launch_status())) return st;
+            if (st) return st;
         } else {
             size_t off = 0;
             for (int b = 0; b < prm->B; ++b) {
@@ -2909,18 +3167,8 @@ extern "C" int uds_sample_views(const uds_sample_params* prm, const uds_view_des
                 pv.H = views[b].H;
                 Ws wb = layout(&pv, base + slot * (size_t)b);
                 wb.stats = w.stats;
-                Tree Tb = tree_of(wb);
-                switch (R) {
-                    case 1: launch_sample<1>(Tb, wb, &pv, nullptr, b, indices + off, s); break;
-                    case 2: launch_sample<2>(Tb, wb, &pv, nullptr, b, indices + off, s); break;
-                    case 3: launch_sample<3>(Tb, wb, &pv, nullptr, b, indices + off, s); break;
-                    case 4: launch_sample<4>(Tb, wb, &pv, nullptr, b, indices + off, s); break;
-                    case 5: launch_sample<5>(Tb, wb, &pv, nullptr, b, indices + off, s); break;
-                    case 6: launch_sample<6>(Tb, wb, &pv, nullptr, b, indices + off, s); break;
-                    case 7: launch_sample<7>(Tb, wb, &pv, nullptr, b, indices + off, s); break;
-                    default: launch_sample<8>(Tb, wb, &pv, nullptr, b, indices + off, s); break;
-                }
-                if ((st = launch_status())) return st;
+                const Deferred df = deferred_of(prm, wb, base, workspace_bytes);
+                if ((st = launch_descent(tree_of(wb), wb, &pv, df, nullptr, b, indices + off, s))) return st;
                 off += (size_t)views[b].W * views[b].H * prm->K;
             }
         }
@@ -2932,6 +3180,23 @@ extern "C" int uds_sample_views(const uds_sample_params* prm, const uds_view_des
     return UDS_OK;
 }
 
+namespace uds {
+// Draws of one view's pixels (with a mask: of those it marks).
+static int launch_stochastic(const Ws& w, const uds_sample_params* p, const Deferred& df, int view, int* idx,
+                             float* probs, const unsigned char* mask, float* weights, cudaStream_t s) {
+    const dim3 block(8, kDescentThreads / 8);
+    const Tree T = tree_of(w);
+    const unsigned more = long_blocks(p);
+    k_stochastic<<<cell_blocks(p->W, p->H, block), block, 0, s>>>(T, w.vs, p->W, p->H, p->K, p->precision, p->seed,
+                                                                  p->seed_dev, (uint32_t)view, idx, probs,
+                                                                  w.stats + view, mask, weights, df);
+    if (more)
+        k_stochastic_long<<<more, dim3(8, 4), 0, s>>>(T, w.vs, p->H, p->K, p->precision, p->seed, p->seed_dev,
+                                                      (uint32_t)view, idx, probs, w.stats + view, weights, df);
+    return launch_status(more ? 2 : 1);
+}
+}  // namespace uds
+
 extern "C" int uds_sample_stochastic(const uds_sample_params* prm, const float* points, const float* normals,
                                      const float* std_devs, const float* h_override, int32_t* indices,
                                      float* probs, uds_view_stats* stats, void* workspace, size_t workspace_bytes,
@@ -2939,23 +3204,20 @@ extern "C" int uds_sample_stochastic(const uds_sample_params* prm, const float* 
     int st = check_params(prm);
     if (st) return st;
     if (!indices || !probs || (prm->N > 0 && (!points || !normals || !std_devs))) return UDS_ERR_ARGUMENT;
-    Ws w = layout(prm, reinterpret_cast<char*>(workspace));
-    if (!workspace || workspace_bytes < w.bytes) return UDS_ERR_WORKSPACE;
+    char* base = reinterpret_cast<char*>(workspace);
+    Ws w = layout(prm, base);
+    if (!workspace || workspace_bytes < w.bytes + deferred_bytes(prm)) return UDS_ERR_WORKSPACE;
     cudaStream_t s = as_stream(stream);
     size_t per_view = (size_t)prm->W * prm->H * prm->K;
     cudaError_t e = cudaMemsetAsync(indices, 0xFF, sizeof(int32_t) * per_view * prm->B, s);
     if (e == cudaSuccess) e = cudaMemsetAsync(probs, 0, sizeof(float) * per_view * prm->B, s);
     if (e != cudaSuccess) { set_last_error(e); return UDS_ERR_CUDA; }
-    Tree T = tree_of(w);
-    dim3 block(8, kDescentThreads / 8);
-    const unsigned grid = cell_blocks(prm->W, prm->H, block);
+    const Deferred df = deferred_of(prm, w, base, workspace_bytes);
     for (int b = 0; b < prm->B; ++b) {
         if ((st = build_view(prm, w, b, points, normals, std_devs, h_override, s))) return st;
         if (prm->N == 0) continue;
-        k_stochastic<<<grid, block, 0, s>>>(T, w.vs, prm->W, prm->H, prm->K, prm->precision, prm->seed, prm->seed_dev,
-                                            (uint32_t)b, indices + per_view * b, probs + per_view * b, w.stats + b,
-                                            nullptr, nullptr);
-        if ((st = launch_status())) return st;
+        if ((st = launch_stochastic(w, prm, df, b, indices + per_view * b, probs + per_view * b, nullptr, nullptr, s)))
+            return st;
     }
     if (stats) {
         e = cudaMemcpyAsync(stats, w.stats, sizeof(uds_view_stats) * prm->B, cudaMemcpyDeviceToDevice, s);
@@ -3025,21 +3287,11 @@ extern "C" int uds_sample_descent(const uds_sample_params* prm, int view, const 
     if (st) return st;
     if (view < 0 || view >= prm->B || !indices) return UDS_ERR_ARGUMENT;
     Ws w = layout(prm, reinterpret_cast<char*>(workspace));
-    if (!workspace || workspace_bytes < w.bytes) return UDS_ERR_WORKSPACE;
+    if (!workspace || workspace_bytes < w.bytes + deferred_bytes(prm)) return UDS_ERR_WORKSPACE;
     if (prm->N == 0) return UDS_OK;
     cudaStream_t s = as_stream(stream);
-    Tree T = tree_of(w);
-    switch (num_rounds(prm->K)) {
-        case 1: launch_sample<1>(T, w, prm, uniforms, view, indices, s); break;
-        case 2: launch_sample<2>(T, w, prm, uniforms, view, indices, s); break;
-        case 3: launch_sample<3>(T, w, prm, uniforms, view, indices, s); break;
-        case 4: launch_sample<4>(T, w, prm, uniforms, view, indices, s); break;
-        case 5: launch_sample<5>(T, w, prm, uniforms, view, indices, s); break;
-        case 6: launch_sample<6>(T, w, prm, uniforms, view, indices, s); break;
-        case 7: launch_sample<7>(T, w, prm, uniforms, view, indices, s); break;
-        default: launch_sample<8>(T, w, prm, uniforms, view, indices, s); break;
-    }
-    return launch_status();
+    const Deferred df = deferred_of(prm, w, reinterpret_cast<char*>(workspace), workspace_bytes);
+    return launch_descent(tree_of(w), w, prm, df, uniforms, view, indices, s);
 }
 
 extern "C" int uds_fgt_eval(const uds_sample_params* prm, int m, const int32_t* nodes, const float* query_xy,
@@ -3093,7 +3345,7 @@ static PropWs prop_layout(const uds_sample_params* p, char* base) {
 
 extern "C" size_t uds_proposal_workspace_size(const uds_sample_params* prm) {
     if (check_params(prm)) return 0;
-    return layout(prm, nullptr).bytes + prop_layout(prm, nullptr).bytes;
+    return layout(prm, nullptr).bytes + prop_layout(prm, nullptr).bytes + deferred_bytes(prm);
 }
 
 extern "C" int uds_sample_proposal(const uds_sample_params* prm, const float* points, const float* normals,
@@ -3108,7 +3360,7 @@ extern "C" int uds_sample_proposal(const uds_sample_params* prm, const float* po
     char* base = reinterpret_cast<char*>(workspace);
     Ws w = layout(prm, base);
     PropWs q = prop_layout(prm, base ? base + w.bytes : nullptr);
-    if (!workspace || workspace_bytes < w.bytes + q.bytes) return UDS_ERR_WORKSPACE;
+    if (!workspace || workspace_bytes < w.bytes + q.bytes + deferred_bytes(prm)) return UDS_ERR_WORKSPACE;
     cudaStream_t s = as_stream(stream);
     size_t P = (size_t)prm->W * prm->H, per_view = P * prm->K;
     cudaError_t e = cudaMemsetAsync(indices, 0xFF, sizeof(int32_t) * per_view * prm->B, s);
@@ -3118,6 +3370,8 @@ extern "C" int uds_sample_proposal(const uds_sample_params* prm, const float* po
     Tree T = tree_of(w);
     dim3 block(8, kDescentThreads / 8);
     dim3 grid(cdiv(prm->H, block.x), cdiv(prm->W, block.y));
+    const Deferred df = deferred_of(prm, w, base, workspace_bytes);
+    const unsigned more = long_blocks(prm);
     for (int b = 0; b < prm->B; ++b) {
         if ((st = build_view(prm, w, b, points, normals, std_devs, h_override, s))) return st;
         if (prm->N == 0) continue;
@@ -3127,9 +3381,10 @@ extern "C" int uds_sample_proposal(const uds_sample_params* prm, const float* po
         if (mlp_params) {
             e = cudaMemsetAsync(q.counts, 0, 16, s);
             if (e != cudaSuccess) { set_last_error(e); return UDS_ERR_CUDA; }
-            k_prop_init<<<grid, block, 0, s>>>(T, w.vs, prm->W, prm->H, prm->K, prm->precision, q.root_mass,
-                                               q.node[0], q.draw[0], q.logq[0], q.counts, idx, wt);
-            if ((st = launch_status())) return st;
+            const PropInit out{prm->K, prm->precision, q.root_mass, q.node[0], q.draw[0], q.logq[0], q.counts, idx, wt};
+            k_prop_init<<<grid, block, 0, s>>>(T, w.vs, prm->W, prm->H, out, df);
+            if (more) k_prop_init_long<<<more, dim3(8, 4), 0, s>>>(T, w.vs, prm->H, out, df);
+            if ((st = launch_status(more ? 2 : 1))) return st;
             unsigned nb = cdiv(per_view, 256);
             int cur = 0;
             for (int level = 0; level < kTrace; ++level) {
@@ -3169,10 +3424,7 @@ extern "C" int uds_sample_proposal(const uds_sample_params* prm, const float* po
         }
         // the plain stochastic sampler: every pixel, or the fallback pixels
         float* probs = q.logits;  // scratch for the path probabilities
-        const unsigned cells = cell_blocks(prm->W, prm->H, block);
-        k_stochastic<<<cells, block, 0, s>>>(T, w.vs, prm->W, prm->H, prm->K, prm->precision, prm->seed,
-                                             prm->seed_dev, (uint32_t)b, idx, probs, w.stats + b, mask, wt);
-        if ((st = launch_status())) return st;
+        if ((st = launch_stochastic(w, prm, df, b, idx, probs, mask, wt, s))) return st;
     }
     if (stats) {
         e = cudaMemcpyAsync(stats, w.stats, sizeof(uds_view_stats) * prm->B, cudaMemcpyDeviceToDevice, s);
