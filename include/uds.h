@@ -14,7 +14,8 @@
  *    callers may pass uninitialised memory;
  *  - scratch memory is caller-owned: query its size with the matching
  *    *_workspace_size function and pass a device buffer of at least that many
- *    bytes (16-byte aligned).  Nothing here calls cudaMalloc, so every call is
+ *    bytes (16-byte aligned).  It belongs to the call until the GPU has
+ *    finished it: calls on two streams need two.  Nothing here calls cudaMalloc, so every call is
  *    safe inside CUDA graph capture;
  *  - the return value is a uds_status; uds_status_string() names it.
  */
@@ -132,7 +133,7 @@ int uds_backface_backward(int B, int N, const float* cam_normals, const float* g
  *      uniforms from seed.
  *      h_override: optional device float[B]; entries > 0 replace the
  *      computed bandwidth.  stats: device uds_view_stats[B] (may be NULL).
- *      Workspace: B trees, and up to 108 MB (once per call) for tiles with
+ *      Workspace: B trees, and up to 111 MB (once per call) for tiles with
  *      pixels that meet thousands of tree nodes. ---- */
 size_t uds_sample_workspace_size(const uds_sample_params* prm);
 int uds_sample(const uds_sample_params* prm, const float* points, const float* normals,

@@ -220,20 +220,17 @@ def need(t: torch.Tensor, name: str, dtype=torch.float32, device=None) -> torch.
 
 
 class Workspace:
-    """Per-device scratch buffer for the C ABI, taken from torch's caching
-    allocator and grown on demand (never shrunk)."""
-
-    _bufs: dict = {}
+    """Scratch buffers for the C ABI.  Each call takes its own from torch's
+    caching allocator: the kernels keep counters and words that blocks wait
+    for in it, so calls on two streams or from two threads must not share
+    one.  Freed when the call has been enqueued, it is given out again on the
+    same stream only; a captured call's belongs to its graph."""
 
     @classmethod
     def get(cls, device: torch.device, nbytes: int, slot: str = "default") -> torch.Tensor:
-        key = (device.index if device.index is not None else torch.cuda.current_device(), slot)
-        buf = cls._bufs.get(key)
-        if buf is None or buf.numel() < nbytes:
-            buf = torch.empty(max(int(nbytes), 256), dtype=torch.uint8, device=device)
-            cls._bufs[key] = buf
-        return buf
+        return torch.empty(max(int(nbytes), 256), dtype=torch.uint8, device=device)
 
     @classmethod
     def reserve(cls, device: torch.device, nbytes: int, slot: str = "default") -> None:
+        """Leaves a block of this size in the allocator's cache."""
         cls.get(device, nbytes, slot)

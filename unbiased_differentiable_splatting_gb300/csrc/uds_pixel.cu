@@ -117,6 +117,7 @@ __global__ void __launch_bounds__(kTileThreads) k_pixel_pack(size_t S, size_t pe
     if (threadIdx.x == 0) s_tile = (int)atomicAdd(&gs->ticket[kGatherPasses], 1u);
     for (int d = threadIdx.x; d < passes * kDigits; d += kTileThreads) digits[d] = 0;
     __syncthreads();
+    if (s_tile >= (int)gridDim.x) return;  // (a scratch that another call uses at the same time)
     const size_t first = (size_t)s_tile * kPackTile + threadIdx.x;
     auto sample = [&](int r) {
         const size_t t = first + r * kTileThreads;

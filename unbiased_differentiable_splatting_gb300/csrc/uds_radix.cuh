@@ -116,6 +116,7 @@ __device__ __forceinline__ bool sort_tile(unsigned n, int shift, unsigned* ticke
     for (int d = lane; d < kDigits; d += 32) wcnt[warp][d] = 0;
     __syncthreads();
     const int tile = s_tile;
+    if ((unsigned long long)tile * (ITEMS * kTileThreads) >= n) return true;  // (uniform over the block)
     uint32_t key[ITEMS], val[ITEMS];
     unsigned rank[ITEMS];
     const unsigned lt = (1u << lane) - 1u;

@@ -333,6 +333,7 @@ __global__ void __launch_bounds__(kTileThreads) k_cull(int N, Batch bt, const fl
     for (int d = threadIdx.x; d < kPasses * kDigits; d += kTileThreads) digits[0][d] = 0;
     __syncthreads();
     const int tile = s_tile;
+    if (tile >= (int)gridDim.x) return;  // (a workspace that another call uses at the same time)
     const float W = (float)bt.W[k], H = (float)bt.H[k], f = bt.f[k];
     const float lx = vs->lo_x, hx = vs->hi_x, ly = vs->lo_y, hy = vs->hi_y;
     unsigned key[kTileItems], ball[kTileItems];
@@ -734,6 +735,7 @@ __global__ void __launch_bounds__(kNodeTile) k_p2m(Batch bt, ViewState* vs, size
     // 32 consecutive internal nodes per warp: lane l loads the record and
     // links of its node, finds the place of its coefficients, then the warp
     // builds the nodes' expansions
+    if (s_tile >= tiles) return;  // (as in k_cull)
     const int vl = s_tile * kNodeTile + (int)threadIdx.x;
     const bool inner = vl < n - 1;
     float4 cl = inner ? cen[vl] : make_float4(0.0f, 0.0f, 0.0f, make_meta(0, -1));

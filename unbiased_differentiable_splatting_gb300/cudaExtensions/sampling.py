@@ -284,7 +284,7 @@ def build_tree(width, height, focallength, points, normals, stdDevs, numSamples,
 
 
 def fgt_eval(tree: dict, nodes, queries):
-    """getWeight of (node, query) pairs on the tree last built by build_tree."""
+    """getWeight of (node, query) pairs on a tree built by build_tree."""
     ws = tree["_ws"]
     nodes = need(nodes, "nodes", torch.int32)
     queries = need(queries, "queries", device=nodes.device)
