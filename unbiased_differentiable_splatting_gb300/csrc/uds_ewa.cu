@@ -674,8 +674,10 @@ static int mark_sampled(int B, size_t S, int N, const int32_t* indices, unsigned
         const size_t chunk = ((S + blocks - 1) / blocks + 3) / 4 * 4, bytes = (size_t)range / 8;
         const dim3 grid(cdiv(S, chunk), B, ranges);
         auto kernel = vec ? k_ewa_mark<true> : k_ewa_mark<false>;
+        // (the largest map's size, whatever this one's: the attribute is the
+        // function's, and another thread may be between this and its launch)
         if (e == cudaSuccess && bytes > 48 * 1024)
-            e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+            e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kRange / 8);
         if (e == cudaSuccess) kernel<<<grid, kMarkThreads, bytes, s>>>(S, chunk, indices, N, range, used);
     } else if (e == cudaSuccess) {
         k_ewa_mark_direct<<<dim3(cdiv(S, 256), B), 256, 0, s>>>(S, indices, N, used);
