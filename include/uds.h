@@ -293,7 +293,8 @@ int uds_mma_probe(int N, int K, const uint16_t* A, const uint16_t* B, float* C, 
 /* Proposal network 16 -> 64 -> 64 -> 64 -> 2 (ReLU), parameters fp32 in one
  * array of uds_mlp_param_count() floats: W1 (64x16), b1, W2 (64x64), b2,
  * W3 (64x64), b3, W4 (16x64, rows 2..15 zero), b4 (16).  Computed in bf16
- * with fp32 accumulation.  uds_mlp_forward: X (R x 16) -> logits (R x 2). */
+ * with fp32 accumulation.  uds_mlp_forward: X (R x 16) -> logits (R x 2).  X
+ * of these and the gradients below starts on 16 bytes. */
 int uds_mlp_param_count(void);
 int uds_mlp_forward(int R, const float* X, const float* params, float* logits, int* err, void* stream);
 /* Same, the row count read on the device from *R_dev (at most R_max rows). */

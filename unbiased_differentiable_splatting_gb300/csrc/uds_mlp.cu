@@ -779,11 +779,14 @@ __global__ void k_mlp_adam(float* __restrict__ P, float* __restrict__ G, float* 
 
 }  // namespace uds
 
+// Feature rows are read 16 bytes at a time.
+static bool misaligned(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15) != 0; }
+
 extern "C" int uds_mlp_param_count(void) { return uds::mlp::kParams; }
 
 extern "C" int uds_mlp_forward(int R, const float* X, const float* params, float* logits, int* err, void* stream) {
     using namespace uds;
-    if (R < 0 || (R > 0 && (!X || !params || !logits)) || !err) return UDS_ERR_ARGUMENT;
+    if (R < 0 || (R > 0 && (!X || !params || !logits)) || !err || misaligned(X)) return UDS_ERR_ARGUMENT;
     if (R == 0) return UDS_OK;
     static bool attr = false;
     size_t smem = sizeof(MlpFwdSmem) + 1024;
@@ -804,7 +807,8 @@ extern "C" int uds_mlp_forward(int R, const float* X, const float* params, float
 extern "C" int uds_mlp_forward_dev(int R_max, const int* R_dev, const float* X, const float* params, float* logits,
                                    int* err, void* stream) {
     using namespace uds;
-    if (R_max < 0 || !R_dev || (R_max > 0 && (!X || !params || !logits)) || !err) return UDS_ERR_ARGUMENT;
+    if (R_max < 0 || !R_dev || (R_max > 0 && (!X || !params || !logits)) || !err || misaligned(X))
+        return UDS_ERR_ARGUMENT;
     if (R_max == 0) return UDS_OK;
     static bool attr = false;
     size_t smem = sizeof(MlpFwdSmem) + 1024;
@@ -837,7 +841,8 @@ extern "C" size_t uds_mlp_grad_workspace_size(int R) {
 static int mlp_grad(int R, const long long* rows, int n, const float* X, const float* target, const float* params,
                     float* grad, float* loss, int* err, void* workspace, size_t workspace_bytes, void* stream) {
     using namespace uds;
-    if (R < 0 || (R > 0 && (!X || !target || !params || !grad || !loss)) || !err) return UDS_ERR_ARGUMENT;
+    if (R < 0 || (R > 0 && (!X || !target || !params || !grad || !loss)) || !err || misaligned(X))
+        return UDS_ERR_ARGUMENT;
     if (R == 0) return UDS_OK;
     if (!workspace || workspace_bytes < uds_mlp_grad_workspace_size(R)) return UDS_ERR_WORKSPACE;
     static bool attr = false;
@@ -883,7 +888,7 @@ extern "C" int uds_mlp_forward_tiles(int R_max, const int* R_dev, const void* X_
                                      float* logits, int* err, void* stream) {
     using namespace uds;
     if (R_max < 0 || (R_max > 0 && (!X_tiles || !params || !logits)) || !err) return UDS_ERR_ARGUMENT;
-    if ((reinterpret_cast<uintptr_t>(X_tiles) & 15) != 0) return UDS_ERR_ARGUMENT;
+    if (misaligned(X_tiles)) return UDS_ERR_ARGUMENT;
     if (R_max == 0) return UDS_OK;
     static bool attr = false;
     size_t smem = sizeof(MlpTileSmem) + 1024;

@@ -42,6 +42,15 @@ def init_params(seed: int = 0, device="cuda") -> torch.Tensor:
     return P.to(device)
 
 
+def _features(X, device) -> torch.Tensor:
+    """(R,16) float32 feature rows as the kernels read them, 16 bytes at a
+    time: a copy where the storage starts off such a boundary."""
+    X = need(X, "features", device=device)
+    if X.dim() < 2 or X.numel() != 16 * X.shape[0]:
+        raise ValueError(f"features must be (R,16), got {tuple(X.shape)}")
+    return X if X.data_ptr() % 16 == 0 else X.detach().clone()
+
+
 class ProposalNet:
     """Parameters + Adam state of the proposal network, trained and
     evaluated by the library's tensor-core kernels."""
@@ -56,7 +65,7 @@ class ProposalNet:
         self._err = torch.zeros(1, dtype=torch.int32, device=self.device)
 
     def logits(self, X: torch.Tensor) -> torch.Tensor:
-        X = need(X, "features", device=self.device)
+        X = _features(X, self.device)
         out = torch.empty((X.shape[0], 2), device=self.device)
         check(load().uds_mlp_forward(X.shape[0], ptr(X), ptr(self.params), ptr(out), ptr(self._err),
                                      stream_ptr(self.device)), "mlp forward")
@@ -66,8 +75,11 @@ class ProposalNet:
               seed: int = 0):
         """Adam on the mean cross-entropy between softmax(logits) and
         (target, 1 - target); returns the loss of each step (a device tensor)."""
-        X = need(X, "features", device=self.device)
+        X = _features(X, self.device)
         target = need(target, "target", device=self.device)
+        if target.dim() == 0 or target.shape[0] < X.shape[0] or target.numel() != target.shape[0]:
+            raise ValueError(f"target must hold one number per row of features ({X.shape[0]}), got "
+                             f"{tuple(target.shape)}")
         L = load()
         s = stream_ptr(self.device)
         g = torch.Generator(device=self.device).manual_seed(seed)
