@@ -219,6 +219,12 @@ def need(t: torch.Tensor, name: str, dtype=torch.float32, device=None) -> torch.
     return t
 
 
+def need_numel(t: torch.Tensor, count: int, name: str) -> None:
+    """The kernels index an array by the sizes of the others."""
+    if t.numel() != count:
+        raise ValueError(f"{name} must have {count} elements, got shape {tuple(t.shape)}")
+
+
 class Workspace:
     """Scratch buffers for the C ABI.  Each call takes its own from torch's
     caching allocator: the kernels keep counters and words that blocks wait

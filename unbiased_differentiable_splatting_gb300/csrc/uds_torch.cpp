@@ -42,6 +42,11 @@ const Tensor& need(const Tensor& t, const char* name, const Tensor* like = nullp
     return t;
 }
 
+// The kernels index an array by the sizes of the others.
+void need_numel(const Tensor& t, int64_t count, const char* name) {
+    TORCH_CHECK_VALUE(t.numel() == count, name, " must have ", count, " elements, got shape ", t.sizes());
+}
+
 // The UdsError of _lib.py, raised for a failing status of the C ABI.
 void check(int status, const char* what) {
     if (status == UDS_OK) return;
@@ -110,6 +115,8 @@ struct Transform {
         need(g, "gradIn");
         need(M, "transformation", &g);
         need(v, "vector", &g);
+        TORCH_CHECK_VALUE(M.dim() == 3 && M.size(1) == 4 && M.size(2) == 4 && v.dim() == 3 && v.size(2) == 3,
+                          "expected transformation (B,4,4) and vector (1|B,N,3)");
         TORCH_CHECK_VALUE(g.dim() == 3 && g.size(0) == M.size(0) && g.size(1) == v.size(1) && g.size(2) == 3,
                           "gradIn must have shape (B,N,3)");
         On on(v);
@@ -147,6 +154,8 @@ using ViewBwd = std::tuple<Tensor, Tensor>(const Tensor&, const Tensor&);
 Tensor view_forward_cuda(const Tensor& pos, const Tensor& quat) {
     need(pos, "positions");
     need(quat, "quaternions", &pos);
+    need_numel(pos, 3 * quat.size(0), "positions");
+    need_numel(quat, 4 * quat.size(0), "quaternions");
     On on(pos);
     Tensor out = at::empty({quat.size(0), 1, 4, 4}, pos.options());
     check(uds_view_matrix_forward(i32(quat.size(0)), f(pos), f(quat), fm(out), on.stream()), "view matrix forward");
@@ -155,6 +164,8 @@ Tensor view_forward_cuda(const Tensor& pos, const Tensor& quat) {
 std::tuple<Tensor, Tensor> view_backward_cuda(const Tensor& g, const Tensor& quat) {
     need(g, "gradIn");
     need(quat, "quaternions", &g);
+    need_numel(g, 16 * quat.size(0), "gradIn");
+    need_numel(quat, 4 * quat.size(0), "quaternions");
     On on(g);
     Tensor gp = at::empty({quat.size(0), 3}, g.options()), gq = at::empty_like(quat);
     check(uds_view_matrix_backward(i32(quat.size(0)), f(g), f(quat), fm(gp), fm(gq), on.stream()),
@@ -205,12 +216,15 @@ std::vector<Tensor> backface_cuda(const Tensor& cam, const OptTensor& nrm) {
 std::vector<Tensor> backface_backward_cuda(const Tensor& cam, const Tensor& gcam, const OptTensor& gnrm,
                                            int64_t batch) {
     need(cam, "camNormals");
+    TORCH_CHECK_VALUE(cam.dim() == 3 && cam.size(2) == 3, "camNormals must be (B,N,3)");
     need(gcam, "gradCam", &cam);
+    need_numel(gcam, cam.numel(), "gradCam");
     On on(cam);
     std::vector<Tensor> out{at::empty_like(cam)};
     const bool world = gnrm.has_value() && gnrm->defined();
     if (world) {
         need(*gnrm, "gradNormals", &cam);
+        need_numel(*gnrm, cam.numel(), "gradNormals");
         out.push_back(at::empty({batch, cam.size(1), 3}, cam.options()));
     }
     check(uds_backface_backward(i32(cam.size(0)), i32(cam.size(1)), f(cam), f(gcam), i32(batch), fo(gnrm), fm(out[0]),
@@ -272,6 +286,7 @@ void check_splats(const Tensor& ids, const Tensor& pts, const Tensor& nrm, const
     TORCH_CHECK_VALUE(ids.size(0) == pts.size(0) && sd.size(1) == pts.size(1) &&
                           (sd.size(0) == 1 || sd.size(0) == pts.size(0)),
                       "batch / splat counts of indices, points and stdDevs disagree");
+    TORCH_CHECK_VALUE(pts.size(2) == 3 && sd.size(2) == 2, "expected points/normals (B,N,3) and stdDevs (1|B,N,2)");
 }
 Tensor splat_forward_cuda(int64_t width, int64_t height, double focal, const Tensor& ids, const Tensor& pts,
                           const Tensor& nrm, const Tensor& sd, double smoothing) {
@@ -355,7 +370,10 @@ std::vector<Tensor> render_gradients(double focal, const Tensor& gimg, const Opt
             need(**g, name, &pts);
             TORCH_CHECK_VALUE((*g)->sizes() == ids.sizes(), name, " must match indices");
         }
-    const int B = i32(ids.size(0)), N = i32(pts.size(1)), C = i32(attr.size(2));
+    const int B = i32(ids.size(0)), N = i32(pts.size(1));
+    TORCH_CHECK_VALUE(attr.dim() == 3 && attr.size(1) == N && (attr.size(0) == 1 || attr.size(0) == B),
+                      "attribute must be (1|B,N,C)");
+    const int C = i32(attr.size(2));
     TORCH_CHECK_VALUE(gimg.dim() == 4 && gimg.size(0) == B && gimg.size(1) == ids.size(1) &&
                           gimg.size(2) == ids.size(2) && gimg.size(3) == C && w.sizes() == ids.sizes(),
                       "gradImage must be (B,W,H,C) and weights (B,W,H,K)");
@@ -487,6 +505,7 @@ void check_filter(const Tensor& ids, const Tensor& w, const Tensor& pts, const T
     TORCH_CHECK_VALUE(ids.sizes() == w.sizes() && ids.dim() == 4, "indices and weights must both be (B,W,H,K)");
     TORCH_CHECK_VALUE(pts.sizes() == nrm.sizes() && (pts.size(0) == 1 || pts.size(0) == ids.size(0)),
                       "points/normals must be (1|B,N,3)");
+    need_numel(pts, 3 * pts.size(0) * pts.size(1), "points");
 }
 Tensor filter_forward_cuda(const Tensor& ids, const Tensor& w, int64_t, int64_t, double focal, const Tensor& pts,
                            const Tensor& nrm) {
@@ -502,6 +521,7 @@ Tensor filter_backward_cuda(const Tensor& ids, const Tensor& w, const Tensor& g,
                             const Tensor& pts, const Tensor& nrm) {
     check_filter(ids, w, pts, nrm);
     need(g, "gradIn", &ids);
+    need_numel(g, ids.numel(), "gradIn");
     On on(pts);
     Tensor out = at::empty_like(w);
     check(uds_filter_backward(i32(ids.size(0)), i32(ids.size(1)), i32(ids.size(2)), i32(ids.size(3)), idx(ids), f(w),
@@ -560,6 +580,7 @@ std::tuple<Tensor, Tensor> interp_backward_cuda(const Tensor& g, const Tensor& i
                                                 const Tensor& attr) {
     check_interp(ids, w, attr);
     need(g, "gradIn", &ids);
+    need_numel(g, ids.size(0) * ids.size(1) * ids.size(2) * attr.size(2), "gradIn");
     On on(ids);
     Tensor gw = at::empty_like(w), ga = at::empty_like(attr);
     check(uds_interp_backward(i32(ids.size(0)), i32(ids.size(1)), i32(ids.size(2)), i32(ids.size(3)), f(g), idx(ids),
@@ -605,10 +626,23 @@ std::pair<int, int> pixels(const Tensor& nrm, const Tensor& dif) {
     const int64_t B = nrm.size(0);
     return {i32(B), B > 0 ? i32(nrm.numel() / (3 * B)) : 0};
 }
-Tensor shade_forward_cuda(const Tensor& dirs, const Tensor& power, const Tensor& nrm, const Tensor& dif) {
-    auto [B, P] = pixels(nrm, dif);
+void check_lamps(const Tensor& dirs, const Tensor& power, const Tensor& nrm) {
     need(dirs, "directions", &nrm);
     need(power, "intensities", &nrm);
+    need_numel(dirs, 3 * power.size(1) * nrm.size(0), "directions");
+    need_numel(power, 3 * power.size(1) * power.size(0), "intensities");
+}
+void check_sh(const Tensor& coef, const Tensor& nrm) {
+    need(coef, "coefficients", &nrm);
+    need_numel(coef, 27 * coef.size(0), "coefficients");
+}
+void check_grad(const Tensor& g, const Tensor& nrm) {
+    need(g, "gradIn", &nrm);
+    need_numel(g, nrm.numel(), "gradIn");
+}
+Tensor shade_forward_cuda(const Tensor& dirs, const Tensor& power, const Tensor& nrm, const Tensor& dif) {
+    auto [B, P] = pixels(nrm, dif);
+    check_lamps(dirs, power, nrm);
     On on(nrm);
     Tensor out = at::empty_like(nrm);
     check(uds_shade_forward(B, P, i32(power.size(1)), f(dirs), f(power), i32(power.size(0)), f(nrm), f(dif), fm(out),
@@ -619,9 +653,8 @@ Tensor shade_forward_cuda(const Tensor& dirs, const Tensor& power, const Tensor&
 std::vector<Tensor> shade_backward_cuda(const Tensor& g, const Tensor& dirs, const Tensor& power, const Tensor& nrm,
                                         const Tensor& dif) {
     auto [B, P] = pixels(nrm, dif);
-    need(g, "gradIn", &nrm);
-    need(dirs, "directions", &nrm);
-    need(power, "intensities", &nrm);
+    check_grad(g, nrm);
+    check_lamps(dirs, power, nrm);
     On on(nrm);
     Tensor gd = at::empty_like(dirs), gI = at::empty_like(power), gn = at::empty_like(nrm), gf = at::empty_like(dif);
     check(uds_shade_backward(B, P, i32(power.size(1)), f(g), f(dirs), f(power), i32(power.size(0)), f(nrm), f(dif),
@@ -631,7 +664,7 @@ std::vector<Tensor> shade_backward_cuda(const Tensor& g, const Tensor& dirs, con
 }
 Tensor sh_forward_cuda(const Tensor& coef, const Tensor& nrm, const Tensor& dif) {
     auto [B, P] = pixels(nrm, dif);
-    need(coef, "coefficients", &nrm);
+    check_sh(coef, nrm);
     On on(nrm);
     Tensor out = at::empty_like(nrm);
     check(uds_shade_sh_forward(B, P, f(coef), i32(coef.size(0)), f(nrm), f(dif), fm(out), on.stream()),
@@ -640,8 +673,8 @@ Tensor sh_forward_cuda(const Tensor& coef, const Tensor& nrm, const Tensor& dif)
 }
 std::vector<Tensor> sh_backward_cuda(const Tensor& g, const Tensor& coef, const Tensor& nrm, const Tensor& dif) {
     auto [B, P] = pixels(nrm, dif);
-    need(g, "gradIn", &nrm);
-    need(coef, "coefficients", &nrm);
+    check_grad(g, nrm);
+    check_sh(coef, nrm);
     On on(nrm);
     Tensor gc = at::empty_like(coef), gn = at::empty_like(nrm), gd = at::empty_like(dif);
     check(uds_shade_sh_backward(B, P, f(g), f(coef), i32(coef.size(0)), f(nrm), f(dif), fm(gc), fm(gn), fm(gd),
@@ -691,7 +724,7 @@ Tensor lambert_forward_cuda(const Tensor& amb, const Tensor& dirs, const Tensor&
 std::vector<Tensor> lambert_backward_cuda(const Tensor& g, const Tensor& amb, const Tensor& dirs, const Tensor& power,
                                           const Tensor& nrm, const Tensor& dif) {
     LambertShape s = lambert_shape(amb, dirs, power, nrm, dif);
-    need(g, "gradIn", &nrm);
+    check_grad(g, nrm);
     On on(nrm);
     Tensor ga = at::empty_like(amb), gd = at::empty_like(dirs), gI = at::empty_like(power);
     Tensor gn = at::empty_like(nrm), gf = at::empty_like(dif);
@@ -787,6 +820,7 @@ using LossFwd = std::tuple<Tensor, Tensor>(const Tensor&, const Tensor&, SymInt,
 std::tuple<Tensor, Tensor> image_loss_cuda(const Tensor& x, const Tensor& y, int64_t kind, double scale) {
     need(x, "image");
     need(y, "target", &x);
+    need_numel(y, x.numel(), "target");
     On on(x);
     Tensor loss = at::empty({}, x.options()), grad = at::empty_like(x);
     check(uds_image_loss(i32(kind), (size_t)x.numel(), f(x), f(y), (float)scale, fm(loss), fm(grad), on.stream()),

@@ -4,7 +4,7 @@ from __future__ import annotations
 
 import torch
 
-from .._lib import check, load, need, ptr, stream_ptr
+from .._lib import check, load, need, need_numel, ptr, stream_ptr
 
 
 def _check(indices, weights, points, normals):
@@ -17,6 +17,7 @@ def _check(indices, weights, points, normals):
         raise ValueError("indices and weights must both be (B,W,H,K)")
     if points.shape != normals.shape or points.shape[0] not in (1, indices.shape[0]):
         raise ValueError("points/normals must be (1|B,N,3)")
+    need_numel(points, 3 * points.shape[0] * points.shape[1], "points")
 
 
 def forward(indices, weights, width: int, height: int, focallength: float, points, normals):
@@ -32,6 +33,7 @@ def forward(indices, weights, width: int, height: int, focallength: float, point
 def backward(indices, weights, gradIn, width: int, height: int, focallength: float, points, normals):
     _check(indices, weights, points, normals)
     need(gradIn, "gradIn", device=indices.device)
+    need_numel(gradIn, indices.numel(), "gradIn")
     B, W, H, K = indices.shape
     out = torch.empty_like(weights)
     check(load().uds_filter_backward(B, W, H, K, ptr(indices), ptr(weights), ptr(gradIn), float(focallength),

@@ -3,7 +3,7 @@ from __future__ import annotations
 
 import torch
 
-from .._lib import check, load, need, ptr, stream_ptr
+from .._lib import check, load, need, need_numel, ptr, stream_ptr
 
 
 def _check(indices, weights, attribute):
@@ -31,6 +31,7 @@ def backward(gradIn, indices, weights, attribute):
     need(gradIn, "gradIn", device=indices.device)
     B, W, H, K = indices.shape
     C = attribute.shape[2]
+    need_numel(gradIn, B * W * H * C, "gradIn")
     gw = torch.empty_like(weights)
     ga = torch.empty_like(attribute)
     check(load().uds_interp_backward(B, W, H, K, ptr(gradIn), ptr(indices), ptr(weights), attribute.shape[0],

@@ -5,7 +5,7 @@ from __future__ import annotations
 
 import torch
 
-from .._lib import check, load, need, ptr, stream_ptr
+from .._lib import check, load, need, need_numel, ptr, stream_ptr
 
 
 def _pix(normals, diffuse):
@@ -17,11 +17,28 @@ def _pix(normals, diffuse):
     return B, normals.numel() // (3 * B)
 
 
-def forward(directions, intensities, normals, diffuse):
-    B, P = _pix(normals, diffuse)
+def _lamps(directions, intensities, normals):
     need(directions, "directions", device=normals.device)
     need(intensities, "intensities", device=normals.device)
     L = intensities.shape[1]
+    need_numel(directions, 3 * L * normals.shape[0], "directions")
+    need_numel(intensities, 3 * L * intensities.shape[0], "intensities")
+    return L
+
+
+def _sh(coefficients, normals):
+    need(coefficients, "coefficients", device=normals.device)
+    need_numel(coefficients, 27 * coefficients.shape[0], "coefficients")
+
+
+def _grad(gradIn, normals):
+    need(gradIn, "gradIn", device=normals.device)
+    need_numel(gradIn, normals.numel(), "gradIn")
+
+
+def forward(directions, intensities, normals, diffuse):
+    B, P = _pix(normals, diffuse)
+    L = _lamps(directions, intensities, normals)
     out = torch.empty_like(normals)
     check(load().uds_shade_forward(B, P, L, ptr(directions), ptr(intensities), intensities.shape[0], ptr(normals),
                                    ptr(diffuse), ptr(out), stream_ptr(normals.device)), "shading forward")
@@ -30,10 +47,8 @@ def forward(directions, intensities, normals, diffuse):
 
 def backward(gradIn, directions, intensities, normals, diffuse):
     B, P = _pix(normals, diffuse)
-    need(gradIn, "gradIn", device=normals.device)
-    need(directions, "directions", device=normals.device)
-    need(intensities, "intensities", device=normals.device)
-    L = intensities.shape[1]
+    _grad(gradIn, normals)
+    L = _lamps(directions, intensities, normals)
     gd, gI = torch.empty_like(directions), torch.empty_like(intensities)
     gn, gdf = torch.empty_like(normals), torch.empty_like(diffuse)
     check(load().uds_shade_backward(B, P, L, ptr(gradIn), ptr(directions), ptr(intensities), intensities.shape[0],
@@ -44,7 +59,7 @@ def backward(gradIn, directions, intensities, normals, diffuse):
 
 def forwardSh(coefficients, normals, diffuse):
     B, P = _pix(normals, diffuse)
-    need(coefficients, "coefficients", device=normals.device)
+    _sh(coefficients, normals)
     out = torch.empty_like(normals)
     check(load().uds_shade_sh_forward(B, P, ptr(coefficients), coefficients.shape[0], ptr(normals), ptr(diffuse),
                                       ptr(out), stream_ptr(normals.device)), "shading forwardSh")
@@ -53,8 +68,8 @@ def forwardSh(coefficients, normals, diffuse):
 
 def backwardSh(gradIn, coefficients, normals, diffuse):
     B, P = _pix(normals, diffuse)
-    need(gradIn, "gradIn", device=normals.device)
-    need(coefficients, "coefficients", device=normals.device)
+    _grad(gradIn, normals)
+    _sh(coefficients, normals)
     gc, gn, gd = torch.empty_like(coefficients), torch.empty_like(normals), torch.empty_like(diffuse)
     check(load().uds_shade_sh_backward(B, P, ptr(gradIn), ptr(coefficients), coefficients.shape[0], ptr(normals),
                                        ptr(diffuse), ptr(gc), ptr(gn), ptr(gd), stream_ptr(normals.device)),
@@ -114,7 +129,7 @@ def lambertForward(ambient, directions, intensities, normals, diffuse):
 
 def lambertBackward(gradIn, ambient, directions, intensities, normals, diffuse):
     B, N, L, aB, IB, dB = lambert_shapes(ambient, directions, intensities, normals, diffuse)
-    need(gradIn, "gradIn", device=normals.device)
+    _grad(gradIn, normals)
     ga, gdir, gI = torch.empty_like(ambient), torch.empty_like(directions), torch.empty_like(intensities)
     gn, gd = torch.empty_like(normals), torch.empty_like(diffuse)
     check(load().uds_lambert_backward(B, N, L, ptr(gradIn), ptr(ambient), aB, ptr(directions), ptr(intensities),

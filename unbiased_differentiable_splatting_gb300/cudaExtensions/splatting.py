@@ -17,6 +17,8 @@ def _check(indices, points, normals, stdDevs):
     B, N = points.shape[0], points.shape[1]
     if indices.shape[0] != B or stdDevs.shape[1] != N or stdDevs.shape[0] not in (1, B):
         raise ValueError("batch / splat counts of indices, points and stdDevs disagree")
+    if points.shape[2] != 3 or stdDevs.shape[2] != 2:
+        raise ValueError("expected points/normals (B,N,3) and stdDevs (1|B,N,2)")
 
 
 def forward(width: int, height: int, focallength: float, indices, points, normals, stdDevs, smoothing: float):
@@ -98,7 +100,10 @@ def renderBackward(width: int, height: int, focallength: float, gradImage, gradD
             if g.shape != indices.shape:
                 raise ValueError(f"{name} must match indices")
     B, W, H, K = indices.shape
-    N, C = points.shape[1], attribute.shape[2]
+    N = points.shape[1]
+    if attribute.dim() != 3 or attribute.shape[1] != N or attribute.shape[0] not in (1, B):
+        raise ValueError("attribute must be (1|B,N,C)")
+    C = attribute.shape[2]
     if tuple(gradImage.shape) != (B, W, H, C) or weights.shape != indices.shape:
         raise ValueError("gradImage must be (B,W,H,C) and weights (B,W,H,K)")
     L = load()

@@ -5,7 +5,7 @@ from __future__ import annotations
 
 import torch
 
-from .._lib import check, load, need, ptr, stream_ptr
+from .._lib import check, load, need, need_numel, ptr, stream_ptr
 
 
 def _forward(affine: bool, transformation: torch.Tensor, vector: torch.Tensor) -> torch.Tensor:
@@ -24,6 +24,8 @@ def _backward(affine: bool, gradIn: torch.Tensor, transformation: torch.Tensor, 
     need(gradIn, "gradIn")
     need(transformation, "transformation", device=gradIn.device)
     need(vector, "vector", device=gradIn.device)
+    if transformation.shape[1:] != (4, 4) or vector.dim() != 3 or vector.shape[2] != 3:
+        raise ValueError("expected transformation (B,4,4) and vector (1|B,N,3)")
     B, N = transformation.shape[0], vector.shape[1]
     if tuple(gradIn.shape) != (B, N, 3):
         raise ValueError("gradIn must have shape (B,N,3)")
@@ -56,6 +58,8 @@ def viewMatrixForward(positions: torch.Tensor, quaternions: torch.Tensor) -> tor
     need(positions, "positions")
     need(quaternions, "quaternions", device=positions.device)
     B = quaternions.shape[0]
+    need_numel(positions, 3 * B, "positions")
+    need_numel(quaternions, 4 * B, "quaternions")
     out = torch.empty((B, 1, 4, 4), dtype=torch.float32, device=positions.device)
     check(load().uds_view_matrix_forward(B, ptr(positions), ptr(quaternions), ptr(out), stream_ptr(positions.device)),
           "view matrix forward")
@@ -66,6 +70,8 @@ def viewMatrixBackward(gradIn: torch.Tensor, quaternions: torch.Tensor):
     need(gradIn, "gradIn")
     need(quaternions, "quaternions", device=gradIn.device)
     B = quaternions.shape[0]
+    need_numel(gradIn, 16 * B, "gradIn")
+    need_numel(quaternions, 4 * B, "quaternions")
     gp = torch.empty((B, 3), dtype=torch.float32, device=gradIn.device)
     gq = torch.empty_like(quaternions)
     check(load().uds_view_matrix_backward(B, ptr(gradIn), ptr(quaternions), ptr(gp), ptr(gq),
@@ -98,13 +104,17 @@ def backfaceBackward(camNormals: torch.Tensor, gradCam=None, gradNormals=None, n
     """Gradients of backfaceForward: [grad camNormals or None, grad normals
     (normalsBatch,N,3) or None]."""
     need(camNormals, "camNormals")
+    if camNormals.dim() != 3 or camNormals.shape[2] != 3:
+        raise ValueError("camNormals must be (B,N,3)")
     B, N = camNormals.shape[0], camNormals.shape[1]
     gc = gw = None
     if gradCam is not None:
         need(gradCam, "gradCam", device=camNormals.device)
+        need_numel(gradCam, 3 * B * N, "gradCam")
         gc = torch.empty_like(camNormals)
     if gradNormals is not None:
         need(gradNormals, "gradNormals", device=camNormals.device)
+        need_numel(gradNormals, 3 * B * N, "gradNormals")
         gw = torch.empty((normalsBatch, N, 3), dtype=torch.float32, device=camNormals.device)
     check(load().uds_backface_backward(B, N, ptr(camNormals), ptr(gradCam), normalsBatch, ptr(gradNormals), ptr(gc),
                                        ptr(gw), stream_ptr(camNormals.device)), "backface backward")

@@ -619,6 +619,7 @@ def image_loss(image: Tensor, target: Tensor, kind: int, scale: float) -> Tuple[
 
 @image_loss.register_fake
 def _(image, target, kind, scale):
+    torch._check_value(image.numel() == target.numel(), lambda: "target must have as many elements as image")
     return image.new_empty(()), torch.empty_like(image)
 
 

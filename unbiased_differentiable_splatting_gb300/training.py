@@ -8,13 +8,14 @@ from __future__ import annotations
 
 import torch as th
 
-from ._lib import check, load, need, ptr, stream_ptr
+from ._lib import check, load, need, need_numel, ptr, stream_ptr
 
 
 def image_loss(x, y, kind, scale):
     """(loss, gradient w.r.t. x) of the L1 (kind 0) or L2 (kind 1) image loss."""
     x = need(x, "image")
     y = need(y, "target", device=x.device)
+    need_numel(y, x.numel(), "target")
     loss = th.empty((), device=x.device)
     grad = th.empty_like(x)
     check(load().uds_image_loss(kind, x.numel(), ptr(x), ptr(y), float(scale), ptr(loss), ptr(grad),
