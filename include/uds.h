@@ -43,6 +43,13 @@ const char* uds_last_error(void);
 int uds_version(void);
 /* Number of kernels this library has enqueued since it was loaded. */
 unsigned long long uds_launch_count(void);
+/* Waits of one block for another (the prefix sums and sorts of the tree build
+ * and of the deterministic gather) that ran out on the current device since
+ * the library was loaded, counted by block, of work that has finished; copies
+ * from the device.  0 unless something is broken: a block waits for blocks
+ * that have started, and gives up after about a second.  The view then
+ * samples nothing (uds_view_stats), the gather returns NaNs. */
+int uds_wait_failures(uint32_t* count);
 
 /* Per-view record written by uds_sample (32 bytes). */
 typedef struct {

@@ -44,6 +44,7 @@ _SIGS = {
     "uds_status_string": (ctypes.c_char_p, [c_int]),
     "uds_last_error": (ctypes.c_char_p, []),
     "uds_version": (c_int, []),
+    "uds_wait_failures": (c_int, [ctypes.POINTER(ctypes.c_uint32)]),
     "uds_launch_count": (ctypes.c_ulonglong, []),
     "uds_transform_forward": (c_int, [c_int, c_int, c_void_p, c_int, c_int, c_void_p, c_void_p, c_void_p]),
     "uds_transform_backward": (c_int, [c_int, c_int, c_void_p, c_void_p, c_int, c_int, c_void_p, c_void_p,
@@ -193,6 +194,17 @@ def check(status: int, what: str) -> None:
         msg = L.uds_status_string(status).decode()
         detail = L.uds_last_error().decode() if status in (3, 4) else ""
         raise UdsError(f"{what}: {msg}" + (f" ({detail})" if detail else ""))
+
+
+def wait_failures(device=None) -> int:
+    """Waits between blocks of a kernel that ran out on a device since the
+    library was loaded (synchronises; see uds_wait_failures).  Not 0: views
+    sampled nothing, or gathers are NaN, for that reason."""
+    count = ctypes.c_uint32()
+    with torch.cuda.device(device if device is not None else torch.cuda.current_device()):
+        torch.cuda.synchronize()
+        check(load().uds_wait_failures(ctypes.byref(count)), "wait failures")
+    return count.value
 
 
 def stream_ptr(device=None) -> int:

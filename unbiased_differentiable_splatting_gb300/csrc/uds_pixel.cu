@@ -87,8 +87,8 @@ __global__ void k_pixel_gather_atomic(size_t S, size_t per_view, int N, int C, c
 
 // Deterministic mode.
 struct GatherState {
-    unsigned n;       // valid samples
-    unsigned failed;  // a wait ran out (see look_back): the sums are left at 0
+    unsigned n;   // valid samples
+    int failed;   // a wait ran out (see look_back): the sums are NaN
     unsigned ticket[6];
 };
 constexpr int kGatherPasses = 4;  // of 10 bits at most: 32-bit splat keys
@@ -146,7 +146,7 @@ __global__ void __launch_bounds__(kTileThreads) k_pixel_pack(size_t S, size_t pe
         if (lane == 0) {
             s_first = (unsigned)at;
             s_failed = !ok;
-            if (!ok) gs->failed = 1;
+            if (!ok) wait_failed(&gs->failed);
             else if (s_tile == (int)gridDim.x - 1) gs->n = (unsigned)at + total;
         }
     }
@@ -173,11 +173,11 @@ __global__ void __launch_bounds__(kTileThreads) k_pixel_sort(int pass, GatherSta
                                                              const unsigned* __restrict__ kin,
                                                              const unsigned* __restrict__ vin,
                                                              unsigned* __restrict__ kout, unsigned* __restrict__ vout) {
-    const unsigned n = gs->failed ? 0u : gs->n;
+    const unsigned n = failed_yet(&gs->failed) ? 0u : gs->n;
     if ((size_t)blockIdx.x * kSortTile >= n) return;
     if (!sort_tile<kSortItems, Word>(n, pass * kDigitBits, &gs->ticket[pass], hist, status, kin, vin, kout, vout) &&
         threadIdx.x == 0)
-        gs->failed = 1;
+        wait_failed(&gs->failed);
 }
 
 // First and one past the last of each splat's sorted samples (0, 0: none).
@@ -191,12 +191,17 @@ __global__ void k_pixel_bounds(const GatherState* gs, const unsigned* __restrict
 }
 
 // One thread per splat sums its bucket (already in sample order), up to four
-// channels at a time, the next samples' values on their way.
-__global__ void k_pixel_sum(size_t M, int C, const uint2* __restrict__ bounds, const unsigned* __restrict__ slots,
+// channels at a time, the next samples' values on their way.  A gather that
+// failed is all NaN.
+__global__ void k_pixel_sum(const GatherState* gs, size_t M, int C, const uint2* __restrict__ bounds, const unsigned* __restrict__ slots,
                             const float* __restrict__ values, float* __restrict__ out) {
     size_t key = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (key >= M) return;
     const uint2 range = bounds[key];
+    if (gs->failed) {
+        for (int c = 0; c < C; ++c) out[key * (size_t)C + c] = __int_as_float(0x7fc00000);
+        return;
+    }
     for (int c0 = 0; c0 < C; c0 += 4) {
         const int cn = min(4, C - c0);
         float s[4] = {0.0f, 0.0f, 0.0f, 0.0f};
@@ -212,6 +217,8 @@ __global__ void k_pixel_sum(size_t M, int C, const uint2* __restrict__ bounds, c
             if (c < cn) out[key * (size_t)C + c0 + c] = s[c];
     }
 }
+
+cudaError_t pixel_wait_failures(unsigned* count) { return cudaMemcpyFromSymbol(count, g_wait_failures, sizeof(*count)); }
 
 }  // namespace uds
 
@@ -323,6 +330,6 @@ extern "C" int uds_pixel_gather(int B, int W, int H, int K, const int32_t* indic
         t = vi; vi = vo; vo = t;
     }
     k_pixel_bounds<<<cdiv(S, 256) < 1216 ? cdiv(S, 256) : 1216, 256, 0, s>>>(g.state, ki, g.bounds);
-    k_pixel_sum<<<cdiv(M, 128), 128, 0, s>>>(M, C, g.bounds, vi, values, out);
+    k_pixel_sum<<<cdiv(M, 128), 128, 0, s>>>(g.state, M, C, g.bounds, vi, values, out);
     return launch_status(3 + g.passes);
 }

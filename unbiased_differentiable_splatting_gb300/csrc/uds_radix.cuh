@@ -16,9 +16,23 @@ constexpr int kTileThreads = 256;
 // before it until it meets one with its prefix, and publishes its own.  Tiles
 // are numbered by a ticket when their block starts, so the ones waited for
 // have all started, and publish before they wait.  A wait still ends after
-// kWait looks: the caller then marks its result as failed.  A word
+// kWait looks: the caller then marks its result as failed and counts that
+// (uds_wait_failures).  What marks it failed is read once per block (failed_yet):
+// another block of the same launch may set it between two threads' reads.  A word
 // holds state and sum together, so no other memory is ordered by it.
-constexpr int kWait = 1 << 20;
+#ifndef UDS_WAIT_LOOKS
+#define UDS_WAIT_LOOKS (1 << 20)
+#endif
+constexpr int kWait = UDS_WAIT_LOOKS;
+static __device__ unsigned g_wait_failures;  // of this file's kernels, since the library was loaded
+__device__ __forceinline__ void wait_failed(int* failed) {
+    atomicExch(failed, 1);
+    atomicAdd(&g_wait_failures, 1u);
+}
+// By a whole block: *failed, the same for all of its threads.
+__device__ __forceinline__ bool failed_yet(const int* failed) {
+    return __syncthreads_or(threadIdx.x == 0 && *(volatile const int*)failed) != 0;
+}
 constexpr unsigned long long kSumReady = 1ull << 62, kPrefixReady = 2ull << 62, kSumMask = kSumReady - 1ull;
 
 // By a whole warp: the sum of the tiles before `tile`; false if a wait ran out.
@@ -196,11 +210,14 @@ __device__ __forceinline__ bool sort_tile(unsigned n, int shift, unsigned* ticke
             }
             ++looks;
         }
-        if (looks >= kWait) s_failed = 1;
+        if (looks >= kWait) {
+            s_failed = 1;  // (and no prefix: the tiles behind fail too)
+        } else {
 #pragma unroll
-        for (int q = 0; q < kPer; ++q)
-            words[(size_t)tile * kDigits + threadIdx.x + q * kTileThreads] =
-                ((Word)2 << kState) | (before[q] + count[q]);
+            for (int q = 0; q < kPer; ++q)
+                words[(size_t)tile * kDigits + threadIdx.x + q * kTileThreads] =
+                    ((Word)2 << kState) | (before[q] + count[q]);
+        }
     }
     __syncthreads();
     if (s_failed) return false;

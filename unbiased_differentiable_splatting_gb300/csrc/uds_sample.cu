@@ -173,7 +173,8 @@ __device__ __forceinline__ P* shifted(P* p, size_t bytes) {
     using C = typename std::conditional<std::is_const<P>::value, const char, char>::type;
     return reinterpret_cast<P*>(reinterpret_cast<C*>(p) + bytes);
 }
-// Visible splats of a view whose build has not failed.
+// Visible splats of a view whose build has not failed (in kernels that cannot
+// make it fail; the others: failed_yet).
 __device__ __forceinline__ int visible(const ViewState* vs) { return vs->failed ? 0 : vs->n; }
 
 // --------------------------------------------------------- 1 bandwidth
@@ -364,7 +365,7 @@ __global__ void __launch_bounds__(kTileThreads) k_cull(int N, Batch bt, const fl
         const bool ok = tile_places<kTileItems * kWarps>(before, status, tile, first, total);
         if (lane == 0) {
             s_first = ok ? (int)first : -1;
-            if (!ok) vs->failed = 1;
+            if (!ok) wait_failed(&vs->failed);
             else if (tile == (int)gridDim.x - 1) vs->n = (int)(first + total);
         }
     }
@@ -392,13 +393,13 @@ __global__ void __launch_bounds__(kTileThreads) k_sort_pass(Batch bt, int pass, 
                                                             uint32_t* __restrict__ kout, uint32_t* __restrict__ vout) {
     const size_t off = bt.slot * blockIdx.y;
     vs = shifted(vs, off);
-    const int n = visible(vs);
+    const int n = failed_yet(&vs->failed) ? 0 : vs->n;
     if ((long long)blockIdx.x * kTile >= n) return;
     if (!sort_tile<kTileItems, uint32_t>(n, pass * kDigitBits, &vs->ticket[pass], shifted(hist, off) + pass * kDigits,
                              shifted(status, off) + (size_t)pass * tiles_max * kDigits, shifted(kin, off),
                              shifted(vin, off), shifted(kout, off), shifted(vout, off)) &&
         threadIdx.x == 0)
-        vs->failed = 1;
+        wait_failed(&vs->failed);
 }
 
 // ---------------------------------------------------- 4 leaves + Karras
@@ -722,7 +723,7 @@ __global__ void __launch_bounds__(kNodeTile) k_p2m(Batch bt, ViewState* vs, size
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const size_t shift = bt.slot * blockIdx.y;
     vs = shifted(vs, shift);
-    const int n = visible(vs);
+    const int n = failed_yet(&vs->failed) ? 0 : vs->n;
     const int tiles = (n - 1 + kNodeTile - 1) / kNodeTile;
     if (n < 2 || (int)blockIdx.x >= tiles) return;
     const int4* __restrict__ lnk = shifted(w.lnk, shift);
@@ -757,7 +758,7 @@ __global__ void __launch_bounds__(kNodeTile) k_p2m(Batch bt, ViewState* vs, size
         const bool ok = look_back(shifted(w.node_status, shift), s_tile, sum, first);
         if (lane == 0) {
             s_first = ok ? first : ~0ull;
-            if (!ok) vs->failed = 1;
+            if (!ok) wait_failed(&vs->failed);
         }
     }
     __syncthreads();
@@ -2861,6 +2862,10 @@ __global__ void k_fgt_eval(Tree T, const ViewState* vs, int m, const int* __rest
 }
 
 // ------------------------------------------------------------ host side
+cudaError_t sample_wait_failures(unsigned* count) {
+    return cudaMemcpyFromSymbol(count, g_wait_failures, sizeof(*count));
+}
+
 // Trees of the batch's views in the slots from w on; w.stats: the first view's
 // of the call.
 static int build_batch(const uds_sample_params* p, const Ws& w, const Batch& bt, const float* pts, const float* nrm,

@@ -33,6 +33,9 @@ int launch_status(int launches) {
     return UDS_ERR_LAUNCH;
 }
 
+cudaError_t sample_wait_failures(unsigned* count);  // uds_sample.cu
+cudaError_t pixel_wait_failures(unsigned* count);   // uds_pixel.cu
+
 }  // namespace uds
 
 extern "C" const char* uds_status_string(int status) {
@@ -47,6 +50,16 @@ extern "C" const char* uds_status_string(int status) {
 }
 
 extern "C" const char* uds_last_error(void) { return uds::g_last_error; }
+
+extern "C" int uds_wait_failures(uint32_t* count) {
+    if (!count) return UDS_ERR_ARGUMENT;
+    unsigned a = 0, b = 0;
+    cudaError_t e = uds::sample_wait_failures(&a);
+    if (e == cudaSuccess) e = uds::pixel_wait_failures(&b);
+    if (e != cudaSuccess) { uds::set_last_error(e); return UDS_ERR_CUDA; }
+    *count = a + b;
+    return UDS_OK;
+}
 
 extern "C" int uds_version(void) { return 100; }
 

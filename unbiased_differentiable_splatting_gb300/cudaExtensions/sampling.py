@@ -47,7 +47,7 @@ import math
 
 import torch
 
-from .._lib import SampleParams, ViewDesc, Workspace, check, load, need, ptr, stream_ptr
+from .._lib import SampleParams, UdsError, ViewDesc, Workspace, check, load, need, ptr, stream_ptr
 
 MAX_DEGREE = 16
 
@@ -240,9 +240,13 @@ def sample_stochastic(width: int, height: int, focallength: float, points, norma
 
 
 def view_stats(stats: torch.Tensor) -> dict:
-    """Decode a (B,8) uds_view_stats tensor (synchronises)."""
+    """Decode a (B,8) uds_view_stats tensor (synchronises).  Raises UdsError
+    where a view's tree could not be built."""
     s = stats.detach().cpu()
     ints = s.view(torch.int32)
+    failed = ints[:, 6].nonzero().flatten().tolist()
+    if failed:
+        raise UdsError(f"tree build: a wait between blocks ran out (views {failed}); nothing was sampled there")
     return dict(h=s[:, 0].clone(), radius=s[:, 1].clone(), n_visible=ints[:, 2].clone(), n_coefs=ints[:, 3].clone(),
                 demoted=ints[:, 4].clone(), overflow=ints[:, 5].clone())
 
