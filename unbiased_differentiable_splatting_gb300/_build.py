@@ -5,7 +5,8 @@ objects are linked into ``libuds.so`` next to this file against the shared CUDA
 runtime (the same ``libcudart.so`` torch loads).  ``csrc/uds_torch.cpp`` (the
 ops' CUDA kernels and autograd formulas in native code) becomes
 ``libuds_torch.so``, linked against it and torch.  A rebuild happens only when
-a source or header is newer than the library.
+a source or header is newer than the library, or, of the second one, when it
+was built for another torch or Python.
 """
 from __future__ import annotations
 
@@ -23,6 +24,7 @@ LIB = os.path.join(PKG, "libuds.so")
 OPS_LIB = os.path.join(PKG, "libuds_torch.so")
 OPS_SRC = os.path.join(CSRC, "uds_torch.cpp")
 OBJ = os.path.join(PKG, "_build")
+OPS_STAMP = os.path.join(OBJ, "uds_torch.built_for")
 ARCH = ["-gencode", "arch=compute_103a,code=sm_103a"]
 FLAGS = ["-std=c++17", "-O3", "-lineinfo", "-Xcompiler", "-fPIC", "-Xcompiler", "-fno-fast-math"]
 
@@ -51,8 +53,25 @@ def up_to_date() -> bool:
     return _newer(LIB, _deps())
 
 
+def _ops_target() -> str:
+    """What libuds_torch.so is linked against: torch's C++ interface and
+    Python's."""
+    import torch
+    return f"torch {torch.__version__}, {sysconfig.get_config_var('SOABI') or sys.version}\n"
+
+
+def ops_built() -> bool:
+    """Whether libuds_torch.so is there and was built for this torch and
+    Python."""
+    try:
+        with open(OPS_STAMP) as f:
+            return os.path.exists(OPS_LIB) and f.read() == _ops_target()
+    except OSError:
+        return False
+
+
 def _ops_up_to_date() -> bool:
-    return _newer(OPS_LIB, [OPS_SRC, os.path.join(ROOT, "include", "uds.h"), os.path.abspath(__file__)])
+    return ops_built() and _newer(OPS_LIB, [OPS_SRC, os.path.join(ROOT, "include", "uds.h"), os.path.abspath(__file__)])
 
 
 def _torch_dir() -> str:
@@ -116,6 +135,8 @@ def build(force: bool = False, verbose: bool = False) -> str:
                            "-rpath,/usr/local/cuda/lib64", "-Xlinker", "-soname,libuds.so"], LIB)
     if ops:
         _link(lambda tmp: _ops_link(ops_obj, tmp), OPS_LIB)
+        with open(OPS_STAMP, "w") as f:
+            f.write(_ops_target())
     return LIB
 
 

@@ -9,12 +9,13 @@ from __future__ import annotations
 import ctypes
 import os
 import threading
+import warnings
 
 import torch
 
 from . import _build
 
-_lock = threading.Lock()
+_lock = threading.RLock()
 _lib = None
 
 c_int, c_float, c_size_t, c_void_p = ctypes.c_int, ctypes.c_float, ctypes.c_size_t, ctypes.c_void_p
@@ -165,23 +166,42 @@ def load(build_if_missing: bool = True):
                 fn.restype = res
                 fn.argtypes = args
             _lib = L
+            if _ops_defined:
+                load_ops()
     return _lib
 
 
-_ops_loaded = False
+_ops_defined = _ops_loaded = False
+
+
+def ops_defined() -> None:
+    """library.py has defined torch.ops.uds: their native implementations are
+    loaded with libuds.so, which the first call does (importing the package
+    needs neither)."""
+    global _ops_defined
+    with _lock:
+        _ops_defined = True
+        if _lib is not None:
+            load_ops()
 
 
 def load_ops() -> None:
     """Load libuds_torch.so (the native CUDA implementations of torch.ops.uds),
-    building it in-tree first when it is missing."""
+    building it in-tree first when it is missing or was built for another torch
+    or Python.  Where that cannot be done, the Python definitions, which call
+    the same kernels, stay in use."""
     global _ops_loaded
-    load()
     with _lock:
-        if not _ops_loaded:
-            if not os.path.exists(_build.OPS_LIB):
+        if _ops_loaded:
+            return
+        _ops_loaded = True
+        load()
+        try:
+            if not _build.ops_built():
                 _build.build()
             torch.ops.load_library(_build.OPS_LIB)
-            _ops_loaded = True
+        except (OSError, RuntimeError) as e:
+            warnings.warn(f"torch.ops.uds run their Python definitions: {e}", RuntimeWarning, stacklevel=2)
 
 
 class UdsError(RuntimeError):

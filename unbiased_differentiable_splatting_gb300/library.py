@@ -13,8 +13,8 @@ dropped normal gradient), which ``extensions.EWASplatting`` and the renderer
 use.
 
 For CUDA tensors the implementations and autograd formulas of most ops are
-replaced by the same ones in native code (csrc/uds_torch.cpp, loaded at the
-end of this module): an eager call then runs no Python below the op.
+replaced by the same ones in native code (csrc/uds_torch.cpp, loaded by the
+first call of the library): an eager call then runs no Python below the op.
 
 Schemas use the reference's argument order; names are snake_case
 (``splat_forward`` for ``splatting.forward``).
@@ -641,4 +641,4 @@ OPS = ("sample", "sample_views", "splat_forward", "splat_backward", "ewa_weights
        "shade_sh_backward", "lambert_forward", "lambert_backward", "pixel_scatter", "pixel_gather", "nearest",
        "nearest_regularizer", "nearest_losses", "image_loss", "splat_gradients", "render_splats_gradients")
 
-_lib.load_ops()
+_lib.ops_defined()
