@@ -140,6 +140,20 @@ def choose(timings_ms: dict):
     return min(sorted(timings_ms), key=lambda t: timings_ms[t])
 
 
+def once_per_kernel(timer):
+    """The widths that run as 8 take its time: timed once, not again, so that
+    their difference from it is not noise (``choose`` then takes 8)."""
+    times = {}
+
+    def timed(tx, spread, leaf):
+        at = (4 if tx == 4 else 8, spread, leaf)
+        if at not in times:
+            times[at] = timer(*at)
+        return times[at]
+
+    return timed
+
+
 def tune_descent(width, height, focallength, points, normals, stdDevs, numSamples, smoothing, precision,
                  view=0, reps=3, candidates=CANDIDATES, timer=None, save=True, leaf_sizes=None, spreads=SPREADS):
     """Time the descent of view `view` for each (tile_x, spread) pair, and
@@ -177,6 +191,7 @@ def tune_descent(width, height, focallength, points, normals, stdDevs, numSample
                 if r:
                     ts.append(e0.elapsed_time(e1))
             return min(ts)
+        timer = once_per_kernel(timer)
     best, timings = _sweep(timer, candidates, spreads, leaf_sizes)
     if save:
         record(name, W, H, N, K, best, timings)
@@ -225,6 +240,7 @@ def tune_views(views, points, normals, stdDevs, numSamples, smoothing, precision
                 if r:
                     ts.append(e0.elapsed_time(e1))
             return min(ts)
+        timer = once_per_kernel(timer)
     best, timings = _sweep(timer, candidates, spreads, leaf_sizes)
     if save:
         record(name, 0, 0, N, K, best, timings, views=views)

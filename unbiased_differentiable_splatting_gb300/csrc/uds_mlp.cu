@@ -413,10 +413,6 @@ struct MlpGradSmem {
     uint32_t taddr;
 };
 
-__device__ __forceinline__ float get_bf16(const unsigned char* base, uint32_t off) {
-    return __bfloat162float(*reinterpret_cast<const __nv_bfloat16*>(base + off));
-}
-
 constexpr int kGradThreads = 256;
 
 // 8 consecutive K elements (k0 multiple of 8) of row r of a K-major operand.
