@@ -80,3 +80,27 @@ def test_calls_side_by_side(threads):
         for out in got[k]:
             for a, b in zip(out, alone[k]):
                 assert torch.equal(a, b)
+
+
+@pytest.mark.gpu
+def test_tree_freed_before_its_evaluation_has_run():
+    """A tree's memory is not given out again while a side stream reads it."""
+    if not torch.cuda.is_available():
+        pytest.skip("no CUDA device")
+    from unbiased_differentiable_splatting_gb300.cudaExtensions import sampling
+    W, H, f, p, n, sd = _scene(5, 20_000)
+    nodes = torch.arange(64, dtype=torch.int32, device=DEV)
+    queries = torch.rand((64, 2), device=DEV) * torch.tensor([W, H], device=DEV)
+    tree = sampling.build_tree(W, H, f, p, n, sd, 8, 0.0, 0.01)
+    expected = sampling.fgt_eval(tree, nodes, queries)
+    bytes_, at = tree["_ws"].numel(), tree["_ws"].data_ptr()
+    torch.cuda.synchronize()
+    side = torch.cuda.Stream()
+    with torch.cuda.stream(side):
+        torch.cuda._sleep(50_000_000)  # clock cycles: some 25 ms
+        got = sampling.fgt_eval(tree, nodes, queries)
+    del tree
+    other = torch.empty(bytes_, dtype=torch.uint8, device=DEV)
+    assert other.data_ptr() != at  # still held for the side stream
+    torch.cuda.synchronize()
+    assert torch.equal(got, expected) and bool((expected > 0).any())

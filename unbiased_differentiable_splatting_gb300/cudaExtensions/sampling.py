@@ -293,6 +293,7 @@ def fgt_eval(tree: dict, nodes, queries):
     nodes = need(nodes, "nodes", torch.int32)
     queries = need(queries, "queries", device=nodes.device)
     out = torch.empty(nodes.numel(), dtype=torch.float32, device=nodes.device)
+    ws.record_stream(torch.cuda.current_stream(nodes.device))  # (the tree may be freed before this has run)
     check(load().uds_fgt_eval(tree["_prm"], nodes.numel(), ptr(nodes), ptr(queries), ptr(out), ptr(ws), ws.numel(),
                               stream_ptr(nodes.device)), "fgt eval")
     return out
